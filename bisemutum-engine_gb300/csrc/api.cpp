@@ -1357,6 +1357,9 @@ void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t 
         cudaEventRecord((*ev)[k++], st);
         if (tag >= 0) tags->push_back(tag);
     };
+    // one traversal launch per segment boundary (shadow rays of segment s with the extension rays of s + 1),
+    // or one per stage when the stages are timed or counted one by one
+    const bool split = ev != nullptr || count_traversal;
     mark(-1);
     for (uint64_t begin = 0; begin < total_paths; begin += capacity) {
         uint32_t count = (uint32_t)std::min<uint64_t>(capacity, total_paths - begin);
@@ -1365,11 +1368,12 @@ void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t 
         mark(0);
         int q = 0;
         for (uint32_t seg = 0; seg < max_seg; ++seg) {
-            launch_extend(lc, st, sc->dev, wf, q, seg, count_traversal);
+            if (count_traversal) launch_extend_count(lc, st, sc->dev, wf, q, seg);
+            else launch_trace(lc, st, sc->dev, wf, q, seg, split || seg == 0 ? kNoSegment : seg - 1, accum);
             mark(1);
             launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, cache_wb != nullptr);
             mark(2);
-            launch_shadow(lc, st, sc->dev, wf, seg, accum);
+            if (split || seg + 1 == max_seg) launch_trace(lc, st, sc->dev, wf, q, kNoSegment, seg, accum);
             mark(3);
             q ^= 1;
         }

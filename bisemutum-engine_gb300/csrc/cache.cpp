@@ -313,7 +313,7 @@ bsm_status cache_train_frame(bsm_cache* c, const DevScene& sc, const DevView& vi
     }
     const uint32_t lights1 = sc.num_lights + 1u;
     if (bsm_status e = ensure_train_verts(c, cs.train_paths, cap, lights1)) return e;
-    // shadow queue view (the fields launch_shadow reads), sized for `cap` vertices x (lights + 1) rays
+    // shadow queue view (the fields launch_trace reads for shadow rays), sized for `cap` vertices x (lights + 1) rays
     const size_t sh = (size_t)cap * lights1;
     char* qb = (char*)c->tv_queue;
     Wavefront q{};
@@ -331,7 +331,7 @@ bsm_status cache_train_frame(bsm_cache* c, const DevScene& sc, const DevView& vi
     cudaMemsetAsync(c->sample_count, 0, 4, st);
     cudaMemsetAsync(q.counters, 0, kCntWords * 4, st);
     launch_train_paths(st, sc, c->view_dev, cs.train_paths, c->frame++, tv, q);
-    launch_shadow(lc, st, sc, q, 0, c->tv_rad);
+    launch_trace(lc, st, sc, q, 0, kNoSegment, 0, c->tv_rad);
     launch_train_targets(st, cs.train_paths, tv, c->samples, c->sample_count, c->sample_cap);
     if (cudaGetLastError() != cudaSuccess) return BSM_ERR_CUDA;
     uint32_t n = 0;

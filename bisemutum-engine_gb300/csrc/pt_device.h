@@ -35,6 +35,7 @@ constexpr int kMaxLights = 8;     // directional + point/spot + rect lights of a
 enum : uint32_t { kLightDir = 0, kLightPoint = 1, kLightRect = 2 };
 struct DevLight { float4 a, b, c, d; };
 constexpr int kMaxSeg = 16;
+constexpr uint32_t kNoSegment = kMaxSeg;   // launch_trace: no rays of that kind
 
 struct DevSky {
     uint32_t kind;             // BSM_SKY_CONSTANT / BSM_SKY_EQUIRECT
@@ -146,13 +147,17 @@ __device__ __forceinline__ void accum_fixed_add(unsigned long long* fx, uint32_t
 // ---- launch wrappers (pt_kernels.cu) ----
 void launch_camera(const LaunchCfg& lc, cudaStream_t st, const DevView* views, uint32_t n_views,
                    uint64_t path_begin, uint32_t path_count, const Wavefront& wf, uint32_t max_segments);
-void launch_extend(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
-                   uint32_t seg, bool count_traversal);
+// The extension rays of segment `ext` (queue q) and the shadow rays of segment `shd` in one launch; kNoSegment
+// leaves one kind out.  The two kinds are independent of each other: shading segment s queues both shd = s and
+// ext = s + 1.
+void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
+                  uint32_t shd, float4* accum);
+// The extension rays of `seg` with the traversal counters of BSM_PT_COUNT_TRAVERSAL.
+void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
+                         uint32_t seg);
 // `cache`: some view of the launch queries the radiance cache
 void launch_shade(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView* views,
                   const Wavefront& wf, int q, uint32_t seg, float4* accum, bool cache = false);
-void launch_shadow(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, uint32_t seg,
-                   float4* accum);
 void launch_resolve(cudaStream_t st, const float4* accum, uint32_t width, uint32_t height, float inv_spp,
                     float4* out, uint32_t pitch_px);
 // accum[p] += fx[3p .. 3p + 2] * 2^-32 for the n accumulator pixels (one add per pixel: deterministic)
@@ -198,7 +203,7 @@ cudaError_t launch_mlp_adam(cudaStream_t st, float* wm, void* wb, const float* d
 // training paths (train_paths.cu): full-length paths that record per-vertex cache samples.
 // Vertex v = path x segments + k.  The path kernel writes each vertex's raw inputs (3 float4), throughput
 // and directly gathered radiance, and queues its next-event shadow rays in `shadow` (sun/light rays from the
-// front, sky rays from the back, contribution.w = the vertex's bits); the shadow pass (launch_shadow with the
+// front, sky rays from the back, contribution.w = the vertex's bits); the shadow pass (launch_trace with the
 // queue's accum_fx = fx) adds the unoccluded ones as exact fixed-point sums; the targets kernels turn each
 // vertex into a training sample, written at an offset from a scan of the per-path counts, so the samples'
 // order (and everything trained on them) does not depend on the order of the GPU's atomics.

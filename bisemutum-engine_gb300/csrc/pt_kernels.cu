@@ -1,16 +1,17 @@
 // pt_kernels.cu — the sm_103a kernels of the wavefront path-tracing pass.
 //
 // One render is a sequence of chunks; each chunk runs
-//   k_camera  -> [k_extend -> k_shade -> k_shadow] x segments
+//   k_camera -> k_trace(extend 0) -> k_shade(0) -> k_trace(extend 1, shadow 0) -> k_shade(1) -> ...
+//            -> k_trace(shadow of the last segment)
 // over device-resident queues whose sizes live in device counters, so no
 // stage waits for the host and a whole render can be captured as one CUDA
 // graph.  Stage <-> reference shader:
 //   k_camera   generate_camera_ray_cs   (direction_sample/generate_camera_ray.hlsl:4-16)
-//   k_extend   rt_gbuffer_rgen/rchit/rmiss (rt_gbuffer.hlsl:7-36, hits/rt_gbuffer_hit.hlsl:6-18)
+//   k_trace    extension rays: rt_gbuffer_rgen/rchit/rmiss (rt_gbuffer.hlsl:7-36, hits/rt_gbuffer_hit.hlsl:6-18);
+//              shadow rays: the visibility term of the direct light (there: shadow maps,
+//              lights.hlsl:27-104; here: any-hit rays)
 //   k_shade    deferred_lighting_secondary_cs + sample_secondary_ray_cs
 //              (deferred_lighting_secondary.hlsl:11-111, sample_secondary_ray.hlsl:11-69)
-//   k_shadow   the visibility term of the direct light (there: shadow maps,
-//              lights.hlsl:27-104; here: any-hit rays)
 //   k_resolve  additive blit + pt_accumulate_cs (path_tracing.cpp:436-478, pt_accumulate.hlsl:3-11)
 // Compiled with --fmad=false: every float operation outside the explicit
 // __fmaf_rn of the box test rounds once, as on the CPU oracle.
@@ -138,105 +139,122 @@ __global__ void k_camera(const DevView* __restrict__ views, uint32_t n_views, ui
 }
 
 // ---------------------------------------------------------------- extend ----
-template <bool kCount, int kMinBlocks, bool kOpacity>
-__global__ void __launch_bounds__(256, kMinBlocks) k_extend(DevScene sc, const float4* __restrict__ ray_o,
-                                                const float4* __restrict__ ray_d, const uint4* __restrict__ path,
-                                                float4* __restrict__ hit, uint32_t* counters,
-                                                unsigned long long* stats, uint32_t seg, int postpone_sp,
-                                                int refill_min) {
-    uint32_t n = counters[kCntQueue + seg];
+// Counting variant of the closest-hit stage (BSM_PT_COUNT_TRAVERSAL).
+struct CountRays {
+    const float4 *ray_o, *ray_d;
+    const uint4* path;
+    float4* hits;
+    __device__ __forceinline__ bool any(uint32_t) const { return false; }
+    __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) const { o = ray_o[i]; d = ray_d[i]; }
+    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v) const {
+        hits[i] = make_float4(t, __uint_as_float(leaf), u, v);
+    }
+    __device__ __forceinline__ void miss(uint32_t i, float tmax) const { hit(i, kMissPrim, tmax, 0.0f, 0.0f); }
+    __device__ __forceinline__ uint32_t seed(uint32_t i) const { return path[i].z; }   // the path's PCG32 word
+};
+template <bool kOpacity>
+__global__ void __launch_bounds__(256) k_extend_count(DevScene sc, CountRays rays, uint32_t* counters,
+                                                      unsigned long long* stats, uint32_t seg, int postpone_sp,
+                                                      int refill_min) {
+    const uint32_t n = counters[kCntQueue + seg];
     if (blockIdx.x == 0 && threadIdx.x == 0) stats[kStatExtend + seg] += n;
     TraceCounters c{0, 0};
-    trace_queue<false, kCount, kOpacity>(
-        sc.nodes, sc.tris, n, counters + kCntWork + 2 * seg,
-        [&](uint32_t i, float4& o, float4& d) { o = ray_o[i]; d = ray_d[i]; },
-        [&](uint32_t i, uint32_t leaf, float t, float u, float v) {
-            hit[i] = make_float4(t, __uint_as_float(leaf), u, v);
-        },
-        [&](uint32_t i) { return path[i].z; },   // the path's PCG32 word
-        &c, postpone_sp, refill_min);
-    if (kCount) {
-        uint32_t cn = c.nodes, ct = c.tris;
-        for (int off = 16; off > 0; off >>= 1) {
-            cn += __shfl_xor_sync(0xffffffffu, cn, off);
-            ct += __shfl_xor_sync(0xffffffffu, ct, off);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(stats + kStatNodes, (unsigned long long)cn);
-            atomicAdd(stats + kStatTris, (unsigned long long)ct);
-        }
+    trace_queue<true, kOpacity>(sc.nodes, sc.tris, n, counters + kCntWork + 2 * seg, rays, &c, postpone_sp, refill_min);
+    uint32_t cn = c.nodes, ct = c.tris;
+    for (int off = 16; off > 0; off >>= 1) {
+        cn += __shfl_xor_sync(0xffffffffu, cn, off);
+        ct += __shfl_xor_sync(0xffffffffu, ct, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(stats + kStatNodes, (unsigned long long)cn);
+        atomicAdd(stats + kStatTris, (unsigned long long)ct);
     }
 }
 
-// ---------------------------------------------------------------- shadow ----
+// ------------------------------------------------------- extend + shadow ----
+// The extension rays of segment `ext` (closest hit) and the shadow rays of
+// segment `shd` (any hit) as one queue: index i < n_ext is extension ray i,
+// then the sun rays from the front of the shadow queue, then the sky rays from
+// its back.  A launch is bound by instruction issue while its queue lasts and
+// by the latency of its last rays after that (60-100 us on the terrain: a
+// grazing ray visits over 100 nodes, each a round trip to L2).  Both kinds are
+// queued by the same shading launch and neither reads what the other writes,
+// so tracing them together leaves one such tail per segment instead of two.
+// Against a launch per kind: 128x128 preview of the room 534 -> 381 us,
+// 1920x1080 1-spp frame of the 1.48 M-triangle terrain 5.01 -> 4.21 ms, its
+// 64-spp frame 180.6 -> 179.1 ms.
+struct TraceArgs {
+    const float4 *ray_o, *ray_d;
+    const uint4* path;
+    float4* hit;
+    const float4 *sh_o, *sh_d, *sh_c;
+    const uint32_t* sh_seed;
+    float4* accum;
+    unsigned long long* accum_fx;
+    uint32_t* counters;
+    unsigned long long* stats;
+    uint32_t ext, shd, sh_last;   // segments (kNoSegment: none); the shadow queue's last slot
+    int postpone_sp, refill_min;
+};
+struct TraceRays {
+    const TraceArgs& a;
+    uint32_t n_ext, n_front, n;   // extension rays; with the sun rays; all
+    __device__ __forceinline__ uint32_t* work() const {
+        return a.counters + kCntWork + (a.ext < kNoSegment ? 2u * a.ext : 2u * a.shd + 1u);
+    }
+    __device__ __forceinline__ uint32_t slot(uint32_t i) const { return i < n_front ? i - n_ext : a.sh_last - (i - n_front); }
+    __device__ __forceinline__ bool any(uint32_t i) const { return i >= n_ext; }
+    __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) const {
+        if (i < n_ext) { o = __ldg(a.ray_o + i); d = __ldg(a.ray_d + i); }
+        else { const uint32_t k = slot(i); o = __ldg(a.sh_o + k); d = __ldg(a.sh_d + k); }
+    }
+    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v) const {
+        if (i < n_ext) a.hit[i] = make_float4(t, __uint_as_float(leaf), u, v);
+    }
+    __device__ __forceinline__ void miss(uint32_t i, float tmax) const {
+        if (i < n_ext) {
+            a.hit[i] = make_float4(tmax, __uint_as_float(kMissPrim), 0.0f, 0.0f);
+        } else {
+            const float4 c = __ldg(a.sh_c + slot(i));
+            accum_add(a.accum, a.accum_fx, __float_as_uint(c.w), v3(c.x, c.y, c.z));
+        }
+    }
+    // opacity seed: the path's PCG32 word, or the shadow ray's own
+    __device__ __forceinline__ uint32_t seed(uint32_t i) const {
+        return i < n_ext ? __ldg(&a.path[i].z) : (a.sh_seed ? __ldg(a.sh_seed + slot(i)) : 0u);
+    }
+};
+// The launch's queue sizes from the device counters; the first thread adds them to the statistics.
+__device__ __forceinline__ TraceRays trace_rays(const TraceArgs& a) {
+    const uint32_t n_ext = a.ext < kNoSegment ? a.counters[kCntQueue + a.ext] : 0u;
+    uint32_t n_sun = 0, n_sky = 0;
+    if (a.shd < kNoSegment) {
+        n_sun = a.counters[kCntShadow + a.shd];
+        n_sky = a.counters[kCntSky + a.shd];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (n_ext) a.stats[kStatExtend + a.ext] += n_ext;
+        if (n_sun + n_sky) a.stats[kStatShadow + a.shd] += n_sun + n_sky;
+    }
+    return TraceRays{a, n_ext, n_ext + n_sun, n_ext + n_sun + n_sky};
+}
+
 template <int kMinBlocks, bool kOpacity>
-__global__ void __launch_bounds__(256, kMinBlocks) k_shadow(DevScene sc, Wavefront wf, uint32_t seg, float4* accum,
-                                                            int postpone_sp, int refill_min) {
-    const uint32_t n_sun = wf.counters[kCntShadow + seg], n_sky = wf.counters[kCntSky + seg];
-    const uint32_t sh_cap = wf.capacity * (sc.num_lights + 1u);
-    const uint32_t n = n_sun + n_sky;
-    if (blockIdx.x == 0 && threadIdx.x == 0) wf.stats[kStatShadow + seg] += n;
-    const float4* __restrict__ so = wf.sh_o;
-    const float4* __restrict__ sd = wf.sh_d;
-    const float4* __restrict__ scn = wf.sh_c;
-    // work index i < n_sun: sun ray i; otherwise sky ray at the back of the queue
-    auto slot = [=](uint32_t i) { return i < n_sun ? i : sh_cap - 1u - (i - n_sun); };
-    trace_queue<true, false, kOpacity>(
-        sc.nodes, sc.tris, n, wf.counters + kCntWork + 2 * seg + 1,
-        [&](uint32_t i, float4& o, float4& d) { uint32_t k = slot(i); o = so[k]; d = sd[k]; },
-        [&](uint32_t i, uint32_t leaf, float, float, float) {
-            if (leaf == kMissPrim) {
-                float4 c = scn[slot(i)];
-                accum_add(accum, wf.accum_fx, __float_as_uint(c.w), v3(c.x, c.y, c.z));
-            }
-        },
-        [&](uint32_t i) { return wf.sh_seed ? wf.sh_seed[slot(i)] : 0u; },
-        nullptr, postpone_sp, refill_min);
+__global__ void __launch_bounds__(256, kMinBlocks) k_trace(const CwNode* __restrict__ nodes,
+                                                           const CwTri* __restrict__ tris,
+                                                           const __grid_constant__ TraceArgs a) {
+    const TraceRays rays = trace_rays(a);
+    trace_queue<false, kOpacity>(nodes, tris, rays.n, rays.work(), rays, nullptr, a.postpone_sp, a.refill_min);
 }
 
-// ------------------------------------------------- two-level extend / shadow ----
-// Two-level scenes: persistent warps over the queue with trace_queue2 (TLAS
-// leaves enter instances).  The hit record carries the instance in place of u.
+// The same for two-level scenes: trace_queue2 (TLAS leaves enter instances).
+// The hit record carries the instance in place of u.
 template <bool kOpacity>
-__global__ void __launch_bounds__(256, 4) k_extend2(DevScene sc, const float4* __restrict__ ray_o,
-                                                    const float4* __restrict__ ray_d, const uint4* __restrict__ path,
-                                                    float4* __restrict__ hit, uint32_t* counters,
-                                                    unsigned long long* stats, uint32_t seg, int postpone_sp,
-                                                    int refill_min) {
-    const uint32_t n = counters[kCntQueue + seg];
-    if (blockIdx.x == 0 && threadIdx.x == 0) stats[kStatExtend + seg] += n;
-    trace_queue2<false, kOpacity>(
-        sc.nodes, sc.insts, sc.mat_tr, n, counters + kCntWork + 2 * seg,
-        [&](uint32_t i, float4& o, float4& d) { o = ray_o[i]; d = ray_d[i]; },
-        [&](uint32_t i, uint32_t leaf, float t, float, float v, uint32_t inst) {
-            hit[i] = make_float4(t, __uint_as_float(leaf), __uint_as_float(inst), v);
-        },
-        [&](uint32_t i) { return path[i].z; },   // the path's PCG32 word
-        postpone_sp, refill_min);
-}
-
-template <bool kOpacity>
-__global__ void __launch_bounds__(256, 4) k_shadow2(DevScene sc, Wavefront wf, uint32_t seg, float4* accum,
-                                                    int postpone_sp, int refill_min) {
-    const uint32_t n_sun = wf.counters[kCntShadow + seg], n_sky = wf.counters[kCntSky + seg];
-    const uint32_t sh_cap = wf.capacity * (sc.num_lights + 1u);
-    const uint32_t n = n_sun + n_sky;
-    if (blockIdx.x == 0 && threadIdx.x == 0) wf.stats[kStatShadow + seg] += n;
-    const float4* __restrict__ so = wf.sh_o;
-    const float4* __restrict__ sd = wf.sh_d;
-    const float4* __restrict__ scn = wf.sh_c;
-    auto slot = [=](uint32_t i) { return i < n_sun ? i : sh_cap - 1u - (i - n_sun); };
-    trace_queue2<true, kOpacity>(
-        sc.nodes, sc.insts, sc.mat_tr, n, wf.counters + kCntWork + 2 * seg + 1,
-        [&](uint32_t i, float4& o, float4& d) { uint32_t k = slot(i); o = so[k]; d = sd[k]; },
-        [&](uint32_t i, uint32_t leaf, float, float, float, uint32_t) {
-            if (leaf == kMissPrim) {
-                float4 c = scn[slot(i)];
-                accum_add(accum, wf.accum_fx, __float_as_uint(c.w), v3(c.x, c.y, c.z));
-            }
-        },
-        [&](uint32_t i) { return wf.sh_seed ? wf.sh_seed[slot(i)] : 0u; },
-        postpone_sp, refill_min);
+__global__ void __launch_bounds__(256, 4) k_trace2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
+                                                   const float* __restrict__ mat_tr,
+                                                   const __grid_constant__ TraceArgs a) {
+    const TraceRays rays = trace_rays(a);
+    trace_queue2<kOpacity>(tlas, insts, mat_tr, rays.n, rays.work(), rays, a.postpone_sp, a.refill_min);
 }
 
 // ----------------------------------------------------------------- shade ----
@@ -666,27 +684,32 @@ void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const
     if (n) k_gather_normals<<<(n + 255) / 256, 256, 0, st>>>(tris, n, vn, idx, out);
 }
 
-void launch_extend(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
-                   uint32_t seg, bool count_traversal) {
-#define BSM_EXTEND(C, B, O)                                                                                    \
-    k_extend<C, B, O><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc, wf.ray_o[q], wf.ray_d[q], wf.path[q], \
-                                                                     wf.hit, wf.counters, wf.stats, seg,        \
-                                                                     lc.postpone_sp, lc.refill_min)
+void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
+                  uint32_t shd, float4* accum) {
     const bool op = sc.has_non_opaque != 0;
+    const TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
+                      wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u,
+                      lc.postpone_sp, lc.refill_min};
     if (sc.insts) {
-        if (op)
-            k_extend2<true><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(
-                sc, wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.counters, wf.stats, seg, lc.postpone_sp,
-                lc.refill_min);
-        else
-            k_extend2<false><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(
-                sc, wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.counters, wf.stats, seg, lc.postpone_sp,
-                lc.refill_min);
+        if (op) k_trace2<true><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else k_trace2<false><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        return;
     }
-    else if (count_traversal) { if (op) BSM_EXTEND(true, 1, true); else BSM_EXTEND(true, 1, false); }
-    else if (lc.regcap) { if (op) BSM_EXTEND(false, 4, true); else BSM_EXTEND(false, 4, false); }
-    else { if (op) BSM_EXTEND(false, 1, true); else BSM_EXTEND(false, 1, false); }
-#undef BSM_EXTEND
+#define BSM_TRACE(B, O) k_trace<B, O><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc.nodes, sc.tris, a)
+    if (lc.regcap) { if (op) BSM_TRACE(4, true); else BSM_TRACE(4, false); }
+    else { if (op) BSM_TRACE(1, true); else BSM_TRACE(1, false); }
+#undef BSM_TRACE
+}
+void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
+                         uint32_t seg) {
+    if (sc.insts) { launch_trace(lc, st, sc, wf, q, seg, kNoSegment, nullptr); return; }   // counters: single-level only
+    const CountRays rays{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit};
+    if (sc.has_non_opaque)
+        k_extend_count<true><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc, rays, wf.counters, wf.stats, seg,
+                                                                            lc.postpone_sp, lc.refill_min);
+    else
+        k_extend_count<false><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc, rays, wf.counters, wf.stats, seg,
+                                                                             lc.postpone_sp, lc.refill_min);
 }
 void launch_shade(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView* views,
                   const Wavefront& wf, int q, uint32_t seg, float4* accum, bool cache) {
@@ -694,22 +717,6 @@ void launch_shade(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, cons
         k_shade<true><<<lc.grid_shade, lc.block_shade, 0, st>>>(sc, views, wf, q, seg, accum);
     else
         k_shade<false><<<lc.grid_shade, lc.block_shade, 0, st>>>(sc, views, wf, q, seg, accum);
-}
-void launch_shadow(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, uint32_t seg,
-                   float4* accum) {
-#define BSM_SHADOW(B, O) \
-    k_shadow<B, O><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc, wf, seg, accum, lc.postpone_sp, lc.refill_min)
-    const bool op = sc.has_non_opaque != 0;
-    if (sc.insts) {
-        if (op)
-            k_shadow2<true><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc, wf, seg, accum, lc.postpone_sp,
-                                                                            lc.refill_min);
-        else
-            k_shadow2<false><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc, wf, seg, accum, lc.postpone_sp,
-                                                                             lc.refill_min);
-    } else if (lc.regcap) { if (op) BSM_SHADOW(4, true); else BSM_SHADOW(4, false); }
-    else { if (op) BSM_SHADOW(1, true); else BSM_SHADOW(1, false); }
-#undef BSM_SHADOW
 }
 void launch_resolve(cudaStream_t st, const float4* accum, uint32_t width, uint32_t height, float inv_spp,
                     float4* out, uint32_t pitch_px) {
@@ -750,22 +757,16 @@ void launch_trace_count(cudaStream_t st, const DevScene& sc, const float4* rays,
 void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int per_sm_ext = 0, per_sm_sh = 0, per_sm_shade = 0;
-    if (lc->regcap) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_ext, k_extend<false, 4, true>, block_trace, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_sh, k_shadow<4, true>, block_trace, 0);
-    } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_ext, k_extend<false, 1, true>, block_trace, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_sh, k_shadow<1, true>, block_trace, 0);
-    }
+    int per_sm = 0, per_sm_shade = 0;
+    if (lc->regcap)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<4, true>, block_trace, 0);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<1, true>, block_trace, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_shade, k_shade<true>, 512, 0);
-    int per_sm2_ext = 0, per_sm2_sh = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2_ext, k_extend2<true>, block_trace, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2_sh, k_shadow2<true>, block_trace, 0);
-    int per_sm2 = per_sm2_ext < per_sm2_sh ? per_sm2_ext : per_sm2_sh;
+    int per_sm2 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_trace2<true>, block_trace, 0);
     if (per_sm2 < 1) per_sm2 = 1;
     lc->grid_persistent2 = sms * per_sm2;
-    int per_sm = per_sm_ext < per_sm_sh ? per_sm_ext : per_sm_sh;
     if (per_sm < 1) per_sm = 1;
     if (per_sm_shade < 1) per_sm_shade = 1;
     lc->block_trace = block_trace;

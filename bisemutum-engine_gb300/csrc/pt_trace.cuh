@@ -437,26 +437,29 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 // Persistent, warp-synchronous traversal of a queue of n rays.  Every lane of
-// the warp runs this loop together (all ballots use the full mask).  `load`
-// (index -> (origin/tmin, direction/tmax)) supplies rays; `finish(index, leaf,
-// t, u, v)` receives each result (leaf = kMissPrim on a miss; for any-hit the
-// first hit found); with kOpacity, `seed(index)` gives the ray's opacity seed,
-// read only when a candidate hit lies on a non-opaque triangle (scenes without
-// one use the kOpacity = false instantiation, which skips the rule).
+// the warp runs this loop together (all ballots use the full mask).  `rays`
+// supplies them: `load` (index -> (origin/tmin, direction/tmax)); `any(index)`,
+// whether the ray stops at its first hit; `hit(index, leaf, t, u, v)`, called
+// at every closer hit (the last call stands: keeping the record in memory
+// instead of registers frees three of the 64, which is what it takes to keep
+// this loop from spilling), and `miss(index, tmax)`; with kOpacity,
+// `seed(index)` gives the ray's opacity seed, read only when a candidate hit
+// lies on a non-opaque triangle (scenes without one use the kOpacity = false
+// instantiation, which skips the rule).
 // `postpone_sp` (<= kPostponeMaxSp) is the stack depth below which triangle
 // groups may be postponed (0 disables postponing); `refill_min` is the number
 // of idle lanes that makes the warp fetch new rays.  Both are tuning knobs.
-template <bool kAnyHit, bool kCount, bool kOpacity, class Load, class Finish, class Seed>
+template <bool kCount, bool kOpacity, class Rays>
 __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
-                                            uint32_t n, uint32_t* work, Load load, Finish finish, Seed seed,
-                                            TraceCounters* cnt, int postpone_sp, int refill_min) {
+                                            uint32_t n, uint32_t* work, const Rays& rays, TraceCounters* cnt,
+                                            int postpone_sp, int refill_min) {
     postpone_sp = postpone_sp < kPostponeMaxSp ? postpone_sp : kPostponeMaxSp;
     const uint32_t lane = threadIdx.x & 31u;
     bool has = false;
-    bool exhausted = false;  // warp-uniform
+    bool exhausted = n == 0u;  // warp-uniform
     RayPre r;
-    float tbest = 0.0f, bu = 0.0f, bv = 0.0f;
-    uint32_t best_leaf = kMissPrim, best_prim = kMissPrim, idx = 0;
+    float tbest = 0.0f;
+    uint32_t best_prim = kMissPrim, idx = 0;
     uint2 G = make_uint2(0, 0), T = make_uint2(0, 0);
     uint2 stack[kStackSize];
     int sp = 0;
@@ -473,10 +476,10 @@ __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, co
                 uint32_t i = base + (uint32_t)__popc(idle & lanemask_lt());
                 if (i < n) {
                     float4 o, d;
-                    load(i, o, d);
+                    rays.load(i, o, d);
                     r = make_ray(o, d);
                     tbest = d.w;
-                    best_leaf = kMissPrim; best_prim = kMissPrim; bu = 0.0f; bv = 0.0f;
+                    best_prim = kMissPrim;
                     G = make_uint2(0u, ray_traceable(r, d.w) ? (0x80000000u | (1u << (7u ^ r.oct_key))) : 0u);
                     T = make_uint2(0u, 0u);
                     sp = 0;
@@ -522,18 +525,20 @@ __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, co
                 if (kCount) cnt->tris++;
                 float t, u, v;
                 if (tri_test(r, a, b, c, tbest, prim, best_prim, t, u, v) &&
-                    (!kOpacity || c.w == 0.0f || keep_hit(r, c.w, seed(idx)))) {
-                    tbest = t; best_leaf = ti; best_prim = prim; bu = u; bv = v;
-                    if (kAnyHit) { T.y = 0u; G.y = 0u; sp = 0; }
+                    (!kOpacity || c.w == 0.0f || keep_hit(r, c.w, rays.seed(idx)))) {
+                    tbest = t;
+                    best_prim = prim;
+                    rays.hit(idx, ti, t, u, v);
+                    if (rays.any(idx)) { T.y = 0u; G.y = 0u; sp = 0; }
                 }
             }
         }
         // next group, or done
         if (has && (G.y & 0xff000000u) == 0u && !has_tris(T)) {
-            if (sp > 0 && !(kAnyHit && best_leaf != kMissPrim)) {
+            if (sp > 0) {
                 G = stack[--sp];
             } else {
-                finish(idx, best_leaf, tbest, bu, bv);
+                if (best_prim == kMissPrim) rays.miss(idx, tbest);
                 has = false;
             }
         }
@@ -563,18 +568,18 @@ static_assert(kMaxTlasDepth + 3 + kMaxTraversalDepth + 2 * kPostponeMaxSp <= kSt
 // Results and the opacity rule are those of trace_ray2: object-space
 // triangle tests with t unchanged, ties to the lower global primitive id,
 // candidate hits on non-opaque triangles decided with the world ray.
-// `finish(index, leaf, t, u, v, instance)`.
-template <bool kAnyHit, bool kOpacity, class Load, class Finish, class Seed>
+// The hit record carries the instance in place of u (`hit(index, leaf, t, instance bits, v)`).
+template <bool kOpacity, class Rays>
 __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
-                                             const float* __restrict__ mat_tr, uint32_t n, uint32_t* work, Load load,
-                                             Finish finish, Seed seed, int postpone_sp, int refill_min) {
+                                             const float* __restrict__ mat_tr, uint32_t n, uint32_t* work,
+                                             const Rays& rays, int postpone_sp, int refill_min) {
     postpone_sp = postpone_sp < kPostponeMaxSp ? postpone_sp : kPostponeMaxSp;
     const uint32_t lane = threadIdx.x & 31u;
     bool has = false;
     bool exhausted = false;  // warp-uniform
     RayPre r;
-    float tbest = 0.0f, bu = 0.0f, bv = 0.0f;
-    uint32_t best_leaf = kMissPrim, best_prim = kMissPrim, best_inst = kMissPrim, idx = 0;
+    float tbest = 0.0f;
+    uint32_t best_prim = kMissPrim, idx = 0;
     const CwNode* nodes = tlas;
     const CwTri* tris = nullptr;   // nullptr: traversing the TLAS
     uint32_t inst = kMissPrim, prim_base = 0u, mat_override = kMissPrim;
@@ -595,14 +600,14 @@ __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, co
                 uint32_t i = base + (uint32_t)__popc(idle & lanemask_lt());
                 if (i < n) {
                     float4 o, d;
-                    load(i, o, d);
+                    rays.load(i, o, d);
                     r = make_ray(o, d);
                     s_world[threadIdx.x][0] = make_float4(
                         r.idx, r.idy, r.idz,
                         __uint_as_float(r.oct_key | ((uint32_t)r.kx << 4) | ((uint32_t)r.ky << 8) | ((uint32_t)r.kz << 12)));
                     s_world[threadIdx.x][1] = make_float4(r.Sx, r.Sy, r.Sz, 0.0f);
                     tbest = d.w;
-                    best_leaf = kMissPrim; best_prim = kMissPrim; best_inst = kMissPrim; bu = 0.0f; bv = 0.0f;
+                    best_prim = kMissPrim;
                     nodes = tlas; tris = nullptr; inst = kMissPrim; prim_base = 0u; mat_override = kMissPrim;
                     G = make_uint2(0u, ray_traceable(r, d.w) ? (0x80000000u | (1u << (7u ^ r.oct_key))) : 0u);
                     T = make_uint2(0u, 0u);
@@ -674,25 +679,26 @@ __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, co
                     float tr = mat_tr[mat_override != kMissPrim ? mat_override : __float_as_uint(b.w)];
                     if (tr != 0.0f) {   // the rule reads the world ray
                         float4 o4, d4;
-                        load(idx, o4, d4);
-                        keep = keep_hit(make_ray(o4, d4), tr, seed(idx));
+                        rays.load(idx, o4, d4);
+                        keep = keep_hit(make_ray(o4, d4), tr, rays.seed(idx));
                     }
                 }
                 if (keep) {
-                    tbest = t; best_leaf = ti; best_prim = prim; best_inst = inst; bu = u; bv = v;
-                    if (kAnyHit) { T.y = 0u; G.y = 0u; sp = 0; }
+                    tbest = t;
+                    best_prim = prim;
+                    rays.hit(idx, ti, t, __uint_as_float(inst), v);
+                    if (rays.any(idx)) { T.y = 0u; G.y = 0u; sp = 0; }
                 }
             }
         }
         // next group, or done
         if (has && (G.y & 0xff000000u) == 0u && !has_tris(T)) {
-            const bool done = kAnyHit && best_leaf != kMissPrim;
             uint2 e = make_uint2(0u, 0u);
-            if (!done && sp > 0) {
+            if (sp > 0) {
                 e = stack[--sp];
                 if (e.y == 0u) {  // exit marker: back to the world ray and the TLAS
                     float4 o4, d4, c0 = s_world[threadIdx.x][0], c1 = s_world[threadIdx.x][1];
-                    load(idx, o4, d4);
+                    rays.load(idx, o4, d4);
                     const uint32_t pk = __float_as_uint(c0.w);
                     r.ox = o4.x; r.oy = o4.y; r.oz = o4.z; r.tmin = o4.w;
                     r.dx = d4.x; r.dy = d4.y; r.dz = d4.z;
@@ -708,7 +714,7 @@ __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, co
             if (e.y != 0u) {
                 G = e;
             } else {
-                finish(idx, best_leaf, tbest, bu, bv, best_inst);
+                if (best_prim == kMissPrim) rays.miss(idx, tbest);
                 has = false;
             }
         }
