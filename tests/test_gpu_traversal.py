@@ -1,0 +1,66 @@
+"""The traversal kernels against the oracle where their shortcuts could go wrong: exact zeros on edges and
+vertices for every dominant axis and sign of the direction."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def cube_scene(bsm, n=4):
+    """The surface of the cube [-2, 2]^3, n x n squares a side with alternating diagonals and windings."""
+    P, idx = [], []
+    for axis in range(3):
+        for side in (-2.0, 2.0):
+            base = len(P)
+            for i in range(n + 1):
+                for j in range(n + 1):
+                    p = [0.0, 0.0, 0.0]
+                    p[axis], p[(axis + 1) % 3], p[(axis + 2) % 3] = side, -2.0 + 4.0 * i / n, -2.0 + 4.0 * j / n
+                    P.append(p)
+            for i in range(n):
+                for j in range(n):
+                    a, b = base + i * (n + 1) + j, base + (i + 1) * (n + 1) + j
+                    quad = [(a, b, b + 1), (a, b + 1, a + 1)] if (i + j) % 2 else [(a, a + 1, b), (b + 1, b, a + 1)]
+                    idx += quad
+    mats = np.array([[0.5, 0.5, 0.5, 0.5, 0.0]], np.float32)
+    lights = np.array([[0.3, 0.4, -1.0, 2.0, 2.0, 2.0]], np.float32)
+    cam = bsm.make_camera((0.5, 0.5, -1.0), (0.0, 0.0, 1.0), yfov_deg=40.0, width=16, height=16)
+    return bsm.SceneData(np.array(P, np.float32), np.array(idx, np.uint32), np.zeros(len(idx), np.uint32), mats, lights,
+                         bsm.BSM_SKY_CONSTANT, (0.3, 0.3, 0.3), None, cam)
+
+
+def lattice_rays(tmin):
+    """From lattice points inside the cube through its vertices, edge midpoints and face centres (every edge
+    function there is exactly zero or exact in float32), and along the axes."""
+    pts = np.array([[x, y, z] for x in (-1, 0, 0.5) for y in (0, 1, -0.5) for z in (-1, 0, 1)], np.float32)
+    half = np.arange(-4, 5, dtype=np.float32) * 0.5
+    to = []
+    for axis in range(3):
+        for side in (-2.0, 2.0):
+            for u in half:
+                for v in half:
+                    p = np.zeros(3, np.float32)
+                    p[axis], p[(axis + 1) % 3], p[(axis + 2) % 3] = side, u, v
+                    to.append(p)
+    to = np.array(to)
+    o = np.repeat(pts, len(to), 0)
+    d = np.tile(to, (len(pts), 1)) - o
+    rays = np.concatenate([o, np.full((len(o), 1), tmin, np.float32), d, np.full((len(o), 1), 4.0, np.float32)], 1)
+    axes = np.concatenate([np.eye(3), -np.eye(3)]).astype(np.float32)
+    ax = np.concatenate([np.repeat(pts, 6, 0), np.full((len(pts) * 6, 1), tmin, np.float32), np.tile(axes, (len(pts), 1)),
+                         np.full((len(pts) * 6, 1), 9.0, np.float32)], 1)
+    surface = np.concatenate([to, np.full((len(to), 1), tmin, np.float32), to[::-1] * 0.25 + 0.125,
+                              np.full((len(to), 1), 9.0, np.float32)], 1)   # origins on the surface: t = 0 hits
+    return np.ascontiguousarray(np.concatenate([rays, ax, surface]), np.float32)
+
+
+@pytest.mark.parametrize("tmin", [0.0, -0.125])   # the second also takes hits at t = 0, all of which are zeros
+def test_exact_zeros_match_the_oracle_bit_for_bit(bsm, ctx, oracle, tmin):
+    sc = cube_scene(bsm)
+    sid = ctx.load_scene(sc)
+    rays = lattice_rays(tmin)
+    g, c = ctx.trace_closest(sid, rays), oracle.OracleScene(sc).trace(rays)
+    assert (c[:, 1] != 0xFFFFFFFF).sum() > 1000
+    bad = np.argwhere(g != c)
+    assert bad.size == 0, f"{len(bad)} words differ, first ray {rays[bad[0, 0]].tolist()}: {g[bad[0, 0]]} {c[bad[0, 0]]}"
+    ctx.release(sid)
