@@ -32,7 +32,7 @@
 
 namespace bsm {
 
-// Far-plane pad: a box is kept when max(near) <= min(far) * (1 + 2^-20).  The
+// Far-plane pad: a box is kept when max(near) <= min(far, t_best) * (1 + 2^-20).  The
 // builder also pads every child box outward by one quantisation step, so the
 // rounding of the slab arithmetic never culls a box that holds a hit.
 #define BSM_BOX_PAD 1.00000095f
@@ -215,7 +215,24 @@ __device__ __forceinline__ float qbyte(uint32_t w, uint32_t k) {
     return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u | k));
 }
 
-// Intersects the eight children of node `ni`; returns the group of internal
+// (q0 s + a, q1 s + a) in one instruction, each rounded as __fmaf_rn: a child's
+// near and far plane of one axis.
+__device__ __forceinline__ void fma2(float q0, float q1, float s, float a, float& t0, float& t1) {
+    asm("{.reg .b64 q, s, a, t;\n\tmov.b64 q, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\tmov.b64 a, {%5, %5};\n\t"
+        "fma.rn.f32x2 t, q, s, a;\n\tmov.b64 {%0, %1}, t;}"
+        : "=f"(t0), "=f"(t1) : "f"(q0), "f"(q1), "f"(s), "f"(a));
+}
+
+// Intersects the eight children of node `ni`.  The traversal loop is bound by
+// instruction issue (0.8 of the issue slots) and most of what it issues is this
+// function, so it is written for few instructions: one packed multiply-add per
+// child and axis, which works within 64 registers because near and far planes
+// share their constants (the pad multiplies the far distance in the comparison,
+// as one more multiply-add, instead of six constants), and the comparison's
+// sign shifted into the miss mask instead of compared, selected and merged.
+// 1080p 64-spp terrain 169.5 -> 160.8 ms against separate pads, comparisons and
+// single multiply-adds (of which the mask by signs gave 3.4 ms).
+// Returns the group of internal
 // children hit (child base, hit bits 24..31 in octant order | imask) and the
 // group of triangles hit (triangle base, hit bits 0..15 | the node's
 // tri_mask in bits 16..31, which locates each triangle: next_tri).
@@ -224,7 +241,7 @@ __device__ __forceinline__ void node_test(const RayPre& r, const CwNode* __restr
     const uint4* p = reinterpret_cast<const uint4*>(nodes + ni);
     uint4 n0 = __ldg(p + 0), n1 = __ldg(p + 1), n2 = __ldg(p + 2), n3 = __ldg(p + 3), n4 = __ldg(p + 4);
     uint32_t ew = n0.w;
-    // slab distance of plane q: q * s + a (near planes) and (q * s + a) * pad (far planes)
+    // slab distance of plane q: q * s + a
     float sx = __uint_as_float((ew & 0xffu) << 23) * r.idx;
     float sy = __uint_as_float(((ew >> 8) & 0xffu) << 23) * r.idy;
     float sz = __uint_as_float(((ew >> 16) & 0xffu) << 23) * r.idz;
@@ -234,8 +251,7 @@ __device__ __forceinline__ void node_test(const RayPre& r, const CwNode* __restr
     ax = __fsub_rn(ax, 8388608.0f * sx);
     ay = __fsub_rn(ay, 8388608.0f * sy);
     az = __fsub_rn(az, 8388608.0f * sz);
-    float sxf = sx * BSM_BOX_PAD, syf = sy * BSM_BOX_PAD, szf = sz * BSM_BOX_PAD;
-    float axf = ax * BSM_BOX_PAD, ayf = ay * BSM_BOX_PAD, azf = az * BSM_BOX_PAD;
+    const float tb = fmaxf(tbest, tbest * 0.9999981f);   // a negative bound moves up by more than the pad below takes off
     uint32_t imask = ew >> 24;
     bool nx = r.idx < 0.0f, ny = r.idy < 0.0f, nz = r.idz < 0.0f;
     uint32_t nlx0 = nx ? n3.z : n2.x, nlx1 = nx ? n3.w : n2.y;
@@ -244,21 +260,20 @@ __device__ __forceinline__ void node_test(const RayPre& r, const CwNode* __restr
     uint32_t nfy0 = ny ? n2.z : n4.x, nfy1 = ny ? n2.w : n4.y;
     uint32_t nlz0 = nz ? n4.z : n3.x, nlz1 = nz ? n4.w : n3.y;
     uint32_t nfz0 = nz ? n3.x : n4.z, nfz1 = nz ? n3.y : n4.w;
-    uint32_t hm = 0;
+    uint32_t miss = 0;   // bit c: child c is missed (the sign of far - near; a NaN keeps the child)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 7; c >= 0; --c) {
         const uint32_t k = (uint32_t)(c & 3);
         const bool lo = c < 4;
-        float tnx = __fmaf_rn(qbyte(lo ? nlx0 : nlx1, k), sx, ax);
-        float tny = __fmaf_rn(qbyte(lo ? nly0 : nly1, k), sy, ay);
-        float tnz = __fmaf_rn(qbyte(lo ? nlz0 : nlz1, k), sz, az);
-        float tfx = __fmaf_rn(qbyte(lo ? nfx0 : nfx1, k), sxf, axf);
-        float tfy = __fmaf_rn(qbyte(lo ? nfy0 : nfy1, k), syf, ayf);
-        float tfz = __fmaf_rn(qbyte(lo ? nfz0 : nfz1, k), szf, azf);
+        float tnx, tny, tnz, tfx, tfy, tfz;
+        fma2(qbyte(lo ? nlx0 : nlx1, k), qbyte(lo ? nfx0 : nfx1, k), sx, ax, tnx, tfx);
+        fma2(qbyte(lo ? nly0 : nly1, k), qbyte(lo ? nfy0 : nfy1, k), sy, ay, tny, tfy);
+        fma2(qbyte(lo ? nlz0 : nlz1, k), qbyte(lo ? nfz0 : nfz1, k), sz, az, tnz, tfz);
         float tn = max3f(tnx, tny, fmaxf(tnz, r.tmin));
-        float tf = min3f(tfx, tfy, fminf(tfz, tbest));
-        hm |= (tn <= tf) ? (1u << c) : 0u;
+        float tf = min3f(tfx, tfy, fminf(tfz, tb));
+        miss = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, BSM_BOX_PAD, -tn)), miss, 1);
     }
+    const uint32_t hm = ~miss & 0xffu;
     // hit slots that are empty have neither an imask nor a tri_mask bit, so they drop out here
     uint32_t inner = __ldg(&g_child_perm.v[r.oct_key * 256u + (hm & imask)]);
     uint32_t tm = n1.z & 0xffffu;

@@ -1528,9 +1528,10 @@ ORC_API int orc_light_eval(const float* row, const float* P, const float* u, uin
 // Arithmetic, in this order, as the device kernel evaluates it: per axis the
 // slab scale s = 2^(e-127) / d and offset a = (p - o) / d - 2^23 s (a component
 // d below 1e-20 in magnitude taken as +-1e-20, as the device does); the plane
-// of byte q is at fma(2^23 + q, s, a) (near) or fma(2^23 + q, s PAD, a PAD)
-// (far), PAD = 1.00000095; a child is hit when max(near x/y/z, tmin) <=
-// min(far x/y/z, t_best).  Children are visited nearest-octant first
+// of byte q is at fma(2^23 + q, s, a); with tn = max(near x/y/z, tmin) and
+// tf = min(far x/y/z, t_best) a child is missed when fma(tf, PAD, -tn) is
+// negative, PAD = 1.00000095 (a negative t_best is first moved up by 1.9e-6 of
+// itself, since the pad moves it down).  Children are visited nearest-octant first
 // (descending slot ^ (7 ^ octant)), the hit triangles in ascending index,
 // all of a node's triangles before its next child.
 namespace orc {
@@ -1553,14 +1554,13 @@ static float pow2_biased(uint8_t e) { uint32_t u = (uint32_t)e << 23; float f; s
 static uint32_t cw_node_hits(const Ray& r, const CwNodeO& n, uint32_t key, float tbest) {
     const float PAD = 1.00000095f;
     float o[3] = {r.o.x, r.o.y, r.o.z};
-    float s[3], a[3], sf[3], af[3];
+    float s[3], a[3];
     for (int k = 0; k < 3; ++k) {
         s[k] = pow2_biased(n.e[k]) * r.idc[k];
         a[k] = (n.p[k] - o[k]) * r.idc[k];
         a[k] = a[k] - 8388608.0f * s[k];
-        sf[k] = s[k] * PAD;
-        af[k] = a[k] * PAD;
     }
+    const float tb = std::fmax(tbest, tbest * 0.9999981f);
     uint32_t hits = 0;
     for (int c = 0; c < 8; ++c) {
         bool inner = (n.imask >> c) & 1u;
@@ -1572,11 +1572,12 @@ static uint32_t cw_node_hits(const Ray& r, const CwNodeO& n, uint32_t key, float
             float qn = 8388608.0f + (float)(neg ? n.qhi[k][c] : n.qlo[k][c]);
             float qf = 8388608.0f + (float)(neg ? n.qlo[k][c] : n.qhi[k][c]);
             tnear[k] = std::fmaf(qn, s[k], a[k]);
-            tfar[k] = std::fmaf(qf, sf[k], af[k]);
+            tfar[k] = std::fmaf(qf, s[k], a[k]);
         }
         float tn = std::fmax(std::fmax(tnear[0], tnear[1]), std::fmax(tnear[2], r.tmin));
-        float tf = std::fmin(std::fmin(tfar[0], tfar[1]), std::fmin(tfar[2], tbest));
-        if (!(tn <= tf)) continue;
+        float tf = std::fmin(std::fmin(tfar[0], tfar[1]), std::fmin(tfar[2], tb));
+        const float d = std::fmaf(tf, PAD, -tn);
+        if (std::signbit(d) && !std::isnan(d)) continue;   // the device's NaN has no sign: the child is kept
         if (inner) hits |= 1u << (24 + ((uint32_t)c ^ key));
         else hits |= tm << (2 * c);
     }
