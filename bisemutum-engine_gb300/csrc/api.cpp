@@ -1369,11 +1369,11 @@ void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t 
         int q = 0;
         for (uint32_t seg = 0; seg < max_seg; ++seg) {
             if (count_traversal) launch_extend_count(lc, st, sc->dev, wf, q, seg);
-            else launch_trace(lc, st, sc->dev, wf, q, seg, split || seg == 0 ? kNoSegment : seg - 1, accum);
+            else launch_trace(lc, st, sc->dev, wf, q, seg, split || seg == 0 ? kNoSegment : seg - 1, accum, count);
             mark(1);
             launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, cache_wb != nullptr);
             mark(2);
-            if (split || seg + 1 == max_seg) launch_trace(lc, st, sc->dev, wf, q, kNoSegment, seg, accum);
+            if (split || seg + 1 == max_seg) launch_trace(lc, st, sc->dev, wf, q, kNoSegment, seg, accum, count);
             mark(3);
             q ^= 1;
         }

@@ -129,6 +129,7 @@ struct LaunchCfg {
     int grid_shade;
     int postpone_sp = 16;   // traversal stack budget for postponed triangle groups
     int refill_min = 8;     // idle lanes that trigger a warp refill
+    int grid_group;         // blocks of the traversal kernel for small chunks (eight lanes per ray)
     int regcap = 1;         // 1: traversal kernels compiled for 4 blocks of 256 (64 registers); the default
 };
 
@@ -149,9 +150,9 @@ void launch_camera(const LaunchCfg& lc, cudaStream_t st, const DevView* views, u
                    uint64_t path_begin, uint32_t path_count, const Wavefront& wf, uint32_t max_segments);
 // The extension rays of segment `ext` (queue q) and the shadow rays of segment `shd` in one launch; kNoSegment
 // leaves one kind out.  The two kinds are independent of each other: shading segment s queues both shd = s and
-// ext = s + 1.
+// ext = s + 1.  `paths` (the chunk's paths) bounds both queues and picks the kernel.
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
-                  uint32_t shd, float4* accum);
+                  uint32_t shd, float4* accum, uint32_t paths);
 // The extension rays of `seg` with the traversal counters of BSM_PT_COUNT_TRAVERSAL.
 void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
                          uint32_t seg);

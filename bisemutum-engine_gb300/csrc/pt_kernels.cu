@@ -247,6 +247,20 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_trace(const CwNode* __restr
     trace_queue<false, kOpacity>(nodes, tris, rays.n, rays.work(), rays, nullptr, a.postpone_sp, a.refill_min);
 }
 
+// k_trace for chunks of at most kGroupPaths paths: eight lanes per ray.  A
+// kernel of its own, because its loop in k_trace costs that one registers
+// (1080p 64-spp frame 160.8 -> 168.7 ms with both), and 80 registers are worth
+// more here than occupancy (64 of them spill: 443 against 377 us for a 128x128
+// 8-segment frame of the room; 96: 369, but slower from 256x256 on).
+template <bool kOpacity>
+__global__ void __launch_bounds__(kGroupBlock, 6) k_trace_group(const CwNode* __restrict__ nodes,
+                                                                const CwTri* __restrict__ tris,
+                                                                const __grid_constant__ TraceArgs a) {
+    __shared__ GroupStacks stacks;
+    const TraceRays rays = trace_rays(a);
+    trace_queue_group<kOpacity>(nodes, tris, rays.n, rays.work(), rays, stacks);
+}
+
 // The same for two-level scenes: trace_queue2 (TLAS leaves enter instances).
 // The hit record carries the instance in place of u.
 template <bool kOpacity>
@@ -684,8 +698,15 @@ void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const
     if (n) k_gather_normals<<<(n + 255) / 256, 256, 0, st>>>(tris, n, vn, idx, out);
 }
 
+// Chunks of at most this many paths (the queues of every segment are known only to the device) are traced with
+// eight lanes per ray.  Their launches are too short for the lane-per-ray loop's throughput to show: 8-segment
+// 1-spp frames of the room take 539 / 597 / 680 / 782 us lane by lane and 337 / 377 / 548 / 839 us in groups at
+// 64^2 / 128^2 / 256^2 / 362^2 pixels, of the 1.48 M-triangle terrain 806 / 909 / 1050 / 1184 and
+// 472 / 551 / 823 / 1222 us: the lines cross near 110,000 paths.
+constexpr uint32_t kGroupPaths = 98304;
+
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
-                  uint32_t shd, float4* accum) {
+                  uint32_t shd, float4* accum, uint32_t paths) {
     const bool op = sc.has_non_opaque != 0;
     const TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
                       wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u,
@@ -695,6 +716,11 @@ void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, cons
         else k_trace2<false><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
         return;
     }
+    if (paths <= kGroupPaths) {
+        if (op) k_trace_group<true><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        else k_trace_group<false><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        return;
+    }
 #define BSM_TRACE(B, O) k_trace<B, O><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc.nodes, sc.tris, a)
     if (lc.regcap) { if (op) BSM_TRACE(4, true); else BSM_TRACE(4, false); }
     else { if (op) BSM_TRACE(1, true); else BSM_TRACE(1, false); }
@@ -702,7 +728,7 @@ void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, cons
 }
 void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
                          uint32_t seg) {
-    if (sc.insts) { launch_trace(lc, st, sc, wf, q, seg, kNoSegment, nullptr); return; }   // counters: single-level only
+    if (sc.insts) { launch_trace(lc, st, sc, wf, q, seg, kNoSegment, nullptr, 0xffffffffu); return; }   // counters: single-level only
     const CountRays rays{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit};
     if (sc.has_non_opaque)
         k_extend_count<true><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc, rays, wf.counters, wf.stats, seg,
@@ -770,6 +796,9 @@ void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     if (per_sm < 1) per_sm = 1;
     if (per_sm_shade < 1) per_sm_shade = 1;
     lc->block_trace = block_trace;
+    int per_sm_group = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_group, k_trace_group<true>, kGroupBlock, 0);
+    lc->grid_group = sms * (per_sm_group < 1 ? 1 : per_sm_group);
     lc->grid_persistent = sms * per_sm;
     lc->block_shade = 512;   // the direction grouping of the next rays spans a block
     lc->grid_shade = sms * per_sm_shade * 4;

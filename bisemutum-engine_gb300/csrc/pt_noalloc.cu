@@ -205,11 +205,11 @@ extern "C" bsm_status bsm_render_noalloc(bsm_context* ctx, uint32_t scene_id, co
         launch_camera(lc, st, view_dev, 1, begin, count, wf, max_seg);
         int q = 0;
         for (uint32_t seg = 0; seg < max_seg; ++seg) {
-            launch_trace(lc, st, sc, wf, q, seg, seg ? seg - 1 : kNoSegment, accum);
+            launch_trace(lc, st, sc, wf, q, seg, seg ? seg - 1 : kNoSegment, accum, count);
             launch_shade(lc, st, sc, view_dev, wf, q, seg, accum);
             q ^= 1;
         }
-        launch_trace(lc, st, sc, wf, q, kNoSegment, max_seg - 1, accum);
+        launch_trace(lc, st, sc, wf, q, kNoSegment, max_seg - 1, accum, count);
     }
     k_noalloc_mean<<<(uint32_t)((npix + 255) / 256), 256, 0, st>>>(accum, (uint32_t)npix, 1.0f / (float)s->spp);
     NA_CK(cudaGetLastError());

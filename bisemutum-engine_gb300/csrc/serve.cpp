@@ -237,11 +237,11 @@ bool launch_chunk(Server& S, Lane& lane, uint32_t scene) {
     launch_camera(S.lc, st, lane.views_dev, (uint32_t)lane.ranges.size(), 0, (uint32_t)base, lane.wf, max_seg);
     int q = 0;
     for (uint32_t seg = 0; seg < max_seg; ++seg) {
-        launch_trace(S.lc, st, sc, lane.wf, q, seg, seg ? seg - 1 : kNoSegment, S.pool_mem);
+        launch_trace(S.lc, st, sc, lane.wf, q, seg, seg ? seg - 1 : kNoSegment, S.pool_mem, (uint32_t)base);
         launch_shade(S.lc, st, sc, lane.views_dev, lane.wf, q, seg, S.pool_mem);
         q ^= 1;
     }
-    launch_trace(S.lc, st, sc, lane.wf, q, kNoSegment, max_seg - 1, S.pool_mem);
+    launch_trace(S.lc, st, sc, lane.wf, q, kNoSegment, max_seg - 1, S.pool_mem, (uint32_t)base);
     size_t li = &lane - S.lanes.data();
     cudaMemcpyAsync(S.stats_host + li * kStatWords, lane.wf.stats, kStatWords * 8, cudaMemcpyDeviceToHost, st);
     cudaEventRecord(lane.ev, st);

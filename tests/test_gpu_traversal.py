@@ -1,7 +1,11 @@
 """The traversal kernels against the oracle where their shortcuts could go wrong: exact zeros on edges and
-vertices for every dominant axis and sign of the direction."""
+vertices for every dominant axis and sign of the direction; frames on both sides of the chunk size at which the
+kernel with eight lanes per ray hands over to the one with a lane per ray (98,304 paths), with and without
+non-opaque materials."""
 import numpy as np
 import pytest
+
+from conftest import assert_bits_equal
 
 pytestmark = pytest.mark.gpu
 
@@ -63,4 +67,19 @@ def test_exact_zeros_match_the_oracle_bit_for_bit(bsm, ctx, oracle, tmin):
     assert (c[:, 1] != 0xFFFFFFFF).sum() > 1000
     bad = np.argwhere(g != c)
     assert bad.size == 0, f"{len(bad)} words differ, first ray {rays[bad[0, 0]].tolist()}: {g[bad[0, 0]]} {c[bad[0, 0]]}"
+    ctx.release(sid)
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (9, 3, 1), (384, 256, 1), (385, 256, 1), (128, 96, 9)])
+@pytest.mark.parametrize("opaque", [True, False])
+def test_both_sides_of_the_group_kernel_limit(bsm, ctx, oracle, w, h, spp, opaque):
+    sc = bsm.generate_scene(bsm.BSM_SCENE_ROOM, seed=11, width=w, height=h)
+    if not opaque:
+        sc.materials[1::2, 5], sc.materials[1::2, 6] = 0.6, bsm.BSM_BLEND_TRANSLUCENT
+    sid = ctx.load_scene(sc)
+    det = bsm.BSM_PT_DETERMINISTIC
+    imgs, st = ctx.render(sid, [sc.camera], bsm.settings(spp=spp, max_segments=4, seed=5, flags=det))
+    ref, ost, _ = oracle.OracleScene(sc).render(sc.camera.as_array(), spp=spp, max_segments=4, seed=5, flags=det)
+    assert list(st.rays_per_segment[:4]) == [int(x) for x in ost[:4]]
+    assert_bits_equal(imgs[0][..., :3], ref[..., :3])
     ctx.release(sid)
