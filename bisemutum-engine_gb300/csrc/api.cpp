@@ -2003,12 +2003,12 @@ extern "C" bsm_status bsm_render_primary(bsm_context* ctx, uint32_t scene_id, co
     } else {
         size_t total = 0;
         for (int k = 0; k < 6; ++k)
-            if (dst[k]) total += bytes[k];
+            if (dst[k]) total += (bytes[k] + 15) & ~(size_t)15;
         if (total == 0) return BSM_OK;
         if ((st = dev_alloc(ctx, ctx->tmp, total))) return st;
         char* b = (char*)ctx->tmp.ptr;
         for (int k = 0; k < 6; ++k)
-            if (dst[k]) { dev[k] = (float*)b; b += bytes[k]; }
+            if (dst[k]) { dev[k] = (float*)b; b += (bytes[k] + 15) & ~(size_t)15; }   // float4 arrays follow
     }
     float4* gb[4] = {(float4*)dev[1], (float4*)dev[2], (float4*)dev[3], (float4*)dev[4]};
     launch_primary(WS(ctx), sc->dev, v, near_z, far_z, dev[0], gb, (float4*)dev[5]);
