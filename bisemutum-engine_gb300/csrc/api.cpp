@@ -79,6 +79,8 @@ struct ViewHist {
     bool valid = false;
 };
 
+constexpr uint32_t kStageSlots = 1024;
+
 struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     std::vector<uint8_t> key;
@@ -118,6 +120,10 @@ struct bsm_context {
     std::vector<std::pair<uint32_t, uint32_t>> layout;  // (width, height) per view
     DevBuf out_stage;             // device staging for host outputs
     DevBuf tmp;                   // stage entry points (host buffers)
+    // their kernels' work counters: kStageSlots pairs of words, zero between launches, one pair per launch in
+    // turn, so that a launch captured into a caller's graph does not share its pair with the calls around it
+    uint32_t* stage_work = nullptr;
+    uint32_t stage_slot = 0;
     std::vector<GraphEntry> graphs;
     cudaEvent_t ev[16] = {};
     std::vector<cudaEvent_t> stage_ev;
@@ -410,6 +416,15 @@ extern "C" bsm_status bsm_create(bsm_context** out, int device, uint64_t budget)
     ctx->device = device;
     if (cudaSetDevice(device) != cudaSuccess) { delete ctx; return BSM_ERR_CUDA; }
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return BSM_ERR_CUDA; }
+    if (cudaMalloc((void**)&ctx->stage_work, kStageSlots * 8) != cudaSuccess ||
+        cudaMemsetAsync(ctx->stage_work, 0, kStageSlots * 8, ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ctx->stage_work);
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return BSM_ERR_OUT_OF_MEMORY;
+    }
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     ctx->budget = budget ? budget : (uint64_t)((double)fr * 0.9);
@@ -437,6 +452,7 @@ extern "C" void bsm_destroy(bsm_context* ctx) {
     dev_free(ctx, ctx->accum_fx);
     dev_free(ctx, ctx->out_stage);
     dev_free(ctx, ctx->tmp);
+    cudaFree(ctx->stage_work);
     for (auto& ev : ctx->ev) if (ev) cudaEventDestroy(ev);
     for (auto& ev : ctx->stage_ev) cudaEventDestroy(ev);
     cudaStreamDestroy(ctx->stream);
@@ -1888,6 +1904,8 @@ extern "C" bsm_status bsm_import_history(bsm_context* ctx, uint32_t view_index, 
 
 // ===================================================== stage entry points ====
 namespace {
+uint32_t* next_stage_work(bsm_context* ctx) { return ctx->stage_work + 2 * (ctx->stage_slot++ % kStageSlots); }
+
 bsm_status stage_prep(bsm_context* ctx, uint32_t scene_id, Scene** out) {
     if (!ctx) return BSM_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
@@ -1895,7 +1913,7 @@ bsm_status stage_prep(bsm_context* ctx, uint32_t scene_id, Scene** out) {
     if (!sc) return fail(ctx, BSM_ERR_NOT_FOUND, "unknown scene id");
     if (!sc->has_bvh) return fail(ctx, BSM_ERR_BAD_STATE, "scene BVH not built");
     *out = sc;
-    return BSM_OK;
+    return ctx->lc_block ? BSM_OK : ensure_launch_cfg(ctx, 0, 1);
 }
 }  // namespace
 
@@ -1907,7 +1925,7 @@ extern "C" bsm_status bsm_trace_closest(bsm_context* ctx, uint32_t scene_id, con
     if (n == 0) return BSM_OK;
     if (!rays || !hits) return BSM_ERR_INVALID_ARG;
     if (location == BSM_DEVICE) {
-        launch_trace_closest(WS(ctx), sc->dev, (const float4*)rays, n, (uint4*)hits, 128);
+        launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, (uint4*)hits, next_stage_work(ctx));
         CK(cudaGetLastError());
         return BSM_OK;   // queued on the work stream
     }
@@ -1915,7 +1933,7 @@ extern "C" bsm_status bsm_trace_closest(bsm_context* ctx, uint32_t scene_id, con
     if ((st = dev_alloc(ctx, ctx->tmp, rb + hb))) return st;
     char* b = (char*)ctx->tmp.ptr;
     CK(cudaMemcpyAsync(b, rays, rb, cudaMemcpyHostToDevice, WS(ctx)));
-    launch_trace_closest(WS(ctx), sc->dev, (const float4*)b, n, (uint4*)(b + rb), 128);
+    launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint4*)(b + rb), next_stage_work(ctx));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(hits, b + rb, hb, cudaMemcpyDeviceToHost, WS(ctx)));
     CK(cudaStreamSynchronize(WS(ctx)));
@@ -1930,7 +1948,7 @@ extern "C" bsm_status bsm_trace_any(bsm_context* ctx, uint32_t scene_id, const f
     if (n == 0) return BSM_OK;
     if (!rays || !occluded) return BSM_ERR_INVALID_ARG;
     if (location == BSM_DEVICE) {
-        launch_trace_any(WS(ctx), sc->dev, (const float4*)rays, n, occluded, 128);
+        launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, occluded, next_stage_work(ctx));
         CK(cudaGetLastError());
         return BSM_OK;   // queued on the work stream
     }
@@ -1938,7 +1956,7 @@ extern "C" bsm_status bsm_trace_any(bsm_context* ctx, uint32_t scene_id, const f
     if ((st = dev_alloc(ctx, ctx->tmp, rb + n + 16))) return st;
     char* b = (char*)ctx->tmp.ptr;
     CK(cudaMemcpyAsync(b, rays, rb, cudaMemcpyHostToDevice, WS(ctx)));
-    launch_trace_any(WS(ctx), sc->dev, (const float4*)b, n, (uint8_t*)(b + rb), 128);
+    launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint8_t*)(b + rb), next_stage_work(ctx));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(occluded, b + rb, n, cudaMemcpyDeviceToHost, WS(ctx)));
     CK(cudaStreamSynchronize(WS(ctx)));
@@ -2011,7 +2029,8 @@ extern "C" bsm_status bsm_render_primary(bsm_context* ctx, uint32_t scene_id, co
             if (dst[k]) { dev[k] = (float*)b; b += (bytes[k] + 15) & ~(size_t)15; }   // float4 arrays follow
     }
     float4* gb[4] = {(float4*)dev[1], (float4*)dev[2], (float4*)dev[3], (float4*)dev[4]};
-    launch_primary(WS(ctx), sc->dev, v, near_z, far_z, dev[0], gb, (float4*)dev[5]);
+    launch_primary(ctx->lc, WS(ctx), sc->dev, v, near_z, far_z, dev[0], gb, (float4*)dev[5],
+                   next_stage_work(ctx));
     CK(cudaGetLastError());
     if (out->location == BSM_DEVICE) return BSM_OK;   // queued on the work stream
     for (int k = 0; k < 6; ++k)

@@ -129,6 +129,7 @@ struct LaunchCfg {
     int grid_shade;
     int postpone_sp = 16;   // traversal stack budget for postponed triangle groups
     int refill_min = 8;     // idle lanes that trigger a warp refill
+    int grid_stage, grid_stage2;   // blocks of the stage entry points' kernels (one / two levels)
     int grid_group;         // blocks of the traversal kernel for small chunks (eight lanes per ray)
     int regcap = 1;         // 1: traversal kernels compiled for 4 blocks of 256 (64 registers); the default
 };
@@ -167,10 +168,11 @@ void launch_fold_fixed(cudaStream_t st, const unsigned long long* fx, float4* ac
 // fold into a cleared accumulator followed by launch_resolve)
 void launch_resolve_fixed(cudaStream_t st, const unsigned long long* fx, uint32_t width, uint32_t height,
                           float inv_spp, float4* out, uint32_t pitch_px);
-void launch_trace_closest(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint4* hits,
-                          int block);
-void launch_trace_any(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint8_t* occluded,
-                      int block);
+// Stage entry points; `work`: two device words that are zero, and are zero again when the launch is done.
+void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
+                          uint4* hits, uint32_t* work);
+void launch_trace_any(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
+                      uint8_t* occluded, uint32_t* work);
 void launch_trace_count(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint2* counts);
 // Vertex normals of every leaf triangle in leaf order (3 float4 each) from per-vertex normals (3 floats each,
 // indexed by `idx`, or a soup when idx is null); all pointers are device memory.
@@ -178,8 +180,9 @@ void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const
                            float4* out);
 void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box, uint32_t begin,
                        uint32_t end);
-void launch_primary(cudaStream_t st, const DevScene& sc, const DevView& v, float near_z, float far_z, float* depth,
-                    float4* const gb[4], float4* hitpos);
+// Traces the view's camera rays and writes the outputs that are not null (the hit records wait in one of them).
+void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView& v, float near_z,
+                    float far_z, float* depth, float4* const gb[4], float4* hitpos, uint32_t* work);
 // radiance cache: the network's tensor-core kernels (mlp_tc.cu; `err`: a device word that gets bit 1 if a
 // tensor-core wait timed out) and Adam (mlp.cu)
 cudaError_t launch_mlp_infer(int device, cudaStream_t st, const void* wb, const float4* queries, const uint32_t* count,

@@ -146,10 +146,10 @@ struct CountRays {
     float4* hits;
     __device__ __forceinline__ bool any(uint32_t) const { return false; }
     __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) const { o = ray_o[i]; d = ray_d[i]; }
-    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v) const {
+    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v, uint32_t) const {
         hits[i] = make_float4(t, __uint_as_float(leaf), u, v);
     }
-    __device__ __forceinline__ void miss(uint32_t i, float tmax) const { hit(i, kMissPrim, tmax, 0.0f, 0.0f); }
+    __device__ __forceinline__ void miss(uint32_t i, float tmax) const { hit(i, kMissPrim, tmax, 0.0f, 0.0f, kMissPrim); }
     __device__ __forceinline__ uint32_t seed(uint32_t i) const { return path[i].z; }   // the path's PCG32 word
 };
 template <bool kOpacity>
@@ -208,8 +208,9 @@ struct TraceRays {
         if (i < n_ext) { o = __ldg(a.ray_o + i); d = __ldg(a.ray_d + i); }
         else { const uint32_t k = slot(i); o = __ldg(a.sh_o + k); d = __ldg(a.sh_d + k); }
     }
-    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v) const {
-        if (i < n_ext) a.hit[i] = make_float4(t, __uint_as_float(leaf), u, v);
+    // the hit record of a two-level scene carries the instance in place of u
+    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v, uint32_t inst) const {
+        if (i < n_ext) a.hit[i] = make_float4(t, __uint_as_float(leaf), inst != kMissPrim ? __uint_as_float(inst) : u, v);
     }
     __device__ __forceinline__ void miss(uint32_t i, float tmax) const {
         if (i < n_ext) {
@@ -262,7 +263,6 @@ __global__ void __launch_bounds__(kGroupBlock, 6) k_trace_group(const CwNode* __
 }
 
 // The same for two-level scenes: trace_queue2 (TLAS leaves enter instances).
-// The hit record carries the instance in place of u.
 template <bool kOpacity>
 __global__ void __launch_bounds__(256, 4) k_trace2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
                                                    const float* __restrict__ mat_tr,
@@ -554,45 +554,113 @@ __global__ void k_gather_normals(const CwTri* __restrict__ tris, uint32_t n, con
 }
 
 // ------------------------------------------------------ stage entry points ----
-__global__ void __launch_bounds__(256) k_trace_closest(DevScene sc, const float4* __restrict__ rays, uint32_t n,
-                                                       uint4* __restrict__ hits) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 o = rays[2 * (size_t)i], d = rays[2 * (size_t)i + 1];
-    RayPre r = make_ray(o, d);
-    float t, u, v;
-    uint32_t inst;
-    uint32_t leaf = trace_scene<false>(sc, r, d.w, t, u, v, inst, 0u);
-    uint32_t prim = kMissPrim;
-    if (leaf != kMissPrim)
-        prim = inst != kMissPrim ? sc.insts[inst].prim_base + sc.insts[inst].tris[leaf].prim : sc.tris[leaf].prim;
-    hits[i] = make_uint4(__float_as_uint(t), prim, __float_as_uint(u), __float_as_uint(v));
+// Rays of the stage entry points (a caller's array) and of small views' primary
+// outputs (a pixel-centre camera ray per pixel), on the wavefront's loops.
+struct StageArgs {
+    const float4* rays;       // a caller's rays (origin/tmin, direction/tmax), or null: camera rays of `view`
+    uint4* hits;              // t, primitive id, u, v of each ray
+    uint8_t* occluded;        // or whether it hit anything
+    float4* rec;              // camera rays: hit records (t, leaf, u, v) for k_primary_rec
+    const CwTri* tris;        // for the primitive ids
+    const InstDev* insts;
+    uint32_t n;
+    uint32_t* work;           // [2], zero between launches
+    int postpone_sp, refill_min;
+    DevView view;
+};
+struct StageRays {
+    const StageArgs& a;
+    __device__ __forceinline__ bool any(uint32_t) const { return a.occluded != nullptr; }
+    __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) const {
+        if (a.rays) {
+            o = __ldg(a.rays + 2 * (size_t)i);
+            d = __ldg(a.rays + 2 * (size_t)i + 1);
+            return;
+        }
+        o = make_float4(a.view.pos[0], a.view.pos[1], a.view.pos[2], a.view.t_min);
+        const uint32_t py = i / a.view.width;
+        const V3 dw = camera_dir(a.view, i - py * a.view.width, py, 0.5f, 0.5f);
+        d = make_float4(dw.x, dw.y, dw.z, a.view.ray_length);
+    }
+    __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v, uint32_t inst) const {
+        if (a.hits) {
+            const uint32_t prim = inst != kMissPrim ? a.insts[inst].prim_base + a.insts[inst].tris[leaf].prim
+                                                    : a.tris[leaf].prim;
+            a.hits[i] = make_uint4(__float_as_uint(t), prim, __float_as_uint(u), __float_as_uint(v));
+        } else if (a.occluded) {
+            a.occluded[i] = 1;
+        } else {
+            a.rec[i] = make_float4(t, __uint_as_float(leaf), u, v);
+        }
+    }
+    __device__ __forceinline__ void miss(uint32_t i, float tmax) const {
+        if (a.hits) a.hits[i] = make_uint4(__float_as_uint(tmax), kMissPrim, 0u, 0u);
+        else if (a.occluded) a.occluded[i] = 0;
+        else a.rec[i] = make_float4(tmax, __uint_as_float(kMissPrim), 0.0f, 0.0f);
+    }
+    // opacity decisions: a caller's rays draw with seed 0, a pixel's with the camera-ray PCG word of sample 0 of
+    // an unjittered render
+    __device__ __forceinline__ uint32_t seed(uint32_t i) const {
+        if (a.rays) return 0u;
+        return (uint32_t)pcg_seed(path_initstate(a.view.seed, a.view.sample_offset, i), (uint64_t)i).state;
+    }
+};
+
+// The work counter goes back to zero when the launch's last block is done with it.
+__device__ __forceinline__ void stage_done(uint32_t* work) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(work + 1, 1u) == gridDim.x - 1u) { work[0] = 0u; work[1] = 0u; }
+    }
+}
+
+// The caller's rays run on the persistent loops: with a ray per thread to the
+// end, as before, every warp waited for its longest ray and the last rays of a
+// launch held whole blocks. Closest and any hit of 1,000,003 rays, 1.48 M
+// triangles: 1693 -> 854 us (of it 8 % from the node and triangle tests);
+// 4 M rays 6490 -> 2951 us; 300,000 rays in 1,000 instances 752 -> 411 us.
+template <bool kOpacity>
+__global__ void __launch_bounds__(128, 8) k_stage(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
+                                                  const __grid_constant__ StageArgs a) {
+    trace_queue<false, kOpacity>(nodes, tris, a.n, a.work, StageRays{a}, nullptr, a.postpone_sp, a.refill_min);
+    stage_done(a.work);
+}
+template <bool kOpacity>
+__global__ void __launch_bounds__(kGroupBlock, 6) k_stage_group(const CwNode* __restrict__ nodes,
+                                                                const CwTri* __restrict__ tris,
+                                                                const __grid_constant__ StageArgs a) {
+    __shared__ GroupStacks stacks;
+    trace_queue_group<kOpacity>(nodes, tris, a.n, a.work, StageRays{a}, stacks);
+    stage_done(a.work);
+}
+template <bool kOpacity>
+__global__ void __launch_bounds__(128, 8) k_stage2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
+                                                   const float* __restrict__ mat_tr,
+                                                   const __grid_constant__ StageArgs a) {
+    trace_queue2<kOpacity>(tlas, insts, mat_tr, a.n, a.work, StageRays{a}, a.postpone_sp, a.refill_min);
+    stage_done(a.work);
 }
 
 // ------------------------------------------------------ primary outputs ----
-// One pixel-centre camera ray per pixel and its closest hit, as the reference's
-// first trace of a frame (generate_camera_ray.hlsl:9-15, rt_gbuffer.hlsl:7-36),
-// written as the pass's primary-hit outputs: reverse-Z depth (pt_depth.hlsl:7-16),
-// the packed G-buffer (gbuffer.hlsl:18-31) and hit positions.  The normal is the
-// geometric one faced towards the ray (as k_shade), the tangent the triangle's
-// first edge.  A miss writes depth 0, hit position (direction, -1) and a zero
-// G-buffer.  Outputs are tightly packed width*height arrays; any may be null.
-__global__ void __launch_bounds__(256) k_primary(DevScene sc, DevView v, float near_z, float far_z,
-                                                 float* __restrict__ depth, float4* __restrict__ gb0,
-                                                 float4* __restrict__ gb1, float4* __restrict__ gb2,
-                                                 float4* __restrict__ gb3, float4* __restrict__ hitpos) {
-    uint32_t npix = v.width * v.height;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
-    uint32_t px = i % v.width, py = i / v.width;
-    V3 dw = camera_dir(v, px, py, 0.5f, 0.5f);
-    V3 eye = v3(v.pos[0], v.pos[1], v.pos[2]);
-    RayPre r = make_ray(make_float4(eye.x, eye.y, eye.z, v.t_min), make_float4(dw.x, dw.y, dw.z, v.ray_length));
-    float t, hu, hv;
-    // opacity decisions of sample 0 of an unjittered render (its camera-ray PCG word)
-    Pcg pg = pcg_seed(path_initstate(v.seed, v.sample_offset, i), (uint64_t)i);
-    uint32_t inst;
-    uint32_t leaf = trace_scene<false>(sc, r, v.ray_length, t, hu, hv, inst, (uint32_t)pg.state);
+// The primary-hit outputs of the pass: one pixel-centre camera ray per pixel and
+// its closest hit, as the reference's first trace of a frame
+// (generate_camera_ray.hlsl:9-15, rt_gbuffer.hlsl:7-36), written as reverse-Z
+// depth (pt_depth.hlsl:7-16), the packed G-buffer (gbuffer.hlsl:18-31) and hit
+// positions.  The normal is the geometric one faced towards the ray (as
+// k_shade), the tangent the triangle's first edge.  A miss writes depth 0, hit
+// position (direction, -1) and a zero G-buffer.  Outputs are tightly packed
+// width*height arrays; any may be null.
+struct PrimaryOut {
+    float* depth;
+    float4* gb[4];
+    float4* hitpos;
+    float near_z, far_z;
+};
+// Writes pixel i's outputs for its hit (leaf, t, u, v, instance).
+__device__ __forceinline__ void write_primary(const DevScene& sc, const DevView& v, const PrimaryOut& out, uint32_t i,
+                                              V3 dw, uint32_t leaf, float t, float hu, float hv, uint32_t inst) {
+    const V3 eye = v3(v.pos[0], v.pos[1], v.pos[2]);
     float g[16];
     float z = 0.0f;
     float4 hp;
@@ -613,27 +681,53 @@ __global__ void __launch_bounds__(256) k_primary(DevScene sc, DevView v, float n
         float4 m0 = sc.materials[2 * mi], m1 = sc.materials[2 * mi + 1];
         pack_gbuffer(ng, T, v3(m0.x, m0.y, m0.z), v3(m1.x, m1.y, m1.z), m0.w, g);
         V3 P = eye + dw * t;
-        z = reverse_z_depth(eye, v3(v.f[0], v.f[1], v.f[2]), P, near_z, far_z);
+        z = reverse_z_depth(eye, v3(v.f[0], v.f[1], v.f[2]), P, out.near_z, out.far_z);
         hp = make_float4(P.x, P.y, P.z, t);
     }
-    if (depth) depth[i] = z;
-    if (gb0) gb0[i] = make_float4(g[0], g[1], g[2], g[3]);
-    if (gb1) gb1[i] = make_float4(g[4], g[5], g[6], g[7]);
-    if (gb2) gb2[i] = make_float4(g[8], g[9], g[10], g[11]);
-    if (gb3) gb3[i] = make_float4(g[12], g[13], g[14], g[15]);
-    if (hitpos) hitpos[i] = hp;
+    if (out.depth) out.depth[i] = z;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (out.gb[k]) out.gb[k][i] = make_float4(g[4 * k], g[4 * k + 1], g[4 * k + 2], g[4 * k + 3]);
+    if (out.hitpos) out.hitpos[i] = hp;
+}
+// Seed of a pixel's opacity decisions: sample 0 of an unjittered render (its camera-ray PCG word).
+__device__ __forceinline__ uint32_t primary_seed(const DevView& v, uint32_t i) {
+    return (uint32_t)pcg_seed(path_initstate(v.seed, v.sample_offset, i), (uint64_t)i).state;
 }
 
-__global__ void __launch_bounds__(256) k_trace_any(DevScene sc, const float4* __restrict__ rays, uint32_t n,
-                                                   uint8_t* __restrict__ occluded) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 o = rays[2 * (size_t)i], d = rays[2 * (size_t)i + 1];
-    RayPre r = make_ray(o, d);
-    float t, u, v;
-    uint32_t inst;
-    uint32_t leaf = trace_scene<true>(sc, r, d.w, t, u, v, inst, 0u);
-    occluded[i] = leaf == kMissPrim ? 0 : 1;
+// One pixel per lane, eight by four pixels per warp, sixteen by eight per block.
+// The camera rays of such a tile visit nearly the same nodes, so a lane's own
+// loop with neither queue nor refills is the fastest here, at 64 registers, and
+// the outputs leave in whole sectors.  1920x1080 of the 1.48 M-triangle terrain:
+// 831 us with a row of pixels per warp, 637 in tiles, 608 in tiles at 64
+// registers (691 with the queue loop's postponed triangles, 748 as hit records
+// from the persistent loop and a second kernel).
+template <bool kTwoLevel>
+__global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_primary(DevScene sc, const __grid_constant__ DevView v,
+                                                                    PrimaryOut out) {
+    const uint32_t across = (v.width + 15u) / 16u, ty = blockIdx.x / across, tx = blockIdx.x - ty * across;
+    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u;
+    const uint32_t px = tx * 16u + (w & 1u) * 8u + (l & 7u), py = ty * 8u + (w >> 1) * 4u + (l >> 3);
+    if (px >= v.width || py >= v.height) return;
+    const uint32_t i = py * v.width + px;
+    const V3 dw = camera_dir(v, px, py, 0.5f, 0.5f);
+    RayPre r = make_ray(make_float4(v.pos[0], v.pos[1], v.pos[2], v.t_min), make_float4(dw.x, dw.y, dw.z, v.ray_length));
+    float t, hu, hv;
+    uint32_t inst = kMissPrim, leaf;
+    const uint32_t seed = sc.has_non_opaque ? primary_seed(v, i) : 0u;
+    if (kTwoLevel) leaf = trace_ray2<false>(r, v.ray_length, sc.nodes, sc.insts, sc.mat_tr, t, hu, hv, inst, seed);
+    else leaf = trace_ray<false, false>(r, v.ray_length, sc.nodes, sc.tris, t, hu, hv, nullptr, seed);
+    write_primary(sc, v, out, i, dw, leaf, t, hu, hv, inst);
+}
+// Small views, from the hit records that k_stage_group left in one of the outputs.
+__global__ void __launch_bounds__(128) k_primary_rec(DevScene sc, const __grid_constant__ DevView v, PrimaryOut out,
+                                                     const float4* rec) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= v.width * v.height) return;
+    const float4 h = rec[i];
+    const uint32_t py = i / v.width;
+    write_primary(sc, v, out, i, camera_dir(v, i - py * v.width, py, 0.5f, 0.5f), __float_as_uint(h.y), h.x, h.z, h.w,
+                  kMissPrim);
 }
 
 __global__ void __launch_bounds__(256) k_trace_count(DevScene sc, const float4* __restrict__ rays, uint32_t n,
@@ -758,21 +852,75 @@ void launch_fold_fixed(cudaStream_t st, const unsigned long long* fx, float4* ac
     if (n == 0) return;
     k_fold_fixed<<<(unsigned)(((uint64_t)n + 255) / 256), 256, 0, st>>>(fx, accum, n);
 }
-void launch_trace_closest(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint4* hits,
-                          int block) {
-    if (n == 0) return;
-    k_trace_closest<<<(n + block - 1) / block, block, 0, st>>>(sc, rays, n, hits);
+// Calls of at most this many rays are traced with eight lanes per ray. Closest and any hit of half-random rays
+// take 76 / 103 us in groups and 115 / 152 lane by lane at 16,384 rays (room / 1.48 M triangles), 177 / 235 and
+// 132 / 194 us at 65,536.
+constexpr uint32_t kGroupRays = 40000;
+// Views of at most this many pixels take that way too, their hit records waiting in one of the outputs for
+// k_primary_rec: 35 / 58 us against 37 / 113 us in k_primary at 128x128 (room / 1.48 M triangles); at 230x170
+// 48 / 86 against 41 / 111.
+constexpr uint32_t kGroupPixels = 24576;
+
+static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, StageArgs& a) {
+    a.tris = sc.tris;
+    a.insts = sc.insts;
+    a.postpone_sp = 16;
+    a.refill_min = 8;
+    const bool op = sc.has_non_opaque != 0;
+    const bool few = !sc.insts && a.n <= kGroupRays;
+    const uint32_t per_block = few ? 128u / kGroupLanes : 128u;
+    const uint32_t full = sc.insts ? lc.grid_stage2 : few ? lc.grid_group : lc.grid_stage;
+    const uint32_t grid = min(full, (uint32_t)(((uint64_t)a.n + per_block - 1) / per_block));
+    if (sc.insts) {
+        if (op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+    } else if (few) {
+        if (op) k_stage_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        else k_stage_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+    } else {
+        if (op) k_stage<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+        else k_stage<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    }
 }
-void launch_trace_any(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint8_t* occluded,
-                      int block) {
+void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
+                          uint4* hits, uint32_t* work) {
     if (n == 0) return;
-    k_trace_any<<<(n + block - 1) / block, block, 0, st>>>(sc, rays, n, occluded);
+    StageArgs a{};
+    a.rays = rays;
+    a.hits = hits;
+    a.n = n;
+    a.work = work;
+    launch_stage(lc, st, sc, a);
 }
-void launch_primary(cudaStream_t st, const DevScene& sc, const DevView& v, float near_z, float far_z, float* depth,
-                    float4* const gb[4], float4* hitpos) {
-    uint32_t npix = v.width * v.height;
-    if (npix == 0) return;
-    k_primary<<<(npix + 255) / 256, 256, 0, st>>>(sc, v, near_z, far_z, depth, gb[0], gb[1], gb[2], gb[3], hitpos);
+void launch_trace_any(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
+                      uint8_t* occluded, uint32_t* work) {
+    if (n == 0) return;
+    StageArgs a{};
+    a.rays = rays;
+    a.occluded = occluded;
+    a.n = n;
+    a.work = work;
+    launch_stage(lc, st, sc, a);
+}
+void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView& v, float near_z,
+                    float far_z, float* depth, float4* const gb[4], float4* hitpos, uint32_t* work) {
+    const uint32_t n = v.width * v.height;
+    if (n == 0) return;
+    const PrimaryOut out{depth, {gb[0], gb[1], gb[2], gb[3]}, hitpos, near_z, far_z};
+    float4* rec = hitpos ? hitpos : gb[0] ? gb[0] : gb[1] ? gb[1] : gb[2] ? gb[2] : gb[3];
+    if (rec && !sc.insts && n <= kGroupPixels) {
+        StageArgs a{};
+        a.rec = rec;
+        a.n = n;
+        a.work = work;
+        a.view = v;
+        launch_stage(lc, st, sc, a);
+        k_primary_rec<<<(n + 127) / 128, 128, 0, st>>>(sc, v, out, rec);
+        return;
+    }
+    const uint32_t blocks = ((v.width + 15u) / 16u) * ((v.height + 7u) / 8u);
+    if (sc.insts) k_primary<true><<<blocks, 128, 0, st>>>(sc, v, out);
+    else k_primary<false><<<blocks, 128, 0, st>>>(sc, v, out);
 }
 void launch_trace_count(cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n, uint2* counts) {
     if (n == 0) return;
@@ -796,6 +944,11 @@ void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     if (per_sm < 1) per_sm = 1;
     if (per_sm_shade < 1) per_sm_shade = 1;
     lc->block_trace = block_trace;
+    int per_sm_stage = 0, per_sm_stage2 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage, k_stage<true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage2, k_stage2<true>, 128, 0);
+    lc->grid_stage = sms * (per_sm_stage < 1 ? 1 : per_sm_stage);
+    lc->grid_stage2 = sms * (per_sm_stage2 < 1 ? 1 : per_sm_stage2);
     int per_sm_group = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_group, k_trace_group<true>, kGroupBlock, 0);
     lc->grid_group = sms * (per_sm_group < 1 ? 1 : per_sm_group);

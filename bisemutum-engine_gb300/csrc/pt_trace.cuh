@@ -293,7 +293,7 @@ __device__ __forceinline__ bool has_tris(const uint2& T) { return (T.y & 0xffffu
 
 struct TraceCounters { uint32_t nodes, tris; };
 
-// Single-ray closest / any hit (used by the stage entry points).  Returns the
+// Single-ray closest / any hit (primary outputs, training paths, traversal counts).  Returns the
 // leaf-ordered triangle index (kMissPrim on a miss); t = tmax on a miss.
 // Rule of a candidate hit on a triangle of transparency `tr` (0 = opaque).
 __device__ __forceinline__ bool keep_hit(const RayPre& r, float tr, uint32_t oseed) {
@@ -472,8 +472,8 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // Persistent, warp-synchronous traversal of a queue of n rays.  Every lane of
 // the warp runs this loop together (all ballots use the full mask).  `rays`
 // supplies them: `load` (index -> (origin/tmin, direction/tmax)); `any(index)`,
-// whether the ray stops at its first hit; `hit(index, leaf, t, u, v)`, called
-// at every closer hit (the last call stands: keeping the record in memory
+// whether the ray stops at its first hit; `hit(index, leaf, t, u, v, instance)`,
+// called at every closer hit (the last call stands: keeping the record in memory
 // instead of registers frees three of the 64, which is what it takes to keep
 // this loop from spilling), and `miss(index, tmax)`; with kOpacity,
 // `seed(index)` gives the ray's opacity seed, read only when a candidate hit
@@ -561,7 +561,7 @@ __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, co
                     (!kOpacity || c.w == 0.0f || keep_hit(r, c.w, rays.seed(idx)))) {
                     tbest = t;
                     best_prim = prim;
-                    rays.hit(idx, ti, t, u, v);
+                    rays.hit(idx, ti, t, u, v, kMissPrim);
                     if (rays.any(idx)) { T.y = 0u; G.y = 0u; sp = 0; }
                 }
             }
@@ -756,7 +756,7 @@ __device__ __forceinline__ void trace_queue_group(const CwNode* __restrict__ nod
             const uint32_t best = group_min(lprim);
             if (done) {
                 if (best == kMissPrim) { if (sub == 0) rays.miss(idx, lt); }
-                else if (lprim == best) rays.hit(idx, lleaf, lt, lu, lv);
+                else if (lprim == best) rays.hit(idx, lleaf, lt, lu, lv, kMissPrim);
                 has = false;
             }
         }
@@ -786,7 +786,6 @@ static_assert(kMaxTlasDepth + 3 + kMaxTraversalDepth + 2 * kPostponeMaxSp <= kSt
 // Results and the opacity rule are those of trace_ray2: object-space
 // triangle tests with t unchanged, ties to the lower global primitive id,
 // candidate hits on non-opaque triangles decided with the world ray.
-// The hit record carries the instance in place of u (`hit(index, leaf, t, instance bits, v)`).
 template <bool kOpacity, class Rays>
 __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
                                              const float* __restrict__ mat_tr, uint32_t n, uint32_t* work,
@@ -904,7 +903,7 @@ __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, co
                 if (keep) {
                     tbest = t;
                     best_prim = prim;
-                    rays.hit(idx, ti, t, __uint_as_float(inst), v);
+                    rays.hit(idx, ti, t, u, v, inst);
                     if (rays.any(idx)) { T.y = 0u; G.y = 0u; sp = 0; }
                 }
             }

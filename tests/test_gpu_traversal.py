@@ -1,11 +1,13 @@
 """The traversal kernels against the oracle where their shortcuts could go wrong: exact zeros on edges and
 vertices for every dominant axis and sign of the direction; frames on both sides of the chunk size at which the
 kernel with eight lanes per ray hands over to the one with a lane per ray (98,304 paths), with and without
-non-opaque materials."""
+non-opaque materials; stage entry points and primary outputs at the sizes where their kernels change."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from conftest import assert_bits_equal
+from conftest import assert_bits_equal, random_rays
 
 pytestmark = pytest.mark.gpu
 
@@ -82,4 +84,47 @@ def test_both_sides_of_the_group_kernel_limit(bsm, ctx, oracle, w, h, spp, opaqu
     ref, ost, _ = oracle.OracleScene(sc).render(sc.camera.as_array(), spp=spp, max_segments=4, seed=5, flags=det)
     assert list(st.rays_per_segment[:4]) == [int(x) for x in ost[:4]]
     assert_bits_equal(imgs[0][..., :3], ref[..., :3])
+    ctx.release(sid)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 40000, 40001, 300007])   # eight lanes per ray up to 40,000
+@pytest.mark.parametrize("opaque", [True, False])
+def test_stage_entry_points_at_their_kernels_limits(bsm, ctx, oracle, n, opaque):
+    sc = bsm.generate_scene(bsm.BSM_SCENE_ROOM, seed=12)
+    if not opaque:
+        sc.materials[::2, 5], sc.materials[::2, 6] = 0.5, bsm.BSM_BLEND_TRANSLUCENT
+    sid, osc = ctx.load_scene(sc), oracle.OracleScene(sc)
+    rays = random_rays(n, 0.0, 1.0, seed=n)
+    rays[n // 2, 4:7] = 0.0   # one that is not traced
+    for _ in range(2):        # the second call starts from the work counter that the first one left
+        assert np.array_equal(ctx.trace_closest(sid, rays), osc.trace(rays))
+        assert np.array_equal(ctx.trace_any(sid, rays) != 0, osc.trace(rays, any_hit=True)[:, 1] != 0xFFFFFFFF)
+    ctx.release(sid)
+
+
+# a tile is 16 x 8 pixels; up to 24,576 pixels go to the kernel with eight lanes per ray
+@pytest.mark.parametrize("w,h", [(1, 1), (17, 9), (192, 128), (193, 128), (8, 5001), (5001, 8)])
+@pytest.mark.parametrize("which", ["all", "depth", "normals"])
+def test_primary_outputs_at_their_kernels_limits(bsm, ctx, oracle, w, h, which):
+    sc = bsm.generate_scene(bsm.BSM_SCENE_ROOM, seed=13, width=w, height=h)
+    sid, cam = ctx.load_scene(sc), sc.camera
+    d0, g0, h0 = oracle.OracleScene(sc).primary(cam.as_array())
+    d, g, hp = np.zeros_like(d0), np.zeros_like(g0), np.zeros_like(h0)
+    out = bsm.PrimaryOutput()
+    if which != "normals":
+        out.depth = d.ctypes.data
+    for k in range(4):
+        if which == "all" or (which == "normals" and k == 1):
+            out.gbuffer[k] = g[k].ctypes.data
+    if which == "all":
+        out.hit_positions = hp.ctypes.data
+    out.location = bsm.BSM_HOST
+    ctx.check(ctx._L.bsm_render_primary(ctx.h, sid, C.byref(cam), None, 0.0, 0.0, C.byref(out)))
+    if which != "normals":
+        assert_bits_equal(d, d0)
+    if which == "normals":
+        assert_bits_equal(g[1], g0[1])
+    if which == "all":
+        assert_bits_equal(g, g0)
+        assert_bits_equal(hp, h0)
     ctx.release(sid)
