@@ -130,6 +130,7 @@ struct LaunchCfg {
     int postpone_sp = 16;   // traversal stack budget for postponed triangle groups
     int refill_min = 8;     // idle lanes that trigger a warp refill
     int grid_stage, grid_stage2;   // blocks of the stage entry points' kernels (one / two levels)
+    int grid_group2;        // ... of the two-level one
     int grid_group;         // blocks of the traversal kernel for small chunks (eight lanes per ray)
     int regcap = 1;         // 1: traversal kernels compiled for 4 blocks of 256 (64 registers); the default
 };

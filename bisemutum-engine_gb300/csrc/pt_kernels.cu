@@ -194,6 +194,7 @@ struct TraceArgs {
     uint32_t* counters;
     unsigned long long* stats;
     uint32_t ext, shd, sh_last;   // segments (kNoSegment: none); the shadow queue's last slot
+    uint32_t min_rays, max_rays;  // the kernel leaves queues of other lengths alone
     int postpone_sp, refill_min;
 };
 struct TraceRays {
@@ -233,11 +234,13 @@ __device__ __forceinline__ TraceRays trace_rays(const TraceArgs& a) {
         n_sun = a.counters[kCntShadow + a.shd];
         n_sky = a.counters[kCntSky + a.shd];
     }
+    const uint32_t n = n_ext + n_sun + n_sky;
+    if (n < a.min_rays || n > a.max_rays) return TraceRays{a, 0u, 0u, 0u};
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (n_ext) a.stats[kStatExtend + a.ext] += n_ext;
         if (n_sun + n_sky) a.stats[kStatShadow + a.shd] += n_sun + n_sky;
     }
-    return TraceRays{a, n_ext, n_ext + n_sun, n_ext + n_sun + n_sky};
+    return TraceRays{a, n_ext, n_ext + n_sun, n};
 }
 
 template <int kMinBlocks, bool kOpacity>
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_trace(const CwNode* __restr
     trace_queue<false, kOpacity>(nodes, tris, rays.n, rays.work(), rays, nullptr, a.postpone_sp, a.refill_min);
 }
 
-// k_trace for chunks of at most kGroupPaths paths: eight lanes per ray.  A
+// k_trace for small chunks and short queues: eight lanes per ray.  A
 // kernel of its own, because its loop in k_trace costs that one registers
 // (1080p 64-spp frame 160.8 -> 168.7 ms with both), and 80 registers are worth
 // more here than occupancy (64 of them spill: 443 against 377 us for a 128x128
@@ -269,6 +272,17 @@ __global__ void __launch_bounds__(256, 4) k_trace2(const CwNode* __restrict__ tl
                                                    const __grid_constant__ TraceArgs a) {
     const TraceRays rays = trace_rays(a);
     trace_queue2<kOpacity>(tlas, insts, mat_tr, rays.n, rays.work(), rays, a.postpone_sp, a.refill_min);
+}
+
+// The same in two levels.
+template <bool kOpacity>
+__global__ void __launch_bounds__(kGroupBlock, kGroup2Blocks) k_trace2_group(const CwNode* __restrict__ tlas,
+                                                                 const InstDev* __restrict__ insts,
+                                                                 const float* __restrict__ mat_tr,
+                                                                 const __grid_constant__ TraceArgs a) {
+    __shared__ GroupStacks2 stacks;
+    const TraceRays rays = trace_rays(a);
+    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, rays.n, rays.work(), rays, stacks);
 }
 
 // ----------------------------------------------------------------- shade ----
@@ -635,6 +649,15 @@ __global__ void __launch_bounds__(kGroupBlock, 6) k_stage_group(const CwNode* __
     stage_done(a.work);
 }
 template <bool kOpacity>
+__global__ void __launch_bounds__(kGroupBlock, kGroup2Blocks) k_stage2_group(const CwNode* __restrict__ tlas,
+                                                                 const InstDev* __restrict__ insts,
+                                                                 const float* __restrict__ mat_tr,
+                                                                 const __grid_constant__ StageArgs a) {
+    __shared__ GroupStacks2 stacks;
+    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, a.n, a.work, StageRays{a}, stacks);
+    stage_done(a.work);
+}
+template <bool kOpacity>
 __global__ void __launch_bounds__(128, 8) k_stage2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
                                                    const float* __restrict__ mat_tr,
                                                    const __grid_constant__ StageArgs a) {
@@ -792,27 +815,44 @@ void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const
     if (n) k_gather_normals<<<(n + 255) / 256, 256, 0, st>>>(tris, n, vn, idx, out);
 }
 
-// Chunks of at most this many paths (the queues of every segment are known only to the device) are traced with
-// eight lanes per ray.  Their launches are too short for the lane-per-ray loop's throughput to show: 8-segment
-// 1-spp frames of the room take 539 / 597 / 680 / 782 us lane by lane and 337 / 377 / 548 / 839 us in groups at
-// 64^2 / 128^2 / 256^2 / 362^2 pixels, of the 1.48 M-triangle terrain 806 / 909 / 1050 / 1184 and
-// 472 / 551 / 823 / 1222 us: the lines cross near 110,000 paths.
-constexpr uint32_t kGroupPaths = 98304;
+// Which kernel traces a segment's queue. Eight lanes per ray win while a launch is as long as its longest ray, a
+// lane per ray where throughput counts. The queues' lengths are known only to the device, so:
+//  * chunks of up to kGroupPaths paths (two levels: kGroupPaths2) take the group kernel for every segment;
+//  * chunks of up to kMixedPaths launch both after the first segment, and each leaves the queues of the other's
+//    length alone (2 us for the one that does; the first segment's queue is the chunk itself);
+//  * larger chunks, whose later queues are long too, take the lane-per-ray kernel.
+// 8-segment 1-spp frames, us, lane / group / both: room 181^2 629 / 433 / 455, 256^2 680 / 549 / 524, 362^2
+// 772 / 839 / 670, 512^2 922 / - / 889, 724^2 1180 / - / 1181; 1.48 M triangles 181^2 983 / 643 / 700, 256^2
+// 1050 / 825 / 766, 362^2 1173 / 1222 / 934, 512^2 1395 / - / 1240, 724^2 1828 / - / 1775; at 1024^2 (and over)
+// both change nothing. Two levels (4 segments, 1,000 instances): 128x72 873 / 443, 320x180 1021 / 661 / 740,
+// 641x359 1255 / 2012 / 1238.
+constexpr uint32_t kGroupPaths = 40960, kGroupPaths2 = 98304, kMixedPaths = 1000000;
+// Longest queue for the group kernel. One level: of 45,000, 70,000 and 100,000 the first is the best in the room
+// (512^2 889 / 900 / 927 us) and the second in the terrain (512^2 1251 / 1228 / 1241 us); two levels: 60,000 and
+// 90,000 are level, 120,000 is slower (641x359 1240 / 1238 / 1311 us).
+constexpr uint32_t kGroupQueue = 56000, kGroupQueue2 = 90000;
 
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
                   uint32_t shd, float4* accum, uint32_t paths) {
-    const bool op = sc.has_non_opaque != 0;
-    const TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
-                      wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u,
-                      lc.postpone_sp, lc.refill_min};
-    if (sc.insts) {
+    TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
+                wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u, 0u, 0xffffffffu,
+                lc.postpone_sp, lc.refill_min};
+    const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr;
+    const bool only = paths <= (two ? kGroupPaths2 : kGroupPaths), mix = !only && paths <= kMixedPaths && ext != 0u;
+    const uint32_t limit = two ? kGroupQueue2 : kGroupQueue;
+    if (only || mix) {
+        if (mix) a.max_rays = limit;
+        if (two && op) k_trace2_group<true><<<lc.grid_group2, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else if (two) k_trace2_group<false><<<lc.grid_group2, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else if (op) k_trace_group<true><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        else k_trace_group<false><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        if (only) return;
+        a.min_rays = limit + 1u;
+        a.max_rays = 0xffffffffu;
+    }
+    if (two) {
         if (op) k_trace2<true><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
         else k_trace2<false><<<lc.grid_persistent2, lc.block_trace, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-        return;
-    }
-    if (paths <= kGroupPaths) {
-        if (op) k_trace_group<true><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
-        else k_trace_group<false><<<lc.grid_group, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
         return;
     }
 #define BSM_TRACE(B, O) k_trace<B, O><<<lc.grid_persistent, lc.block_trace, 0, st>>>(sc.nodes, sc.tris, a)
@@ -855,7 +895,8 @@ void launch_fold_fixed(cudaStream_t st, const unsigned long long* fx, float4* ac
 // Calls of at most this many rays are traced with eight lanes per ray. Closest and any hit of half-random rays
 // take 76 / 103 us in groups and 115 / 152 lane by lane at 16,384 rays (room / 1.48 M triangles), 177 / 235 and
 // 132 / 194 us at 65,536.
-constexpr uint32_t kGroupRays = 40000;
+// In two levels 65 / 103 / 207 us in groups and 132 / 149 / 191 lane by lane at 3,000 / 30,000 / 100,000 rays.
+constexpr uint32_t kGroupRays = 40000, kGroupRays2 = 60000;
 // Views of at most this many pixels take that way too, their hit records waiting in one of the outputs for
 // k_primary_rec: 35 / 58 us against 37 / 113 us in k_primary at 128x128 (room / 1.48 M triangles); at 230x170
 // 48 / 86 against 41 / 111.
@@ -867,11 +908,14 @@ static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
     a.postpone_sp = 16;
     a.refill_min = 8;
     const bool op = sc.has_non_opaque != 0;
-    const bool few = !sc.insts && a.n <= kGroupRays;
+    const bool few = a.n <= (sc.insts ? kGroupRays2 : kGroupRays);
     const uint32_t per_block = few ? 128u / kGroupLanes : 128u;
-    const uint32_t full = sc.insts ? lc.grid_stage2 : few ? lc.grid_group : lc.grid_stage;
+    const uint32_t full = sc.insts ? (few ? lc.grid_group2 : lc.grid_stage2) : (few ? lc.grid_group : lc.grid_stage);
     const uint32_t grid = min(full, (uint32_t)(((uint64_t)a.n + per_block - 1) / per_block));
-    if (sc.insts) {
+    if (sc.insts && few) {
+        if (op) k_stage2_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else k_stage2_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+    } else if (sc.insts) {
         if (op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
         else k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
     } else if (few) {
@@ -949,7 +993,9 @@ void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage2, k_stage2<true>, 128, 0);
     lc->grid_stage = sms * (per_sm_stage < 1 ? 1 : per_sm_stage);
     lc->grid_stage2 = sms * (per_sm_stage2 < 1 ? 1 : per_sm_stage2);
-    int per_sm_group = 0;
+    int per_sm_group = 0, per_sm_group2 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_group2, k_trace2_group<true>, kGroupBlock, 0);
+    lc->grid_group2 = sms * (per_sm_group2 < 1 ? 1 : per_sm_group2);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_group, k_trace_group<true>, kGroupBlock, 0);
     lc->grid_group = sms * (per_sm_group < 1 ? 1 : per_sm_group);
     lc->grid_persistent = sms * per_sm;

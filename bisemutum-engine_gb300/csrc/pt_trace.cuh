@@ -938,4 +938,243 @@ __device__ __forceinline__ void trace_queue2(const CwNode* __restrict__ tlas, co
     }
 }
 
+// ------------------------------------------------- eight lanes per ray, two levels ----
+// Stack: a rest per TLAS level, a node's inner children, its other instances and an exit marker below a BLAS's own
+// levels.
+// blocks per SM of the kernels that use it (96 registers): 1,000 instances at 320x180, 699 / 655 / 697 / 786 us
+// with 4 / 5 / 6 / 8
+constexpr int kGroup2Blocks = 5;
+constexpr int kGroupStack2 = 44;
+static_assert(kMaxTlasDepth + 3 + kMaxTraversalDepth <= kGroupStack2, "two-level group stack budget");
+struct GroupStacks2 {
+    uint2 e[kGroupBlock / 32][kWarpGroups][kGroupStack2];
+    float4 world[kGroupBlock / 32][kWarpGroups][2];   // the world ray's divided constants
+};
+
+// trace_queue_group for two-level scenes: a TLAS node's leaf children that are
+// hit are instances, entered one after the other in visiting order with the
+// rest of the node's work below an exit marker, as in trace_queue2.
+template <bool kOpacity, class Rays>
+__device__ __forceinline__ void trace_queue2_group(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
+                                                   const float* __restrict__ mat_tr, uint32_t n, uint32_t* work,
+                                                   const Rays& rays, GroupStacks2& stacks) {
+    const uint32_t lane = threadIdx.x & 31u, group = lane / kGroupLanes, sub = lane % kGroupLanes;
+    uint2* stack = stacks.e[threadIdx.x >> 5][group];
+    float4* world = stacks.world[threadIdx.x >> 5][group];
+    bool has = false, exhausted = n == 0u, lead = true;
+    RayPre r;
+    float tb = 0.0f, lt = 0.0f, lu = 0.0f, lv = 0.0f;
+    uint32_t lleaf = kMissPrim, lprim = kMissPrim, linst = kMissPrim, idx = 0, slot = 0;
+    uint32_t near_x = 0, near_y = 0, near_z = 0;
+    const CwNode* nodes = tlas;
+    const CwTri* tris = nullptr;      // nullptr: in the TLAS
+    uint32_t inst = kMissPrim, prim_base = 0, mat_override = kMissPrim;
+    uint2 G = make_uint2(0u, 0u);
+    int sp = 0;
+    uint4 h0 = make_uint4(0, 0, 0, 0), h1 = h0;
+    uint32_t qnx = 0, qny = 0, qnz = 0, qfx = 0, qfy = 0, qfz = 0;
+    auto fetch = [&](uint32_t ni) {
+        const uint8_t* p = reinterpret_cast<const uint8_t*>(nodes + ni);
+        h0 = __ldg(reinterpret_cast<const uint4*>(p));
+        h1 = __ldg(reinterpret_cast<const uint4*>(p + 16));
+        const uint32_t f = 2u * slot;
+        qnx = __ldg(p + near_x); qfx = __ldg(p + (88u + f - near_x));
+        qny = __ldg(p + near_y); qfy = __ldg(p + (104u + f - near_y));
+        qnz = __ldg(p + near_z); qfz = __ldg(p + (120u + f - near_z));
+    };
+    auto aim = [&]() {   // this lane's child slot and plane offsets for the ray r
+        slot = sub ^ r.oct_key;
+        near_x = 32u + slot + (r.idx < 0.0f ? 24u : 0u);
+        near_y = 40u + slot + (r.idy < 0.0f ? 24u : 0u);
+        near_z = 48u + slot + (r.idz < 0.0f ? 24u : 0u);
+    };
+    auto step = [&]() {  // takes the nearest child of G and loads it
+        const uint32_t bit = 31u - (uint32_t)__clz(G.y & 0xff000000u);
+        G.y &= ~(1u << bit);
+        const uint32_t s = (bit - 24u) ^ r.oct_key;
+        fetch(G.x + (uint32_t)__popc(G.y & 0xffu & ((1u << s) - 1u)));
+    };
+    while (true) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !has);
+        if (idle != 0u && !exhausted) {
+            const uint32_t want = (uint32_t)__popc(idle) / kGroupLanes;
+            uint32_t base;
+            if (lead) {
+                base = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kWarpGroups;
+                lead = false;
+            } else {
+                base = 0;
+                if (lane == 0) base = atomicAdd(work, want);
+                base = __shfl_sync(0xffffffffu, base, 0) + gridDim.x * (blockDim.x >> 5) * kWarpGroups;
+            }
+            const uint32_t i = base + (uint32_t)__popc(idle & ((1u << (group * kGroupLanes)) - 1u)) / kGroupLanes;
+            if (!has && i < n) {
+                float4 o, d;
+                rays.load(i, o, d);
+                r = make_ray(o, d);
+                tb = lt = d.w;
+                lleaf = lprim = linst = kMissPrim;
+                lu = lv = 0.0f;
+                idx = i;
+                sp = 0;
+                G = make_uint2(0u, 0u);
+                nodes = tlas; tris = nullptr; inst = kMissPrim; prim_base = 0u; mat_override = kMissPrim;
+                aim();
+                if (ray_traceable(r, d.w)) {
+                    has = true;
+                    // every lane of the group writes the same values and reads back its own
+                    world[0] = make_float4(r.idx, r.idy, r.idz, __uint_as_float(r.oct_key | (r.perm << 4)));
+                    world[1] = make_float4(r.Sx, r.Sy, r.Sz, 0.0f);
+                    fetch(0u);
+                } else if (sub == 0) {
+                    rays.miss(i, d.w);
+                }
+            }
+            if (base + want >= n) exhausted = true;
+            if (__ballot_sync(0xffffffffu, has) == 0u) {
+                if (exhausted) break;
+                continue;
+            }
+        } else if (idle == 0xffffffffu) {
+            break;
+        }
+        // this lane's child slot of the node that was fetched
+        bool hit;
+        const uint32_t ew = h0.w, imask = ew >> 24, child_base = h1.x, tri_base = h1.y, tm = h1.z & 0xffffu;
+        {
+            float sx = __uint_as_float((ew & 0xffu) << 23) * r.idx;
+            float sy = __uint_as_float(((ew >> 8) & 0xffu) << 23) * r.idy;
+            float sz = __uint_as_float(((ew >> 16) & 0xffu) << 23) * r.idz;
+            float ax = (__uint_as_float(h0.x) - r.ox) * r.idx;
+            float ay = (__uint_as_float(h0.y) - r.oy) * r.idy;
+            float az = (__uint_as_float(h0.z) - r.oz) * r.idz;
+            ax = __fsub_rn(ax, 8388608.0f * sx);
+            ay = __fsub_rn(ay, 8388608.0f * sy);
+            az = __fsub_rn(az, 8388608.0f * sz);
+            float tnx = __fmaf_rn(__uint_as_float(0x4b000000u | qnx), sx, ax);
+            float tny = __fmaf_rn(__uint_as_float(0x4b000000u | qny), sy, ay);
+            float tnz = __fmaf_rn(__uint_as_float(0x4b000000u | qnz), sz, az);
+            float tfx = __fmaf_rn(__uint_as_float(0x4b000000u | qfx), sx, ax);
+            float tfy = __fmaf_rn(__uint_as_float(0x4b000000u | qfy), sy, ay);
+            float tfz = __fmaf_rn(__uint_as_float(0x4b000000u | qfz), sz, az);
+            float tn = max3f(tnx, tny, fmaxf(tnz, r.tmin));
+            float tf = min3f(tfx, tfy, fminf(tfz, fmaxf(tb, tb * 0.9999981f)));
+            hit = has && !((int)__float_as_uint(__fmaf_rn(tf, BSM_BOX_PAD, -tn)) < 0);
+        }
+        const uint32_t leaf_bits = hit ? (tm >> (2u * slot)) & 3u : 0u;
+        const uint32_t inner = (__ballot_sync(0xffffffffu, hit && ((imask >> slot) & 1u)) >> (group * kGroupLanes)) & 0xffu;
+        const uint32_t leaves = (__ballot_sync(0xffffffffu, leaf_bits != 0u) >> (group * kGroupLanes)) & 0xffu;
+        const uint32_t nt = tris != nullptr ? leaf_bits : 0u;       // this lane's triangles
+        const uint32_t ti = tri_base + (uint32_t)__popc(tm & ((1u << (2u * slot)) - 1u));
+        // a next node of the same BVH is loaded before the triangles are tested; what needs the stack waits, since
+        // it can change the ray's space
+        bool more = has, from_stack = false;
+        uint2 enter = make_uint2(0u, 0u);
+        if (has) {
+            if (inner != 0u) {
+                if ((G.y & 0xff000000u) != 0u) stack[sp++] = G;   // all lanes of the group write the same entry
+                G = make_uint2(child_base, (inner << 24) | imask);
+            }
+            if (tris == nullptr && leaves != 0u) {
+                if ((G.y & 0xff000000u) != 0u) stack[sp++] = G;
+                G = make_uint2(0u, 0u);
+                enter = make_uint2(tri_base, (leaves << 24) | tm);
+            } else if ((G.y & 0xff000000u) != 0u) {
+                step();
+            } else {
+                from_stack = true;
+            }
+        }
+        if (__ballot_sync(0xffffffffu, nt != 0u) != 0u) {
+            bool got = false;
+            if (nt != 0u) {
+                const float4* tp = reinterpret_cast<const float4*>(tris + ti);
+                float4 a0 = __ldg(tp), b0 = __ldg(tp + 1), c0 = __ldg(tp + 2);
+                float4 a1 = a0, b1 = b0, c1 = c0;
+                if (nt == 3u) { a1 = __ldg(tp + 3); b1 = __ldg(tp + 4); c1 = __ldg(tp + 5); }
+#pragma unroll 1
+                for (uint32_t k = 0; k < (nt == 3u ? 2u : 1u); ++k) {
+                    const uint32_t prim = prim_base + __float_as_uint(a0.w);
+                    float t, u, v;
+                    if (tri_test(r, a0, b0, c0, lt, prim, lprim, t, u, v)) {
+                        bool keep = true;
+                        if (kOpacity && mat_tr) {
+                            const float tr = mat_tr[mat_override != kMissPrim ? mat_override : __float_as_uint(b0.w)];
+                            if (tr != 0.0f) {   // the rule reads the world ray
+                                float4 o4, d4;
+                                rays.load(idx, o4, d4);
+                                keep = keep_hit(make_ray(o4, d4), tr, rays.seed(idx));
+                            }
+                        }
+                        if (keep) {
+                            lt = t; lu = u; lv = v; lleaf = ti + k; lprim = prim; linst = inst;
+                            got = true;
+                        }
+                    }
+                    a0 = a1; b0 = b1; c0 = c1;
+                }
+            }
+            const uint32_t gb = __ballot_sync(0xffffffffu, got);
+            if (gb != 0u) {
+                tb = group_min(lt);
+                if (lt > tb) { lt = tb; lprim = kMissPrim; }
+                if (rays.any(idx) && ((gb >> (group * kGroupLanes)) & 0xffu) != 0u) { more = false; from_stack = false; enter.y = 0u; }
+            }
+        }
+        if (from_stack) {
+            while (true) {
+                if (sp == 0) { more = false; break; }
+                const uint2 e = stack[--sp];
+                if (e.y == 0u) {   // exit marker: back to the world ray and the TLAS
+                    float4 o4, d4, c0 = world[0], c1 = world[1];
+                    rays.load(idx, o4, d4);
+                    const uint32_t pk = __float_as_uint(c0.w);
+                    r.ox = o4.x; r.oy = o4.y; r.oz = o4.z; r.tmin = o4.w;
+                    r.dx = d4.x; r.dy = d4.y; r.dz = d4.z;
+                    r.idx = c0.x; r.idy = c0.y; r.idz = c0.z;
+                    r.oct_key = pk & 15u;
+                    r.perm = pk >> 4;
+                    r.Sx = c1.x; r.Sy = c1.y; r.Sz = c1.z;
+                    nodes = tlas; tris = nullptr; inst = kMissPrim; prim_base = 0u; mat_override = kMissPrim;
+                    aim();
+                    continue;
+                }
+                if (e.x & kTriGroupFlag) enter = make_uint2(e.x & ~kTriGroupFlag, e.y);
+                else { G = e; step(); }
+                break;
+            }
+        }
+        if (enter.y != 0u) {
+            // the nearest of the hit instances; the others wait below an exit marker
+            const uint32_t bit = 31u - (uint32_t)__clz(enter.y);
+            enter.y &= ~(1u << bit);
+            if ((enter.y & 0xff000000u) != 0u) stack[sp++] = make_uint2(enter.x | kTriGroupFlag, enter.y);
+            stack[sp++] = make_uint2(kStackExit, 0u);
+            const uint32_t s = (bit - 24u) ^ r.oct_key;
+            inst = enter.x + (uint32_t)__popc(enter.y & 0xffffu & ((1u << (2u * s)) - 1u));
+            const InstDev* I = insts + inst;
+            float mx[12];
+            load_xform(I->w2o, mx);
+            r = make_ray(xform_point(mx, r.ox, r.oy, r.oz, r.tmin), xform_dir(mx, r.dx, r.dy, r.dz, 0.0f));
+            nodes = I->nodes;
+            tris = I->tris;
+            prim_base = I->prim_base;
+            mat_override = I->material;
+            G = make_uint2(0u, 0u);
+            aim();
+            fetch(0u);
+        }
+        // finished rays: the lane that holds the closest hit of the lowest primitive id reports it
+        const bool done = has && !more;
+        if (__ballot_sync(0xffffffffu, done) != 0u) {
+            const uint32_t best = group_min(lprim);
+            if (done) {
+                if (best == kMissPrim) { if (sub == 0) rays.miss(idx, lt); }
+                else if (lprim == best) rays.hit(idx, lleaf, lt, lu, lv, linst);
+                has = false;
+            }
+        }
+    }
+}
+
 }  // namespace bsm

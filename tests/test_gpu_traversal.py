@@ -1,7 +1,7 @@
 """The traversal kernels against the oracle where their shortcuts could go wrong: exact zeros on edges and
-vertices for every dominant axis and sign of the direction; frames on both sides of the chunk size at which the
-kernel with eight lanes per ray hands over to the one with a lane per ray (98,304 paths), with and without
-non-opaque materials; stage entry points and primary outputs at the sizes where their kernels change."""
+vertices for every dominant axis and sign of the direction; frames on both sides of the chunk sizes at which the
+kernel with eight lanes per ray hands over to both kernels (40,960 paths) and these to the one with a lane per ray
+(1,000,000), with and without non-opaque materials, in one level and in two; stage entry points and primary outputs at the sizes where their kernels change."""
 import ctypes as C
 
 import numpy as np
@@ -72,9 +72,10 @@ def test_exact_zeros_match_the_oracle_bit_for_bit(bsm, ctx, oracle, tmin):
     ctx.release(sid)
 
 
-@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (9, 3, 1), (384, 256, 1), (385, 256, 1), (128, 96, 9)])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (9, 3, 1), (256, 160, 1), (257, 160, 1), (128, 96, 9), (250, 250, 16),
+                                     (251, 250, 16)])
 @pytest.mark.parametrize("opaque", [True, False])
-def test_both_sides_of_the_group_kernel_limit(bsm, ctx, oracle, w, h, spp, opaque):
+def test_both_sides_of_the_group_kernel_limits(bsm, ctx, oracle, w, h, spp, opaque):
     sc = bsm.generate_scene(bsm.BSM_SCENE_ROOM, seed=11, width=w, height=h)
     if not opaque:
         sc.materials[1::2, 5], sc.materials[1::2, 6] = 0.6, bsm.BSM_BLEND_TRANSLUCENT
@@ -127,4 +128,30 @@ def test_primary_outputs_at_their_kernels_limits(bsm, ctx, oracle, w, h, which):
     if which == "all":
         assert_bits_equal(g, g0)
         assert_bits_equal(hp, h0)
+    ctx.release(sid)
+
+
+# eight lanes per ray up to 98,304 paths (512 x 192); beyond, queues of up to 90,000 rays
+@pytest.mark.parametrize("w,h", [(1, 1), (13, 7), (512, 192), (513, 192)])
+@pytest.mark.parametrize("opaque", [True, False])
+def test_two_level_frames_on_both_sides_of_the_limits(bsm, ctx, oracle, w, h, opaque):
+    sc = bsm.generate_instanced_scene(seed=6, instances=120, width=w, height=h, sphere_res=8, ground=16)
+    if not opaque:
+        sc.materials[::3, 5], sc.materials[::3, 6] = 0.5, bsm.BSM_BLEND_TRANSLUCENT
+    sid = ctx.load_instanced(sc)
+    det = bsm.BSM_PT_DETERMINISTIC
+    imgs, st = ctx.render(sid, [sc.camera], bsm.settings(spp=1, max_segments=4, seed=8, flags=det))
+    ref, ost, _ = oracle.OracleScene(sc).render(sc.camera.as_array(), spp=1, max_segments=4, seed=8, flags=det)
+    assert list(st.rays_per_segment[:4]) == [int(x) for x in ost[:4]]
+    assert_bits_equal(imgs[0][..., :3], ref[..., :3])
+    ctx.release(sid)
+
+
+@pytest.mark.parametrize("n", [1, 33, 60000, 60001])   # eight lanes per ray up to 60,000
+def test_two_level_stage_entry_points_on_both_sides_of_the_limit(bsm, ctx, oracle, n):
+    sc = bsm.generate_instanced_scene(seed=6, instances=120, sphere_res=8, ground=16)
+    sid, osc = ctx.load_instanced(sc), oracle.OracleScene(sc)
+    rays = random_rays(n, -3.0, 3.0, seed=n)
+    assert np.array_equal(ctx.trace_closest(sid, rays), osc.trace(rays))
+    assert np.array_equal(ctx.trace_any(sid, rays) != 0, osc.trace(rays, any_hit=True)[:, 1] != 0xFFFFFFFF)
     ctx.release(sid)
