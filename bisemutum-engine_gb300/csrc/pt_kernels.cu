@@ -266,8 +266,10 @@ __global__ void __launch_bounds__(kGroupBlock, 6) k_trace_group(const CwNode* __
 }
 
 // The same for two-level scenes: trace_queue2 (TLAS leaves enter instances).
+// 80 registers: at 64 the loop spills (1,000 instances, 1-spp 4-segment frame:
+// 1241 -> 1116 us at 641x359, 2437 -> 2313 us at 1280x720).
 template <bool kOpacity>
-__global__ void __launch_bounds__(256, 4) k_trace2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
+__global__ void __launch_bounds__(256, 3) k_trace2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
                                                    const float* __restrict__ mat_tr,
                                                    const __grid_constant__ TraceArgs a) {
     const TraceRays rays = trace_rays(a);
