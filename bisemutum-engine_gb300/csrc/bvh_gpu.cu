@@ -506,55 +506,231 @@ __global__ void k_make_children(const Task* __restrict__ tasks, uint32_t ntasks,
     }
 }
 
-// Finishes the subtree of one small node per warp with its references in
-// shared memory: the same binned SAH splits, a stable warp partition, children
-// pushed on a per-warp stack (every entry holds two or more references of a
-// disjoint range, so at most kSmall / 2 entries are live).
-__global__ void __launch_bounds__(kSmallWarps * 32) k_small(const Task* __restrict__ small, uint32_t nsmall,
+// A new pair of binary nodes: the children of `node`, left then right.
+__device__ __forceinline__ void write_child(BNode* nodes, uint32_t id, uint32_t parent, const float* lo, const float* hi,
+                                            uint32_t first, uint32_t count) {
+    uint4* p = reinterpret_cast<uint4*>(nodes + id);
+    p[0] = make_uint4(__float_as_uint(lo[0]), __float_as_uint(lo[1]), __float_as_uint(lo[2]), kNone);
+    p[1] = make_uint4(__float_as_uint(hi[0]), __float_as_uint(hi[1]), __float_as_uint(hi[2]), kNone);
+    p[2] = make_uint4(first, count, parent, 0u);
+}
+
+// A small node's working set in shared memory: its references and their boxes.
+struct SmallSet {
+    uint32_t ref[kSmall];
+    float lo[3][kSmall], hi[3][kSmall];
+};
+
+// Finishes a range of at most 32 references, one per lane, all of its nodes of
+// a level together.  The split of least cost of every node is found without
+// bins: a split between two bins is named by the first reference behind it, so
+// every lane sums up the boxes left and right of its own bin over its node's
+// references (broadcast by shuffles), for the three axes at once.  The counts,
+// boxes and costs are those of the bins, and the least cost of the first axis
+// and then the lowest bin is taken as k_split takes it.
+__device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_t n, uint32_t root_first, uint32_t node,
+                                             float area, BNode* __restrict__ nodes, Counters* cnt, int B,
+                                             uint32_t max_leaf, uint32_t max_nodes) {
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool in = lane < n;
+    uint32_t ref = 0;
+    float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
+    if (in) {
+        ref = S.ref[base + lane];
+        for (int k = 0; k < 3; ++k) { lo[k] = S.lo[k][base + lane]; hi[k] = S.hi[k][base + lane]; }
+    }
+    // this lane's node: references [s0, s0 + sc) of the range
+    uint32_t s0 = in ? 0u : lane, sc = in ? n : 1u;
+    bool open = sc >= 2u;
+    while (true) {
+        const uint32_t most = __reduce_max_sync(kFull, open ? sc : 0u);
+        if (most == 0u) break;
+        float cen[3], cl[3], ch[3];
+        for (int k = 0; k < 3; ++k) { cen[k] = 0.5f * (lo[k] + hi[k]); cl[k] = ch[k] = cen[k]; }
+        for (uint32_t j = 0; j < most; ++j) {
+            const uint32_t src = open && j < sc ? s0 + j : lane;
+            for (int k = 0; k < 3; ++k) {
+                const float c = __shfl_sync(kFull, cen[k], (int)src);
+                cl[k] = fminf(cl[k], c);
+                ch[k] = fmaxf(ch[k], c);
+            }
+        }
+        uint32_t bins = 0;       // this lane's bin per axis, 8 bits each
+        bool use[3];
+        for (int k = 0; k < 3; ++k) {
+            const float ext = ch[k] - cl[k];
+            const float scale = ext > 0.0f ? (float)B / ext : 0.0f;
+            use[k] = ext > 0.0f && scale > 0.0f;
+            if (use[k]) bins |= (uint32_t)bin_of(cen[k], cl[k], scale, B) << (8 * k);
+        }
+        // boxes and count left of each axis' own bin, box from it on
+        float L[3][6], R[3][6];
+        uint32_t nl[3] = {0u, 0u, 0u};
+        for (int a = 0; a < 3; ++a)
+            for (int k = 0; k < 3; ++k) { L[a][k] = R[a][k] = INFINITY; L[a][3 + k] = R[a][3 + k] = -INFINITY; }
+        for (uint32_t j = 0; j < most; ++j) {
+            const uint32_t src = open && j < sc ? s0 + j : lane;   // a lane's own box once more changes nothing
+            const uint32_t ob = __shfl_sync(kFull, bins, (int)src);
+            float o[6];
+            for (int k = 0; k < 3; ++k) {
+                o[k] = __shfl_sync(kFull, lo[k], (int)src);
+                o[3 + k] = __shfl_sync(kFull, hi[k], (int)src);
+            }
+            for (int a = 0; a < 3; ++a) {
+                if (((ob >> (8 * a)) & 255u) < ((bins >> (8 * a)) & 255u)) {
+                    nl[a]++;
+                    for (int k = 0; k < 3; ++k) { L[a][k] = fminf(L[a][k], o[k]); L[a][3 + k] = fmaxf(L[a][3 + k], o[3 + k]); }
+                } else {
+                    for (int k = 0; k < 3; ++k) { R[a][k] = fminf(R[a][k], o[k]); R[a][3 + k] = fmaxf(R[a][3 + k], o[3 + k]); }
+                }
+            }
+        }
+        float best = INFINITY;
+        uint32_t key = kNone;    // axis, then bin; and the lane it came from
+        for (int a = 0; a < 3; ++a) {
+            if (!use[a] || nl[a] == 0u) continue;
+            const float c = area6(L[a], L[a] + 3) * (float)nl[a] + area6(R[a], R[a] + 3) * (float)(sc - nl[a]);
+            if (c < best) { best = c; key = ((uint32_t)a << 16) | (((bins >> (8 * a)) & 255u) << 8) | lane; }
+        }
+        for (uint32_t j = 0; j < most; ++j) {
+            const uint32_t src = open && j < sc ? s0 + j : lane;
+            const float ob = __shfl_sync(kFull, best, (int)src);
+            const uint32_t ok = __shfl_sync(kFull, key, (int)src);
+            if (ob < best || (ob == best && ok < key)) { best = ob; key = ok; }
+        }
+        const bool split_axis = key != kNone;
+        const int axis = split_axis ? (int)(key >> 16) : -1;
+        const Split sp = decide(axis, 0, 0u, best, sc, area, max_leaf);
+        if (open && sp.leaf) open = false;
+        // stable partition
+        const bool left = open && (split_axis ? ((bins >> (8 * axis)) & 255u) < ((key >> 8) & 255u) : lane - s0 < sc / 2u);
+        const uint32_t lmask = __ballot_sync(kFull, left);
+        const uint32_t seg = sc >= 32u ? kFull : ((1u << sc) - 1u) << s0, below = seg & ((1u << lane) - 1u);
+        const uint32_t nleft = (uint32_t)__popc(lmask & seg);
+        // the children's boxes: the winning lane has both, unless the node was split by index
+        const int win = split_axis ? (int)(key & 255u) : (int)lane;
+        float bl[6], br[6];
+        for (int k = 0; k < 6; ++k) {
+            const float l = axis == 0 ? L[0][k] : axis == 1 ? L[1][k] : L[2][k];   // this lane's view of the axis
+            const float r = axis == 0 ? R[0][k] : axis == 1 ? R[1][k] : R[2][k];
+            bl[k] = __shfl_sync(kFull, l, win);   // the whole node agrees on the axis
+            br[k] = __shfl_sync(kFull, r, win);
+        }
+        const bool by_index = open && !split_axis;
+        if (__ballot_sync(kFull, by_index) != 0u) {
+            if (by_index)
+                for (int k = 0; k < 3; ++k) { bl[k] = br[k] = INFINITY; bl[3 + k] = br[3 + k] = -INFINITY; }
+            for (uint32_t j = 0; j < most; ++j) {
+                const uint32_t src = open && j < sc ? s0 + j : lane;
+                const bool ol = (lmask >> src) & 1u;
+                for (int k = 0; k < 3; ++k) {
+                    const float l = __shfl_sync(kFull, lo[k], (int)src), h = __shfl_sync(kFull, hi[k], (int)src);
+                    if (by_index && j < sc) {
+                        if (ol) { bl[k] = fminf(bl[k], l); bl[3 + k] = fmaxf(bl[3 + k], h); }
+                        else { br[k] = fminf(br[k], l); br[3 + k] = fmaxf(br[3 + k], h); }
+                    }
+                }
+            }
+        }
+        const bool lead = open && lane == s0;
+        const uint32_t leads = __ballot_sync(kFull, lead);
+        uint32_t id = 0;
+        if (leads != 0u) {
+            if (lane == 0) id = atomicAdd(&cnt->nodes, 2u * (uint32_t)__popc(leads));
+            id = __shfl_sync(kFull, id, 0);
+            if (id + 2u * (uint32_t)__popc(leads) > max_nodes) {
+                if (lane == 0) atomicOr(&cnt->error, kErrNodes);
+                return;
+            }
+        }
+        id += 2u * (uint32_t)__popc(leads & ((1u << s0) - 1u));
+        if (lead) {
+            nodes[node].left = id;
+            nodes[node].right = id + 1u;
+            write_child(nodes, id, node, bl, bl + 3, root_first + base + s0, nleft);
+            write_child(nodes, id + 1u, node, br, br + 3, root_first + base + s0 + nleft, sc - nleft);
+        }
+        __syncwarp();
+        if (open) {
+            const uint32_t at = base + (left ? s0 + (uint32_t)__popc(lmask & below) : s0 + nleft + (uint32_t)__popc(~lmask & below));
+            S.ref[at] = ref;
+            for (int k = 0; k < 3; ++k) { S.lo[k][at] = lo[k]; S.hi[k][at] = hi[k]; }
+        }
+        __syncwarp();
+        if (open) {
+            ref = S.ref[base + lane];
+            for (int k = 0; k < 3; ++k) { lo[k] = S.lo[k][base + lane]; hi[k] = S.hi[k][base + lane]; }
+            const bool in_left = lane - s0 < nleft;
+            node = in_left ? id : id + 1u;
+            area = in_left ? area6(bl, bl + 3) : area6(br, br + 3);
+            if (in_left) { sc = nleft; } else { s0 += nleft; sc -= nleft; }
+            open = sc >= 2u;
+        }
+        __syncwarp();
+    }
+}
+
+// Finishes the subtree of one small node per warp with its references and boxes
+// in shared memory: the same binned SAH splits and stable partitions down to 32
+// references, which finish_lanes takes from there.  Children wait on a per-warp
+// stack (every entry holds two or more references of a disjoint range, so at
+// most kSmall / 2 entries are live).  Splitting every node on its own, with
+// bins and three scans for two references as for a hundred, took 3.38 ms of the
+// 1.48 M-triangle terrain's build; 1.25 ms now.
+__global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __restrict__ small, uint32_t nsmall,
                                                             uint32_t* __restrict__ final_refs,
                                                             const float4* __restrict__ tlo,
                                                             const float4* __restrict__ thi, BNode* __restrict__ nodes,
                                                             Counters* cnt, int B, uint32_t max_leaf,
                                                             uint32_t max_nodes) {
-    __shared__ uint32_t s_refs[kSmallWarps][kSmall], s_tmp[kSmallWarps][kSmall];
-    __shared__ Bin s_bins[kSmallWarps][3 * kBins];
+    __shared__ SmallSet s_set[kSmallWarps];
+    __shared__ union { Bin bins[3 * kBins]; SmallSet tmp; } s_work[kSmallWarps];
     __shared__ uint32_t s_stack[kSmallWarps][kSmall / 2][3];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t ti = blockIdx.x * kSmallWarps + warp;
-    if (ti >= nsmall) return;   // whole warps; no block-wide barrier below
+    const uint32_t task = blockIdx.x * kSmallWarps + warp;
+    if (task >= nsmall) return;   // whole warps; no block-wide barrier below
     const uint32_t lt = (1u << lane) - 1u;
-    const Task root = small[ti];
+    const Task root = small[task];
     const uint32_t n0 = root.end - root.begin;
     if (n0 > kSmall) { if (lane == 0) atomicOr(&cnt->error, kErrStack); return; }
-    uint32_t* R = s_refs[warp];
-    uint32_t* T = s_tmp[warp];
-    Bin* SB = s_bins[warp];
-    for (uint32_t i = lane; i < n0; i += 32) R[i] = final_refs[root.begin + i];
+    SmallSet& S = s_set[warp];
+    SmallSet& T = s_work[warp].tmp;
+    Bin* SB = s_work[warp].bins;
+    for (uint32_t i = lane; i < n0; i += 32) {
+        const uint32_t r = final_refs[root.begin + i];
+        const float4 l = tlo[r], h = thi[r];
+        S.ref[i] = r;
+        S.lo[0][i] = l.x; S.lo[1][i] = l.y; S.lo[2][i] = l.z;
+        S.hi[0][i] = h.x; S.hi[1][i] = h.y; S.hi[2][i] = h.z;
+    }
     int sp = 0;
     if (lane == 0) { s_stack[warp][0][0] = root.node; s_stack[warp][0][1] = 0; s_stack[warp][0][2] = n0; }
     sp = 1;
     __syncwarp();
-    bool failed = false;
-    while (sp > 0 && !failed) {
+    while (sp > 0) {
         --sp;
         const uint32_t node = s_stack[warp][sp][0], b = s_stack[warp][sp][1], e = s_stack[warp][sp][2];
         __syncwarp();
         const uint32_t n = e - b;
+        const float area = area6(nodes[node].lo, nodes[node].hi);
+        if (n <= 32u) {
+            finish_lanes(S, b, n, root.begin, node, area, nodes, cnt, B, max_leaf, max_nodes);
+            __syncwarp();
+            continue;
+        }
         // centroid bounds
         Task tk;
         tk.node = node;
         tk.begin = b;
         tk.end = e;
         float cl[3] = {INFINITY, INFINITY, INFINITY}, chv[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (uint32_t i = b + lane; i < e; i += 32) {
-            uint32_t r = R[i];
-            float4 l = tlo[r], h = thi[r];
+        for (uint32_t i = b + lane; i < e; i += 32)
             for (int a = 0; a < 3; ++a) {
-                float c = centroid(l, h, a);
+                const float c = 0.5f * (S.lo[a][i] + S.hi[a][i]);
                 cl[a] = fminf(cl[a], c);
                 chv[a] = fmaxf(chv[a], c);
             }
-        }
         for (int a = 0; a < 3; ++a) { tk.clo[a] = warp_min(cl[a]); tk.chi[a] = warp_max(chv[a]); }
         // bins
         for (int i = lane; i < 3 * kBins; i += 32) {
@@ -565,12 +741,11 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(const Task* __restri
         float sc[3];
         for (int a = 0; a < 3; ++a) sc[a] = axis_scale(tk, a, B);
         for (uint32_t i = b + lane; i < e; i += 32) {
-            uint32_t r = R[i];
-            float4 l = tlo[r], h = thi[r];
-            const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)}, kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
+            uint32_t kl[3], kh[3];
+            for (int k = 0; k < 3; ++k) { kl[k] = fkey(S.lo[k][i]); kh[k] = fkey(S.hi[k][i]); }
             for (int a = 0; a < 3; ++a) {
                 if (!(sc[a] > 0.0f)) continue;
-                Bin& bb = SB[a * kBins + bin_of(centroid(l, h, a), tk.clo[a], sc[a], B)];
+                Bin& bb = SB[a * kBins + bin_of(0.5f * (S.lo[a][i] + S.hi[a][i]), tk.clo[a], sc[a], B)];
                 atomicAdd(&bb.cnt, 1u);
                 for (int k = 0; k < 3; ++k) { atomicMin(&bb.lo[k], kl[k]); atomicMax(&bb.hi[k], kh[k]); }
             }
@@ -584,73 +759,71 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(const Task* __restri
             z.cnt = 0;
             return lane < B ? SB[a * kBins + lane] : z;
         }, &bbin, &bnl, &best);
-        const BNode nd = nodes[node];
-        Split s = decide(bax, bbin, bnl, best, n, area6(nd.lo, nd.hi), max_leaf);
+        const Split s = decide(bax, bbin, bnl, best, n, area, max_leaf);   // never a leaf: leaves hold at most two
         __syncwarp();
-        if (s.leaf) continue;
-        if (s.axis >= 0) {   // stable partition through T
-            uint32_t lc = 0, rc = 0;
-            for (uint32_t base = b; base < e; base += 32) {
-                const uint32_t i = base + lane;
-                const bool act = i < e;
-                uint32_t r = act ? R[i] : 0u;
-                bool left = false;
-                if (act) left = goes_left(tk, s, i, tlo[r], thi[r], B);
-                const bool right = act && !left;
-                const uint32_t wl = __ballot_sync(0xffffffffu, left), wr = __ballot_sync(0xffffffffu, right);
-                if (left) T[b + lc + __popc(wl & lt)] = r;
-                if (right) T[b + s.nl + rc + __popc(wr & lt)] = r;
-                lc += __popc(wl);
-                rc += __popc(wr);
+        // stable partition through T, with the children's boxes
+        float bx[2][6];
+        for (int c = 0; c < 2; ++c)
+            for (int k = 0; k < 3; ++k) { bx[c][k] = INFINITY; bx[c][3 + k] = -INFINITY; }
+        uint32_t lc = 0, rc = 0;
+        for (uint32_t base = b; base < e; base += 32) {
+            const uint32_t i = base + lane;
+            const bool act = i < e;
+            float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
+            bool left = false;
+            if (act) {
+                for (int k = 0; k < 3; ++k) { lo[k] = S.lo[k][i]; hi[k] = S.hi[k][i]; }
+                if (s.axis < 0) {
+                    left = i - b < s.nl;
+                } else {
+                    const int a = s.axis;
+                    const float c = a == 0 ? 0.5f * (lo[0] + hi[0]) : a == 1 ? 0.5f * (lo[1] + hi[1]) : 0.5f * (lo[2] + hi[2]);
+                    left = bin_of(c, tk.clo[a], sc[a], B) < s.bin;
+                }
             }
-            __syncwarp();
-            for (uint32_t i = b + lane; i < e; i += 32) R[i] = T[i];
-            __syncwarp();
+            const bool right = act && !left;
+            const uint32_t wl = __ballot_sync(0xffffffffu, left), wr = __ballot_sync(0xffffffffu, right);
+            if (act) {
+                const uint32_t at = left ? lc + __popc(wl & lt) : s.nl + rc + __popc(wr & lt);
+                T.ref[at] = S.ref[i];
+                for (int k = 0; k < 3; ++k) {
+                    T.lo[k][at] = lo[k];
+                    T.hi[k][at] = hi[k];
+                    if (left) { bx[0][k] = fminf(bx[0][k], lo[k]); bx[0][3 + k] = fmaxf(bx[0][3 + k], hi[k]); }
+                    else { bx[1][k] = fminf(bx[1][k], lo[k]); bx[1][3 + k] = fmaxf(bx[1][3 + k], hi[k]); }
+                }
+            }
+            lc += __popc(wl);
+            rc += __popc(wr);
         }
+        __syncwarp();
+        for (uint32_t i = lane; i < n; i += 32) {
+            S.ref[b + i] = T.ref[i];
+            for (int k = 0; k < 3; ++k) { S.lo[k][b + i] = T.lo[k][i]; S.hi[k][b + i] = T.hi[k][i]; }
+        }
+        for (int c = 0; c < 2; ++c)
+            for (int k = 0; k < 3; ++k) { bx[c][k] = warp_min(bx[c][k]); bx[c][3 + k] = warp_max(bx[c][3 + k]); }
         const uint32_t mid = b + s.nl;
-        // children's boxes
-        float bl[2][6];
-        for (int c = 0; c < 2; ++c) {
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-            const uint32_t cb = c ? mid : b, ce = c ? e : mid;
-            for (uint32_t i = cb + lane; i < ce; i += 32) {
-                float4 l = tlo[R[i]], h = thi[R[i]];
-                lo[0] = fminf(lo[0], l.x); lo[1] = fminf(lo[1], l.y); lo[2] = fminf(lo[2], l.z);
-                hi[0] = fmaxf(hi[0], h.x); hi[1] = fmaxf(hi[1], h.y); hi[2] = fmaxf(hi[2], h.z);
-            }
-            for (int k = 0; k < 3; ++k) { bl[c][k] = warp_min(lo[k]); bl[c][3 + k] = warp_max(hi[k]); }
-        }
         uint32_t id = 0;
         if (lane == 0) id = atomicAdd(&cnt->nodes, 2u);
         id = __shfl_sync(0xffffffffu, id, 0);
         if (id + 2u > max_nodes) {
             if (lane == 0) atomicOr(&cnt->error, kErrNodes);
-            failed = true;
-            break;
+            return;
         }
         if (lane == 0) {
             nodes[node].left = id;
             nodes[node].right = id + 1u;
-            for (int c = 0; c < 2; ++c) {
-                BNode cn;
-                for (int k = 0; k < 3; ++k) { cn.lo[k] = bl[c][k]; cn.hi[k] = bl[c][3 + k]; }
-                cn.left = cn.right = kNone;
-                cn.first = root.begin + (c ? mid : b);
-                cn.count = c ? e - mid : mid - b;
-                cn.parent = node;
-                cn.pad = 0;
-                nodes[id + c] = cn;
-            }
+            write_child(nodes, id, node, bx[0], bx[0] + 3, root.begin + b, s.nl);
+            write_child(nodes, id + 1u, node, bx[1], bx[1] + 3, root.begin + mid, e - mid);
         }
         // push right then left (left is finished first); single-reference children are leaves
-        const uint32_t ranges[2][2] = {{mid, e}, {b, mid}};
         for (int c = 0; c < 2; ++c) {
-            const uint32_t cb = ranges[c][0], ce = ranges[c][1];
+            const uint32_t cb = c == 0 ? mid : b, ce = c == 0 ? e : mid;
             if (ce - cb <= 1u) continue;
             if (sp >= (int)(kSmall / 2)) {
                 if (lane == 0) atomicOr(&cnt->error, kErrStack);
-                failed = true;
-                break;
+                return;
             }
             if (lane == 0) {
                 s_stack[warp][sp][0] = id + (c == 0 ? 1u : 0u);
@@ -662,7 +835,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_small(const Task* __restri
         __syncwarp();
     }
     __syncwarp();
-    for (uint32_t i = lane; i < n0; i += 32) final_refs[root.begin + i] = R[i];
+    for (uint32_t i = lane; i < n0; i += 32) final_refs[root.begin + i] = S.ref[i];
 }
 
 // ------------------------------------------------------------ phase 3 ----
