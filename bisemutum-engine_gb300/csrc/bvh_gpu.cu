@@ -56,7 +56,7 @@ constexpr uint32_t kKeyHi = 0u;            // initial key of a maximum
 // error bits of Counters::error
 enum : uint32_t {
     kErrIndex = 1, kErrFinite = 2, kErrNodes = 4, kErrGather = 8, kErrLeaf = 16, kErrStack = 32, kErrClimb = 64,
-    kErrWide = 128
+    kErrWide = 128, kErrPartition = 256
 };
 
 struct BNode {                 // binary node
@@ -70,17 +70,15 @@ struct BNode {                 // binary node
 static_assert(sizeof(BNode) == 48, "BNode must be 48 bytes");
 
 struct Task {                  // a node still to split: its reference range and centroid bounds
-    uint32_t node, begin, end, pad;
+    uint32_t node, begin, end;
+    uint32_t aux;              // in a level: its first chunk; in the small list: the reference buffer (0 or 1)
     float clo[3], chi[3];
-};
-struct Chunk {                 // a CTA's share of one task in a level pass
-    uint32_t task, begin, end, pad;
-    uint32_t left_base, right_base, pad2[2];
 };
 struct Bin { uint32_t cnt, lo[3], hi[3]; };      // box as ordered float keys
 struct Split { int axis; int bin; uint32_t leaf; uint32_t nl; };
+struct ChunkBins { uint16_t below[3][kBins]; };   // a chunk's references in the bins below each, per axis
 struct ChildAcc { uint32_t box[2][6]; uint32_t cen[2][6]; };   // per side: lo xyz, hi xyz (keys)
-struct Counters { uint32_t nodes, next_tasks, small_tasks, error, ni_total, nt_total, pad[2]; };
+struct Counters { uint32_t nodes, tasks[2], chunks, small_tasks, error, ni_total, nt_total; };
 struct WideRec { uint32_t child[8]; uint32_t ni, nt; };     // binary node per slot (kNone: empty slot)
 
 // Order-preserving map of floats to unsigned keys (-0 below +0), so that
@@ -124,7 +122,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // ------------------------------------------------------------ phase 1 ----
 __global__ void __launch_bounds__(256) k_tri_boxes(const float* __restrict__ pos, uint32_t nv,
                                                    const uint32_t* __restrict__ idx, uint32_t nt,
-                                                   float4* __restrict__ tlo, float4* __restrict__ thi,
+                                                   float4* __restrict__ box, uint32_t* __restrict__ refs,
                                                    uint32_t* __restrict__ gkeys, Counters* cnt) {
     __shared__ float s_red[8][12];
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -142,8 +140,9 @@ __global__ void __launch_bounds__(256) k_tri_boxes(const float* __restrict__ pos
                 hi[k] = fmaxf(hi[k], p);
             }
         }
-        tlo[t] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-        thi[t] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        box[2 * (size_t)t] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+        box[2 * (size_t)t + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        refs[t] = t;
         for (int k = 0; k < 3; ++k) {
             float c = 0.5f * (lo[k] + hi[k]);
             v[k] = lo[k]; v[3 + k] = hi[k]; v[6 + k] = c; v[9 + k] = c;
@@ -165,70 +164,144 @@ __global__ void __launch_bounds__(256) k_tri_boxes(const float* __restrict__ pos
     }
 }
 
-__global__ void k_iota(uint32_t* a, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = i;
-}
-
 // ------------------------------------------------------------ phase 2 ----
-__global__ void k_bins_init(Bin* bins, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Bin b;
-    b.cnt = 0;
-    for (int k = 0; k < 3; ++k) { b.lo[k] = kKeyLo; b.hi[k] = kKeyHi; }
-    bins[i] = b;
+// The passes of a level run on what the level before left on the device (its
+// tasks and their number), so the host queues the levels without waiting.  A
+// block takes chunks of at most kChunk references of one task in turn.
+__global__ void k_bins_init(Bin* bins, uint32_t n, ChildAcc* acc, uint32_t nacc) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        Bin b;
+        b.cnt = 0;
+        for (int k = 0; k < 3; ++k) { b.lo[k] = kKeyLo; b.hi[k] = kKeyHi; }
+        bins[i] = b;
+    }
+    if (i < nacc) {
+        ChildAcc a;
+        for (int s = 0; s < 2; ++s)
+            for (int k = 0; k < 3; ++k) {
+                a.box[s][k] = kKeyLo; a.box[s][3 + k] = kKeyHi;
+                a.cen[s][k] = kKeyLo; a.cen[s][3 + k] = kKeyHi;
+            }
+        acc[i] = a;
+    }
 }
 
-__global__ void k_acc_init(ChildAcc* acc, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    ChildAcc a;
-    for (int s = 0; s < 2; ++s)
-        for (int k = 0; k < 3; ++k) {
-            a.box[s][k] = kKeyLo; a.box[s][3 + k] = kKeyHi;
-            a.cen[s][k] = kKeyLo; a.cen[s][3 + k] = kKeyHi;
+// First chunk of every task (one block: a scan over the tasks) and the task of every chunk.
+__global__ void __launch_bounds__(1024) k_level_chunks(Task* __restrict__ tasks, uint32_t* __restrict__ chunk_task,
+                                                       uint32_t chunk_cap, Counters* cnt, int cur) {
+    __shared__ uint32_t s_w[32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nt = cnt->error ? 0u : cnt->tasks[cur];
+    uint32_t carry = 0;
+    __syncthreads();   // every thread has read the counters that thread 0 writes below
+    for (uint32_t base = 0; base < nt; base += blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t n = i < nt ? (tasks[i].end - tasks[i].begin + kChunk - 1u) / kChunk : 0u;
+        uint32_t x = n;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-    acc[i] = a;
+        if (lane == 31u) s_w[warp] = x;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+        for (uint32_t w = 0; w < 32; ++w) { const uint32_t v = s_w[w]; before += w < warp ? v : 0u; all += v; }
+        __syncthreads();
+        const uint32_t first = carry + before + x - n;
+        if (i < nt) {
+            tasks[i].aux = first;
+            if (first + n > chunk_cap) atomicOr(&cnt->error, kErrNodes);
+            else
+                for (uint32_t c = 0; c < n; ++c) chunk_task[first + c] = i;
+        }
+        carry += all;
+    }
+    if (threadIdx.x == 0) { cnt->chunks = min(carry, chunk_cap); cnt->tasks[cur ^ 1] = 0u; }
 }
 
-// Bins one chunk of one task's references by centroid, per axis, into shared
-// bins, then merges the non-empty bins into the task's bins.
-__global__ void __launch_bounds__(kLevelThreads) k_bin(const Chunk* __restrict__ chunks,
+// Adds a warp's references to one axis' shared bins.  Neighbouring references
+// mostly share a bin (they are in input order within a node), and 32 atomics on
+// one address take turns, so up to three groups of lanes with a common bin are
+// reduced in registers first.
+__device__ __forceinline__ void bin_axis(Bin* sb, bool act, uint32_t bin, const uint32_t* kl, const uint32_t* kh) {
+    uint32_t rest = __ballot_sync(0xffffffffu, act);
+    for (int round = 0; round < 3 && rest != 0u; ++round) {
+        const int leader = __ffs(rest) - 1;
+        const uint32_t lb = __shfl_sync(0xffffffffu, bin, leader);
+        const uint32_t m = __ballot_sync(0xffffffffu, bin == lb) & rest;
+        if (__popc(m) < 4) break;
+        if ((m >> (threadIdx.x & 31u)) & 1u) {
+            uint32_t lo[3], hi[3];
+            for (int k = 0; k < 3; ++k) { lo[k] = __reduce_min_sync(m, kl[k]); hi[k] = __reduce_max_sync(m, kh[k]); }
+            if ((int)(threadIdx.x & 31u) == leader) {
+                Bin& b = sb[lb];
+                atomicAdd(&b.cnt, (uint32_t)__popc(m));
+                for (int k = 0; k < 3; ++k) { atomicMin(&b.lo[k], lo[k]); atomicMax(&b.hi[k], hi[k]); }
+            }
+        }
+        rest &= ~m;
+    }
+    if ((rest >> (threadIdx.x & 31u)) & 1u) {
+        Bin& b = sb[bin];
+        atomicAdd(&b.cnt, 1u);
+        for (int k = 0; k < 3; ++k) { atomicMin(&b.lo[k], kl[k]); atomicMax(&b.hi[k], kh[k]); }
+    }
+}
+
+// Bins a chunk's references by centroid, per axis, into shared bins, merges the
+// non-empty bins into the task's and leaves the chunk's running counts for the
+// partition.
+__global__ void __launch_bounds__(kLevelThreads) k_bin(const uint32_t* __restrict__ chunk_task,
                                                        const Task* __restrict__ tasks,
                                                        const uint32_t* __restrict__ refs,
-                                                       const float4* __restrict__ tlo,
-                                                       const float4* __restrict__ thi, Bin* __restrict__ gbins,
-                                                       int B) {
+                                                       const float4* __restrict__ box, Bin* __restrict__ gbins,
+                                                       ChunkBins* __restrict__ cbins, const Counters* cnt, int B) {
     __shared__ Bin sb[3 * kBins];
-    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) {
-        sb[i].cnt = 0;
-        for (int k = 0; k < 3; ++k) { sb[i].lo[k] = kKeyLo; sb[i].hi[k] = kKeyHi; }
-    }
-    __syncthreads();
-    const Chunk ch = chunks[blockIdx.x];
-    const Task tk = tasks[ch.task];
-    float sc[3];
-    for (int a = 0; a < 3; ++a) sc[a] = axis_scale(tk, a, B);
-    for (uint32_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
-        const uint32_t r = refs[i];
-        const float4 l = tlo[r], h = thi[r];
-        const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)}, kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
-        for (int a = 0; a < 3; ++a) {
-            if (!(sc[a] > 0.0f)) continue;
-            Bin& b = sb[a * kBins + bin_of(centroid(l, h, a), tk.clo[a], sc[a], B)];
-            atomicAdd(&b.cnt, 1u);
-            for (int k = 0; k < 3; ++k) { atomicMin(&b.lo[k], kl[k]); atomicMax(&b.hi[k], kh[k]); }
+    const uint32_t nch = cnt->error ? 0u : cnt->chunks;
+    for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
+        for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) {
+            sb[i].cnt = 0;
+            for (int k = 0; k < 3; ++k) { sb[i].lo[k] = kKeyLo; sb[i].hi[k] = kKeyHi; }
         }
-    }
-    __syncthreads();
-    Bin* g = gbins + (size_t)ch.task * 3 * kBins;
-    for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) {
-        if (sb[i].cnt == 0) continue;
-        atomicAdd(&g[i].cnt, sb[i].cnt);
-        for (int k = 0; k < 3; ++k) { atomicMin(&g[i].lo[k], sb[i].lo[k]); atomicMax(&g[i].hi[k], sb[i].hi[k]); }
+        __syncthreads();
+        const uint32_t ti = chunk_task[c];
+        const Task tk = tasks[ti];
+        const uint32_t begin = tk.begin + (c - tk.aux) * kChunk, end = min(tk.end, begin + kChunk);
+        float sc[3];
+        for (int a = 0; a < 3; ++a) sc[a] = axis_scale(tk, a, B);
+        for (uint32_t base = begin; base < end; base += blockDim.x) {
+            const uint32_t i = base + threadIdx.x;
+            const bool act = i < end;
+            float4 l = make_float4(0, 0, 0, 0), h = l;
+            if (act) {
+                const uint32_t r = refs[i];
+                l = box[2 * (size_t)r];
+                h = box[2 * (size_t)r + 1];
+            }
+            const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)}, kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
+            for (int a = 0; a < 3; ++a) {
+                if (!(sc[a] > 0.0f)) continue;   // the same for the whole block
+                bin_axis(sb + a * kBins, act, act ? (uint32_t)bin_of(centroid(l, h, a), tk.clo[a], sc[a], B) : 255u, kl, kh);
+            }
+        }
+        __syncthreads();
+        Bin* g = gbins + (size_t)ti * 3 * kBins;
+        for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) {
+            const uint32_t n = sb[i].cnt;
+            uint32_t x = n;   // a warp holds one axis' bins
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if ((threadIdx.x & 31u) >= o) x += y;
+            }
+            cbins[c].below[i / kBins][i % kBins] = (uint16_t)(x - n);
+            if (n == 0) continue;
+            atomicAdd(&g[i].cnt, n);
+            for (int k = 0; k < 3; ++k) { atomicMin(&g[i].lo[k], sb[i].lo[k]); atomicMax(&g[i].hi[k], sb[i].hi[k]); }
+        }
+        __syncthreads();
     }
 }
+static_assert(kBins == 32 && kChunk < 65536, "a warp scans an axis' bins; a chunk's counts fit 16 bits");
 
 // The least-cost split over three axes of binned SAH (bvh_build.cpp Builder::build):
 // cost(split before bin b) = area(left) * n_left + area(right) * n_right, axes
@@ -315,23 +388,51 @@ __device__ __forceinline__ Split decide(int bax, int bbin, uint32_t bnl, float b
     return s;
 }
 
-__global__ void k_split(const Task* __restrict__ tasks, uint32_t ntasks, const Bin* __restrict__ gbins,
-                        const BNode* __restrict__ nodes, Split* __restrict__ splits, int B, uint32_t max_leaf) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The split of every task (a warp each, its bins cleared for the next level) and
+// where its chunks' left references go.
+__global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins, const ChunkBins* __restrict__ cbins,
+                        const BNode* __restrict__ nodes, Split* __restrict__ splits, uint32_t* __restrict__ left_base,
+                        Counters* cnt, int cur, int B, uint32_t max_leaf) {
     const int lane = threadIdx.x & 31;
-    if (w >= ntasks) return;   // whole warps
-    const Task tk = tasks[w];
-    int bbin;
-    uint32_t bnl;
-    float best;
-    int bax = warp_best_split(tk, B, [&](int a) {
-        Bin e;
-        e.cnt = 0;
-        return lane < B ? gbins[((size_t)w * 3 + a) * kBins + lane] : e;
-    }, &bbin, &bnl, &best);
-    const BNode nd = nodes[tk.node];
-    Split s = decide(bax, bbin, bnl, best, tk.end - tk.begin, area6(nd.lo, nd.hi), max_leaf);
-    if (lane == 0) splits[w] = s;
+    const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur], warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nt; w += warps) {
+        const Task tk = tasks[w];
+        int bbin;
+        uint32_t bnl;
+        float best;
+        int bax = warp_best_split(tk, B, [&](int a) {
+            Bin e;
+            e.cnt = 0;
+            return lane < B ? gbins[((size_t)w * 3 + a) * kBins + lane] : e;
+        }, &bbin, &bnl, &best);
+        Bin z;
+        z.cnt = 0;
+        for (int k = 0; k < 3; ++k) { z.lo[k] = kKeyLo; z.hi[k] = kKeyHi; }
+        for (int a = 0; a < 3; ++a) gbins[((size_t)w * 3 + a) * kBins + lane] = z;
+        const BNode nd = nodes[tk.node];
+        const Split s = decide(bax, bbin, bnl, best, tk.end - tk.begin, area6(nd.lo, nd.hi), max_leaf);
+        if (lane == 0) splits[w] = s;
+        const uint32_t n = (tk.end - tk.begin + kChunk - 1u) / kChunk;
+        uint32_t carry = 0;
+        for (uint32_t base = 0; base < n; base += 32) {
+            const uint32_t c = base + lane;
+            uint32_t left = 0;
+            if (c < n) {
+                const uint32_t size = min(kChunk, tk.end - tk.begin - c * kChunk);
+                if (s.leaf) left = size;
+                else if (s.axis < 0) left = s.nl > c * kChunk ? min(size, s.nl - c * kChunk) : 0u;
+                else left = cbins[tk.aux + c].below[s.axis][s.bin];
+            }
+            uint32_t x = left;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (c < n) left_base[tk.aux + c] = tk.begin + carry + x - left;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0 && carry != s.nl) atomicOr(&cnt->error, kErrPartition);
+    }
 }
 
 __device__ __forceinline__ bool goes_left(const Task& tk, const Split& sp, uint32_t i, const float4& l,
@@ -342,167 +443,152 @@ __device__ __forceinline__ bool goes_left(const Task& tk, const Split& sp, uint3
     return bin_of(centroid(l, h, a), tk.clo[a], axis_scale(tk, a, B), B) < sp.bin;
 }
 
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_tmp) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s_tmp[threadIdx.x >> 5] = v;
-    __syncthreads();
-    uint32_t t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_tmp[w];
-    __syncthreads();
-    return t;
-}
-
-__global__ void __launch_bounds__(kLevelThreads) k_count_left(const Chunk* __restrict__ chunks,
-                                                              const Task* __restrict__ tasks,
-                                                              const Split* __restrict__ splits,
-                                                              const uint32_t* __restrict__ refs,
-                                                              const float4* __restrict__ tlo,
-                                                              const float4* __restrict__ thi,
-                                                              uint32_t* __restrict__ chunk_left, int B) {
-    __shared__ uint32_t s_tmp[32];
-    const Chunk ch = chunks[blockIdx.x];
-    const Task tk = tasks[ch.task];
-    const Split sp = splits[ch.task];
-    uint32_t n = 0;
-    for (uint32_t i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
-        uint32_t r = refs[i];
-        n += goes_left(tk, sp, i, tlo[r], thi[r], B) ? 1u : 0u;
-    }
-    n = block_sum(n, s_tmp);
-    if (threadIdx.x == 0) chunk_left[blockIdx.x] = n;
-}
-
-// Stable partition of one chunk: left references to left_base.., right ones to
-// right_base.. (both in chunk order); the children's boxes and centroid bounds
-// are reduced over the block and merged into the task's accumulator.
-__global__ void __launch_bounds__(kLevelThreads) k_partition(const Chunk* __restrict__ chunks,
+// Stable partition of a chunk: its left references from left_base on, its right
+// ones behind the task's left part (both in chunk order); the children's boxes
+// and centroid bounds are reduced over the block and merged into the task's.
+__global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __restrict__ chunk_task,
                                                              const Task* __restrict__ tasks,
                                                              const Split* __restrict__ splits,
+                                                             const uint32_t* __restrict__ left_base,
                                                              const uint32_t* __restrict__ in,
                                                              uint32_t* __restrict__ out,
-                                                             const float4* __restrict__ tlo,
-                                                             const float4* __restrict__ thi,
-                                                             ChildAcc* __restrict__ acc, int B) {
+                                                             const float4* __restrict__ box,
+                                                             ChildAcc* __restrict__ acc, const Counters* cnt, int B) {
     __shared__ uint32_t s_wl[kLevelThreads / 32], s_wr[kLevelThreads / 32];
     __shared__ float s_red[kLevelThreads / 32][24];
-    const Chunk ch = chunks[blockIdx.x];
-    const Task tk = tasks[ch.task];
-    const Split sp = splits[ch.task];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    float v[24];   // side s: box lo(3) hi(3), centroid lo(3) hi(3) at 12 s
-    for (int s = 0; s < 2; ++s)
-        for (int k = 0; k < 3; ++k) {
-            v[12 * s + k] = v[12 * s + 6 + k] = INFINITY;
-            v[12 * s + 3 + k] = v[12 * s + 9 + k] = -INFINITY;
-        }
-    uint32_t lb = ch.left_base, rb = ch.right_base;
-    for (uint32_t base = ch.begin; base < ch.end; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool act = i < ch.end;
-        uint32_t r = 0;
-        float4 l = make_float4(0, 0, 0, 0), h = l;
-        bool left = false;
-        if (act) {
-            r = in[i];
-            l = tlo[r];
-            h = thi[r];
-            left = goes_left(tk, sp, i, l, h, B);
-        }
-        const bool right = act && !left;
-        const uint32_t wl = __ballot_sync(0xffffffffu, left), wr = __ballot_sync(0xffffffffu, right);
-        if (lane == 0) { s_wl[warp] = __popc(wl); s_wr[warp] = __popc(wr); }
-        __syncthreads();
-        uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
-        for (int w = 0; w < nw; ++w) {
-            if (w < warp) { pl += s_wl[w]; pr += s_wr[w]; }
-            tl += s_wl[w];
-            tr += s_wr[w];
-        }
-        if (left) out[lb + pl + __popc(wl & lt)] = r;
-        if (right) out[rb + pr + __popc(wr & lt)] = r;
-        lb += tl;
-        rb += tr;
-        __syncthreads();
-        if (act) {
-            float* s = v + (left ? 0 : 12);
-            const float lo[3] = {l.x, l.y, l.z}, hi[3] = {h.x, h.y, h.z};
+    const uint32_t nch = cnt->error ? 0u : cnt->chunks;   // after an error the offsets may be wrong
+    for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
+        const uint32_t ti = chunk_task[c];
+        const Task tk = tasks[ti];
+        const Split sp = splits[ti];
+        const uint32_t begin = tk.begin + (c - tk.aux) * kChunk, end = min(tk.end, begin + kChunk);
+        float v[24];   // side s: box lo(3) hi(3), centroid lo(3) hi(3) at 12 s
+        for (int s = 0; s < 2; ++s)
             for (int k = 0; k < 3; ++k) {
-                float c = 0.5f * (lo[k] + hi[k]);
-                s[k] = fminf(s[k], lo[k]);
-                s[3 + k] = fmaxf(s[3 + k], hi[k]);
-                s[6 + k] = fminf(s[6 + k], c);
-                s[9 + k] = fmaxf(s[9 + k], c);
+                v[12 * s + k] = v[12 * s + 6 + k] = INFINITY;
+                v[12 * s + 3 + k] = v[12 * s + 9 + k] = -INFINITY;
+            }
+        uint32_t lb = left_base[c], rb = tk.begin + sp.nl + (begin - lb);
+        for (uint32_t base = begin; base < end; base += blockDim.x) {
+            const uint32_t i = base + threadIdx.x;
+            const bool act = i < end;
+            uint32_t r = 0;
+            float4 l = make_float4(0, 0, 0, 0), h = l;
+            bool left = false;
+            if (act) {
+                r = in[i];
+                l = box[2 * (size_t)r];
+                h = box[2 * (size_t)r + 1];
+                left = goes_left(tk, sp, i, l, h, B);
+            }
+            const bool right = act && !left;
+            const uint32_t wl = __ballot_sync(0xffffffffu, left), wr = __ballot_sync(0xffffffffu, right);
+            if (lane == 0) { s_wl[warp] = __popc(wl); s_wr[warp] = __popc(wr); }
+            __syncthreads();
+            uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
+            for (int w = 0; w < nw; ++w) {
+                if (w < warp) { pl += s_wl[w]; pr += s_wr[w]; }
+                tl += s_wl[w];
+                tr += s_wr[w];
+            }
+            if (left) out[lb + pl + __popc(wl & lt)] = r;
+            if (right) out[rb + pr + __popc(wr & lt)] = r;
+            lb += tl;
+            rb += tr;
+            __syncthreads();
+            if (act) {
+                const float lo[3] = {l.x, l.y, l.z}, hi[3] = {h.x, h.y, h.z};
+                for (int k = 0; k < 3; ++k) {
+                    const float cc = 0.5f * (lo[k] + hi[k]);
+                    if (left) {
+                        v[k] = fminf(v[k], lo[k]); v[3 + k] = fmaxf(v[3 + k], hi[k]);
+                        v[6 + k] = fminf(v[6 + k], cc); v[9 + k] = fmaxf(v[9 + k], cc);
+                    } else {
+                        v[12 + k] = fminf(v[12 + k], lo[k]); v[15 + k] = fmaxf(v[15 + k], hi[k]);
+                        v[18 + k] = fminf(v[18 + k], cc); v[21 + k] = fmaxf(v[21 + k], cc);
+                    }
+                }
             }
         }
-    }
-    for (int k = 0; k < 24; ++k) {
-        const bool mx = (k % 6) >= 3;
-        v[k] = mx ? warp_max(v[k]) : warp_min(v[k]);
-        if (lane == 0) s_red[warp][k] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 24) {
-        const int k = threadIdx.x;
-        const bool mx = (k % 6) >= 3;
-        float r = s_red[0][k];
-        for (int w = 1; w < nw; ++w) r = mx ? fmaxf(r, s_red[w][k]) : fminf(r, s_red[w][k]);
-        if (r == INFINITY || r == -INFINITY) return;   // that side is empty in this chunk
-        const int side = k / 12, j = k % 12;
-        uint32_t* dst = j < 6 ? &acc[ch.task].box[side][j] : &acc[ch.task].cen[side][j - 6];
-        if (mx) atomicMax(dst, fkey(r)); else atomicMin(dst, fkey(r));
+        for (int k = 0; k < 24; ++k) {
+            const uint32_t key = fkey(v[k]);
+            const bool mx = (k % 6) >= 3;
+            const uint32_t m = mx ? __reduce_max_sync(0xffffffffu, key) : __reduce_min_sync(0xffffffffu, key);
+            if (lane == 0) s_red[warp][k] = funkey(m);
+        }
+        __syncthreads();
+        if (threadIdx.x < 24) {
+            const int k = threadIdx.x;
+            const bool mx = (k % 6) >= 3;
+            float r = s_red[0][k];
+            for (int w = 1; w < nw; ++w) r = mx ? fmaxf(r, s_red[w][k]) : fminf(r, s_red[w][k]);
+            if (r != INFINITY && r != -INFINITY) {   // else that side is empty in this chunk
+                const int side = k / 12, j = k % 12;
+                uint32_t* dst = j < 6 ? &acc[ti].box[side][j] : &acc[ti].cen[side][j - 6];
+                if (mx) atomicMax(dst, fkey(r)); else atomicMin(dst, fkey(r));
+            }
+        }
+        __syncthreads();
     }
 }
 
 // Children of every split task: two binary nodes each; a child of one triangle
-// is a leaf, a child of at most kSmall goes to the small list, any other to the
-// next level.  Leaves and small children copy their references to `final`.
-__global__ void k_make_children(const Task* __restrict__ tasks, uint32_t ntasks, const Split* __restrict__ splits,
-                                const ChildAcc* __restrict__ acc, const uint32_t* __restrict__ refs,
+// is a leaf, a child of at most kSmall goes to the small list with the buffer
+// that holds its references, any other to the next level.
+__global__ void k_make_children(const Task* __restrict__ tasks, const Split* __restrict__ splits,
+                                ChildAcc* __restrict__ acc, const uint32_t* __restrict__ refs,
                                 BNode* __restrict__ nodes, uint32_t* __restrict__ final_refs, Task* __restrict__ next,
-                                uint32_t next_cap, Task* __restrict__ small, uint32_t small_cap, Counters* cnt,
+                                uint32_t next_cap, Task* __restrict__ small, uint32_t small_cap, Counters* cnt, int cur,
                                 uint32_t max_nodes) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ntasks) return;
-    const Task tk = tasks[i];
-    const Split sp = splits[i];
-    if (sp.leaf) {
-        for (uint32_t k = tk.begin; k < tk.end; ++k) final_refs[k] = refs[k];
-        return;
-    }
-    const uint32_t id = atomicAdd(&cnt->nodes, 2u);
-    if (id + 2u > max_nodes) { atomicOr(&cnt->error, kErrNodes); return; }
-    nodes[tk.node].left = id;
-    nodes[tk.node].right = id + 1u;
-    const ChildAcc& a = acc[i];
-    for (int s = 0; s < 2; ++s) {
-        const uint32_t cb = s ? tk.begin + sp.nl : tk.begin, ce = s ? tk.end : tk.begin + sp.nl;
-        BNode n;
-        for (int k = 0; k < 3; ++k) { n.lo[k] = funkey(a.box[s][k]); n.hi[k] = funkey(a.box[s][3 + k]); }
-        n.left = n.right = kNone;
-        n.first = cb;
-        n.count = ce - cb;
-        n.parent = tk.node;
-        n.pad = 0;
-        nodes[id + s] = n;
-        if (n.count <= 1u) {
-            for (uint32_t k = cb; k < ce; ++k) final_refs[k] = refs[k];
+    const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
+        const Task tk = tasks[i];
+        const Split sp = splits[i];
+        if (sp.leaf) {   // cannot be: a task holds more than kSmall references
+            atomicOr(&cnt->error, kErrLeaf);
             continue;
         }
-        Task c;
-        c.node = id + s;
-        c.begin = cb;
-        c.end = ce;
-        c.pad = 0;
-        for (int k = 0; k < 3; ++k) { c.clo[k] = funkey(a.cen[s][k]); c.chi[k] = funkey(a.cen[s][3 + k]); }
-        if (n.count <= kSmall) {
-            for (uint32_t k = cb; k < ce; ++k) final_refs[k] = refs[k];
-            uint32_t slot = atomicAdd(&cnt->small_tasks, 1u);
-            if (slot < small_cap) small[slot] = c; else atomicOr(&cnt->error, kErrNodes);
-        } else {
-            uint32_t slot = atomicAdd(&cnt->next_tasks, 1u);
-            if (slot < next_cap) next[slot] = c; else atomicOr(&cnt->error, kErrNodes);
+        const uint32_t id = atomicAdd(&cnt->nodes, 2u);
+        if (id + 2u > max_nodes) { atomicOr(&cnt->error, kErrNodes); continue; }
+        nodes[tk.node].left = id;
+        nodes[tk.node].right = id + 1u;
+        const ChildAcc a = acc[i];
+        ChildAcc z;
+        for (int s = 0; s < 2; ++s) {
+            for (int k = 0; k < 3; ++k) {
+                z.box[s][k] = kKeyLo; z.box[s][3 + k] = kKeyHi;
+                z.cen[s][k] = kKeyLo; z.cen[s][3 + k] = kKeyHi;
+            }
+            const uint32_t cb = s ? tk.begin + sp.nl : tk.begin, ce = s ? tk.end : tk.begin + sp.nl;
+            BNode n;
+            for (int k = 0; k < 3; ++k) { n.lo[k] = funkey(a.box[s][k]); n.hi[k] = funkey(a.box[s][3 + k]); }
+            n.left = n.right = kNone;
+            n.first = cb;
+            n.count = ce - cb;
+            n.parent = tk.node;
+            n.pad = 0;
+            nodes[id + s] = n;
+            if (n.count <= 1u) {
+                if (n.count == 1u) final_refs[cb] = refs[cb];
+                continue;
+            }
+            Task c;
+            c.node = id + s;
+            c.begin = cb;
+            c.end = ce;
+            c.aux = (uint32_t)(cur ^ 1);
+            for (int k = 0; k < 3; ++k) { c.clo[k] = funkey(a.cen[s][k]); c.chi[k] = funkey(a.cen[s][3 + k]); }
+            if (n.count <= kSmall) {
+                const uint32_t slot = atomicAdd(&cnt->small_tasks, 1u);
+                if (slot < small_cap) small[slot] = c; else atomicOr(&cnt->error, kErrNodes);
+            } else {
+                const uint32_t slot = atomicAdd(&cnt->tasks[cur ^ 1], 1u);
+                if (slot < next_cap) next[slot] = c; else atomicOr(&cnt->error, kErrNodes);
+            }
         }
+        acc[i] = z;   // for the next level's task
     }
 }
 
@@ -679,9 +765,10 @@ __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_
 // bins and three scans for two references as for a hundred, took 3.38 ms of the
 // 1.48 M-triangle terrain's build; 1.25 ms now.
 __global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __restrict__ small, uint32_t nsmall,
+                                                            const uint32_t* __restrict__ refs0,
+                                                            const uint32_t* __restrict__ refs1,
                                                             uint32_t* __restrict__ final_refs,
-                                                            const float4* __restrict__ tlo,
-                                                            const float4* __restrict__ thi, BNode* __restrict__ nodes,
+                                                            const float4* __restrict__ box, BNode* __restrict__ nodes,
                                                             Counters* cnt, int B, uint32_t max_leaf,
                                                             uint32_t max_nodes) {
     __shared__ SmallSet s_set[kSmallWarps];
@@ -698,8 +785,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __res
     SmallSet& T = s_work[warp].tmp;
     Bin* SB = s_work[warp].bins;
     for (uint32_t i = lane; i < n0; i += 32) {
-        const uint32_t r = final_refs[root.begin + i];
-        const float4 l = tlo[r], h = thi[r];
+        const uint32_t r = (root.aux ? refs1 : refs0)[root.begin + i];
+        const float4 l = box[2 * (size_t)r], h = box[2 * (size_t)r + 1];
         S.ref[i] = r;
         S.lo[0][i] = l.x; S.lo[1][i] = l.y; S.lo[2][i] = l.z;
         S.hi[0][i] = h.x; S.hi[1][i] = h.y; S.hi[2][i] = h.z;
@@ -1161,8 +1248,8 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Scratch layout for num_tris triangles (all offsets 256-byte aligned).
 struct Layout {
-    size_t tlo, thi, refs0, refs1, final_refs, bnodes, visits, cost, dec, isplit, tasks0, tasks1, small, bins,
-        splits, acc, chunks, chunk_left, queue0, queue1, rec, ni, nt, wnodes, counters, gkeys, sah, total;
+    size_t box, refs0, refs1, final_refs, bnodes, visits, cost, dec, isplit, tasks0, tasks1, small, bins,
+        splits, acc, chunk_task, chunk_bins, left_base, queue0, queue1, rec, ni, nt, wnodes, counters, gkeys, sah, total;
     uint32_t max_nodes, task_cap, small_cap, chunk_cap, wnode_cap;
 };
 
@@ -1175,8 +1262,7 @@ Layout make_layout(uint32_t T) {
     L.small_cap = T / 2 + 2;
     L.chunk_cap = T / kChunk + L.task_cap + 2;
     L.wnode_cap = T + 1;
-    L.tlo = take((size_t)T * 16);
-    L.thi = take((size_t)T * 16);
+    L.box = take((size_t)T * 32);
     L.refs0 = take((size_t)T * 4);
     L.refs1 = take((size_t)T * 4);
     L.final_refs = take((size_t)T * 4);
@@ -1191,8 +1277,9 @@ Layout make_layout(uint32_t T) {
     L.bins = take((size_t)L.task_cap * 3 * kBins * sizeof(Bin));
     L.splits = take((size_t)L.task_cap * sizeof(Split));
     L.acc = take((size_t)L.task_cap * sizeof(ChildAcc));
-    L.chunks = take((size_t)L.chunk_cap * sizeof(Chunk));
-    L.chunk_left = take((size_t)L.chunk_cap * 4);
+    L.chunk_task = take((size_t)L.chunk_cap * 4);
+    L.chunk_bins = take((size_t)L.chunk_cap * sizeof(ChunkBins));
+    L.left_base = take((size_t)L.chunk_cap * 4);
     L.queue0 = take((size_t)L.wnode_cap * 4);
     L.queue1 = take((size_t)L.wnode_cap * 4);
     L.rec = take((size_t)L.wnode_cap * sizeof(WideRec));
@@ -1218,6 +1305,7 @@ std::string error_text(uint32_t e) {
     if (e & kErrStack) m += " small-node stack overflow;";
     if (e & kErrClimb) m += " collapse climb did not end;";
     if (e & kErrWide) m += " wide-node capacity exceeded;";
+    if (e & kErrPartition) m += " partition count mismatch;";
     return m;
 }
 
@@ -1261,8 +1349,7 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         return false;
     }
     auto P = [&](size_t o) { return (void*)(base + o); };
-    float4* tlo = (float4*)P(L.tlo);
-    float4* thi = (float4*)P(L.thi);
+    float4* box = (float4*)P(L.box);
     uint32_t* refs[2] = {(uint32_t*)P(L.refs0), (uint32_t*)P(L.refs1)};
     uint32_t* final_refs = (uint32_t*)P(L.final_refs);
     BNode* bnodes = (BNode*)P(L.bnodes);
@@ -1271,8 +1358,9 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
     Bin* bins = (Bin*)P(L.bins);
     Split* splits = (Split*)P(L.splits);
     ChildAcc* acc = (ChildAcc*)P(L.acc);
-    Chunk* chunks = (Chunk*)P(L.chunks);
-    uint32_t* chunk_left = (uint32_t*)P(L.chunk_left);
+    uint32_t* chunk_task = (uint32_t*)P(L.chunk_task);
+    ChunkBins* chunk_bins = (ChunkBins*)P(L.chunk_bins);
+    uint32_t* left_base = (uint32_t*)P(L.left_base);
     Counters* cnt = (Counters*)P(L.counters);
     uint32_t* gkeys = (uint32_t*)P(L.gkeys);
     double* sah = (double*)P(L.sah);
@@ -1293,8 +1381,7 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         DB_CK(cudaMemcpyAsync(gkeys, keys0, sizeof(keys0), cudaMemcpyHostToDevice, st));
         DB_CK(cudaMemsetAsync(bnodes, 0xff, (size_t)L.max_nodes * sizeof(BNode), st));   // left = right = kNone
         DB_CK(cudaMemsetAsync(P(L.visits), 0, (size_t)L.max_nodes * 4, st));
-        k_tri_boxes<<<blocks_for(T, 256), 256, 0, st>>>(pos, nv, idx, T, tlo, thi, gkeys, cnt);
-        k_iota<<<blocks_for(T, 256), 256, 0, st>>>(refs[0], T);
+        k_tri_boxes<<<blocks_for(T, 256), 256, 0, st>>>(pos, nv, idx, T, box, refs[0], gkeys, cnt);
         DB_CK(cudaGetLastError());
         uint32_t keys[12];
         Counters hc;
@@ -1323,92 +1410,58 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         rt.node = 0;
         rt.begin = 0;
         rt.end = T;
-        rt.pad = 0;
+        rt.aux = 0;
         for (int k = 0; k < 3; ++k) { rt.clo[k] = unkey(keys[6 + k]); rt.chi[k] = unkey(keys[9 + k]); }
-        uint32_t nsmall = 0, ntasks = 0;
-        int cur = 0;   // refs[cur] holds the current level's references
+        uint32_t nsmall = 0;
         if (T == 1) {
             DB_CK(cudaMemcpyAsync(final_refs, refs[0], 4, cudaMemcpyDeviceToDevice, st));
         } else if (T <= kSmall) {
-            DB_CK(cudaMemcpyAsync(final_refs, refs[0], (size_t)T * 4, cudaMemcpyDeviceToDevice, st));
             DB_CK(cudaMemcpyAsync(small, &rt, sizeof(rt), cudaMemcpyHostToDevice, st));
             nsmall = 1;
-            DB_CK(cudaMemcpyAsync(&cnt->small_tasks, &nsmall, 4, cudaMemcpyHostToDevice, st));
         } else {
+            // ---- phase 2: levels of large nodes ----
+            // A level has at most 2^level tasks and T / 4096 chunks and one per task. The first batch of levels
+            // is as many as an even tree has plus four; after it the host looks whether tasks are left.
+            int dev = 0, sms = 0;
+            DB_CK(cudaGetDevice(&dev));
+            DB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             DB_CK(cudaMemcpyAsync(tasks[0], &rt, sizeof(rt), cudaMemcpyHostToDevice, st));
-            ntasks = 1;
-        }
-        // ---- phase 2: levels of large nodes ----
-        std::vector<Task> htasks;
-        std::vector<Chunk> hchunks;
-        std::vector<uint32_t> hleft;
-        std::vector<Split> hsplit;
-        int tq = 0;   // tasks[tq] holds the current level's tasks
-        for (uint32_t level = 0; ntasks > 0; ++level) {
-            if (level > T) { why = "device BVH build: levels do not end"; goto done; }
-            htasks.resize(ntasks);
-            DB_CK(cudaMemcpyAsync(htasks.data(), tasks[tq], ntasks * sizeof(Task), cudaMemcpyDeviceToHost, st));
-            DB_CK(cudaStreamSynchronize(st));
-            hchunks.clear();
-            for (uint32_t t = 0; t < ntasks; ++t)
-                for (uint32_t b = htasks[t].begin; b < htasks[t].end; b += kChunk) {
-                    Chunk c{};
-                    c.task = t;
-                    c.begin = b;
-                    c.end = std::min(htasks[t].end, b + kChunk);
-                    hchunks.push_back(c);
+            DB_CK(cudaMemcpyAsync(&cnt->tasks[0], &one, 4, cudaMemcpyHostToDevice, st));
+            k_bins_init<<<blocks_for((uint64_t)L.task_cap * 3 * kBins, 256), 256, 0, st>>>(bins, L.task_cap * 3 * kBins, acc,
+                                                                                          L.task_cap);
+            uint32_t batch = 4;
+            while ((uint64_t)kSmall << (batch - 4) < T) ++batch;
+            uint32_t ntasks = 1;
+            for (uint32_t level = 0; ntasks > 0;) {
+                if (level > T) { why = "device BVH build: levels do not end"; goto done; }
+                for (uint32_t k = 0; k < batch; ++k, ++level) {
+                    const int cur = (int)(level & 1u);   // tasks[cur] and refs[cur] are the level's
+                    const uint32_t max_tasks = level < 31u ? std::min(1u << level, L.task_cap) : L.task_cap;
+                    const uint32_t max_chunks = std::min(T / kChunk + max_tasks + 1u, L.chunk_cap);
+                    const uint32_t grid = std::min(max_chunks, (uint32_t)sms * 8u);
+                    k_level_chunks<<<1, 1024, 0, st>>>(tasks[cur], chunk_task, L.chunk_cap, cnt, cur);
+                    k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, B);
+                    k_split<<<std::min(blocks_for((uint64_t)max_tasks * 32, 128), (uint32_t)sms * 8u), 128, 0, st>>>(
+                        tasks[cur], bins, chunk_bins, bnodes, splits, left_base, cnt, cur, B, bin_leaf);
+                    k_partition<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], splits, left_base, refs[cur],
+                                                                refs[cur ^ 1], box, acc, cnt, B);
+                    k_make_children<<<std::min(blocks_for(max_tasks, 64), (uint32_t)sms * 4u), 64, 0, st>>>(
+                        tasks[cur], splits, acc, refs[cur ^ 1], bnodes, final_refs, tasks[cur ^ 1], L.task_cap, small,
+                        L.small_cap, cnt, cur, L.max_nodes);
                 }
-            const uint32_t nch = (uint32_t)hchunks.size();
-            if (nch > L.chunk_cap) { why = "device BVH build: chunk capacity exceeded"; goto done; }
-            DB_CK(cudaMemcpyAsync(chunks, hchunks.data(), nch * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-            k_bins_init<<<blocks_for((uint64_t)ntasks * 3 * kBins, 256), 256, 0, st>>>(bins, ntasks * 3 * kBins);
-            k_bin<<<nch, kLevelThreads, 0, st>>>(chunks, tasks[tq], refs[cur], tlo, thi, bins, B);
-            k_split<<<blocks_for((uint64_t)ntasks * 32, 256), 256, 0, st>>>(tasks[tq], ntasks, bins, bnodes, splits, B,
-                                                                          bin_leaf);
-            k_count_left<<<nch, kLevelThreads, 0, st>>>(chunks, tasks[tq], splits, refs[cur], tlo, thi, chunk_left, B);
-            DB_CK(cudaGetLastError());
-            hleft.resize(nch);
-            hsplit.resize(ntasks);
-            DB_CK(cudaMemcpyAsync(hleft.data(), chunk_left, nch * 4, cudaMemcpyDeviceToHost, st));
-            DB_CK(cudaMemcpyAsync(hsplit.data(), splits, ntasks * sizeof(Split), cudaMemcpyDeviceToHost, st));
-            DB_CK(cudaStreamSynchronize(st));
-            {
-                uint32_t prev_task = kNone, lsum = 0, rsum = 0;
-                for (uint32_t c = 0; c < nch; ++c) {
-                    Chunk& ck = hchunks[c];
-                    const Task& tk = htasks[ck.task];
-                    if (ck.task != prev_task) { prev_task = ck.task; lsum = 0; rsum = 0; }
-                    const uint32_t nl = hsplit[ck.task].nl;
-                    ck.left_base = tk.begin + lsum;
-                    ck.right_base = tk.begin + nl + rsum;
-                    lsum += hleft[c];
-                    rsum += (ck.end - ck.begin) - hleft[c];
-                    if (c + 1 == nch || hchunks[c + 1].task != ck.task) {
-                        if (lsum != nl) { why = "device BVH build: partition count mismatch"; goto done; }
-                    }
-                }
+                DB_CK(cudaGetLastError());
+                DB_CK(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
+                DB_CK(cudaStreamSynchronize(st));
+                if (hc.error) { why = "device BVH build:" + error_text(hc.error); goto done; }
+                ntasks = hc.tasks[level & 1u];
+                nsmall = hc.small_tasks;
+                batch = 4;
             }
-            DB_CK(cudaMemcpyAsync(chunks, hchunks.data(), nch * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-            k_acc_init<<<blocks_for(ntasks, 256), 256, 0, st>>>(acc, ntasks);
-            k_partition<<<nch, kLevelThreads, 0, st>>>(chunks, tasks[tq], splits, refs[cur], refs[cur ^ 1], tlo, thi,
-                                                       acc, B);
-            DB_CK(cudaMemsetAsync(&cnt->next_tasks, 0, 4, st));
-            k_make_children<<<blocks_for(ntasks, 128), 128, 0, st>>>(tasks[tq], ntasks, splits, acc, refs[cur ^ 1],
-                                                                      bnodes, final_refs, tasks[tq ^ 1], L.task_cap,
-                                                                      small, L.small_cap, cnt, L.max_nodes);
-            DB_CK(cudaGetLastError());
-            DB_CK(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
-            DB_CK(cudaStreamSynchronize(st));
-            if (hc.error) { why = "device BVH build:" + error_text(hc.error); goto done; }
-            ntasks = hc.next_tasks;
-            nsmall = hc.small_tasks;
-            tq ^= 1;
-            cur ^= 1;
         }
         if (nsmall > 0)
-            k_small<<<blocks_for(nsmall, kSmallWarps), kSmallWarps * 32, 0, st>>>(small, nsmall, final_refs, tlo, thi,
-                                                                                 bnodes, cnt, B, bin_leaf,
-                                                                                 L.max_nodes);
+            k_small<<<blocks_for(nsmall, kSmallWarps), kSmallWarps * 32, 0, st>>>(small, nsmall, refs[0], refs[1],
+                                                                                 final_refs, box, bnodes, cnt, B,
+                                                                                 bin_leaf, L.max_nodes);
         DB_CK(cudaGetLastError());
         DB_CK(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
         DB_CK(cudaStreamSynchronize(st));
