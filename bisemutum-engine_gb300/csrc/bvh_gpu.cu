@@ -927,72 +927,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __res
 }
 
 // ------------------------------------------------------------ phase 3 ----
-// cost(n, i) for i = 1..8 and the decisions, as the host's Collapse::run.
-__global__ void k_collapse(const BNode* __restrict__ nodes, uint32_t n, uint32_t* __restrict__ visits,
-                           float* __restrict__ cost, uint8_t* __restrict__ dec, uint8_t* __restrict__ isplit,
-                           uint32_t max_leaf, float tri_cost, Counters* cnt) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const BNode L = nodes[i];
-    if (L.left != kNone) return;   // climbs start at leaves
-    {
-        const float a = area6(L.lo, L.hi);
-        const float leaf = L.count <= max_leaf ? a * (float)L.count * tri_cost : INFINITY;
-        for (int k = 0; k < 8; ++k) {
-            cost[8 * (size_t)i + k] = leaf;
-            dec[8 * (size_t)i + k] = k == 0 ? kDecLeaf : kDecSame;
-        }
-    }
-    __threadfence();
-    uint32_t x = L.parent;
-    for (uint32_t guard = 0; x != kNone; ++guard) {
-        if (guard > n) { atomicOr(&cnt->error, kErrClimb); return; }
-        if (atomicAdd(&visits[x], 1u) == 0u) return;   // the other child is not done yet
-        __threadfence();
-        const BNode X = nodes[x];
-        float cl[8], cr[8];
-        for (int k = 0; k < 8; ++k) {
-            cl[k] = __ldcg(&cost[8 * (size_t)X.left + k]);
-            cr[k] = __ldcg(&cost[8 * (size_t)X.right + k]);
-        }
-        float dist[9];
-        uint8_t arg[9];
-        for (int j = 2; j <= 8; ++j) {
-            dist[j] = INFINITY;
-            arg[j] = 1;
-            for (int k = 1; k < j; ++k) {
-                float v = cl[k - 1] + cr[j - k - 1];
-                if (v < dist[j]) { dist[j] = v; arg[j] = (uint8_t)k; }
-            }
-        }
-        const float a = area6(X.lo, X.hi);
-        const float leaf = X.count <= max_leaf ? a * (float)X.count * tri_cost : INFINITY;
-        const float inner = a + dist[8];   // node cost 1
-        float c[8];
-        uint8_t d[8];
-        if (leaf <= inner) { c[0] = leaf; d[0] = kDecLeaf; } else { c[0] = inner; d[0] = kDecInner; }
-        for (int k = 2; k <= 8; ++k) {
-            if (c[k - 2] <= dist[k]) { c[k - 1] = c[k - 2]; d[k - 1] = kDecSame; }
-            else { c[k - 1] = dist[k]; d[k - 1] = arg[k]; }
-        }
-        for (int k = 0; k < 8; ++k) {
-            cost[8 * (size_t)x + k] = c[k];
-            dec[8 * (size_t)x + k] = d[k];
-        }
-        isplit[x] = arg[8];
-        __threadfence();
-        x = X.parent;
-    }
-}
-
-__global__ void k_sah_cost(const BNode* __restrict__ nodes, uint32_t n, double* out) {
+__device__ __forceinline__ void block_add(double v, double* out) {   // blocks of 256 threads
     __shared__ double s[8];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 0.0;
-    if (i < n) {
-        const BNode b = nodes[i];
-        v = (double)area6(b.lo, b.hi) * (b.left == kNone ? (double)b.count : 1.0);
-    }
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
     __syncthreads();
@@ -1001,6 +937,93 @@ __global__ void k_sah_cost(const BNode* __restrict__ nodes, uint32_t n, double* 
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
         atomicAdd(out, t);
     }
+}
+
+// cost(n, i) for i = 1..8 and the decisions, as the host's Collapse::run; the
+// nodes' areas and leaf counts go to the tree's SAH cost on the way.
+__device__ __forceinline__ double climb(const BNode* __restrict__ nodes, uint32_t n, uint32_t i,
+                                        uint32_t* __restrict__ visits, float4* __restrict__ cost,
+                                        uint2* __restrict__ dec, uint8_t* __restrict__ isplit, uint32_t max_leaf,
+                                        float tri_cost, Counters* cnt) {
+    if (i >= n) return 0.0;
+    const BNode L = nodes[i];
+    if (L.left != kNone) return 0.0;   // climbs start at leaves
+    double sah;
+    {
+        const float a = area6(L.lo, L.hi);
+        sah = (double)a * (double)L.count;
+        const float leaf = L.count <= max_leaf ? a * (float)L.count * tri_cost : INFINITY;
+        cost[2 * (size_t)i] = make_float4(leaf, leaf, leaf, leaf);
+        cost[2 * (size_t)i + 1] = make_float4(leaf, leaf, leaf, leaf);
+        constexpr uint32_t same = kDecSame * 0x01010101u;
+        dec[i] = make_uint2((same & 0xffffff00u) | kDecLeaf, same);
+    }
+    __threadfence();
+    uint32_t x = L.parent;
+    for (uint32_t guard = 0; x != kNone; ++guard) {
+        if (guard > n) { atomicOr(&cnt->error, kErrClimb); return sah; }
+        if (atomicAdd(&visits[x], 1u) == 0u) return sah;   // the other child is not done yet
+        __threadfence();
+        const BNode X = nodes[x];
+        float cl[8], cr[8];
+        {
+            const float4 a = __ldcg(&cost[2 * (size_t)X.left]), b = __ldcg(&cost[2 * (size_t)X.left + 1]);
+            const float4 c = __ldcg(&cost[2 * (size_t)X.right]), d = __ldcg(&cost[2 * (size_t)X.right + 1]);
+            cl[0] = a.x; cl[1] = a.y; cl[2] = a.z; cl[3] = a.w; cl[4] = b.x; cl[5] = b.y; cl[6] = b.z; cl[7] = b.w;
+            cr[0] = c.x; cr[1] = c.y; cr[2] = c.z; cr[3] = c.w; cr[4] = d.x; cr[5] = d.y; cr[6] = d.z; cr[7] = d.w;
+        }
+        float dist[9];
+        uint32_t arg[9];
+#pragma unroll
+        for (int j = 2; j <= 8; ++j) {
+            dist[j] = INFINITY;
+            arg[j] = 1;
+#pragma unroll
+            for (int k = 1; k < j; ++k) {
+                float v = cl[k - 1] + cr[j - k - 1];
+                if (v < dist[j]) { dist[j] = v; arg[j] = (uint32_t)k; }
+            }
+        }
+        const float a = area6(X.lo, X.hi);
+        sah += (double)a;
+        const float leaf = X.count <= max_leaf ? a * (float)X.count * tri_cost : INFINITY;
+        const float inner = a + dist[8];   // node cost 1
+        float c[8];
+        uint32_t d[2] = {0u, 0u};
+        if (leaf <= inner) { c[0] = leaf; d[0] = kDecLeaf; } else { c[0] = inner; d[0] = kDecInner; }
+#pragma unroll
+        for (int k = 2; k <= 8; ++k) {
+            uint32_t e;
+            if (c[k - 2] <= dist[k]) { c[k - 1] = c[k - 2]; e = kDecSame; }
+            else { c[k - 1] = dist[k]; e = arg[k]; }
+            d[(k - 1) >> 2] |= e << (8 * ((k - 1) & 3));
+        }
+        cost[2 * (size_t)x] = make_float4(c[0], c[1], c[2], c[3]);
+        cost[2 * (size_t)x + 1] = make_float4(c[4], c[5], c[6], c[7]);
+        dec[x] = make_uint2(d[0], d[1]);
+        isplit[x] = (uint8_t)arg[8];
+        __threadfence();
+        x = X.parent;
+    }
+    return sah;
+}
+
+__global__ void __launch_bounds__(256) k_collapse(const BNode* __restrict__ nodes, uint32_t n,
+                                                  uint32_t* __restrict__ visits, float4* __restrict__ cost,
+                                                  uint2* __restrict__ dec, uint8_t* __restrict__ isplit,
+                                                  uint32_t max_leaf, float tri_cost, double* sah, Counters* cnt) {
+    block_add(climb(nodes, n, blockIdx.x * blockDim.x + threadIdx.x, visits, cost, dec, isplit, max_leaf, tri_cost, cnt),
+              sah);
+}
+
+__global__ void __launch_bounds__(256) k_sah_cost(const BNode* __restrict__ nodes, uint32_t n, double* out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v = 0.0;
+    if (i < n) {
+        const BNode b = nodes[i];
+        v = (double)area6(b.lo, b.hi) * (b.left == kNone ? (double)b.count : 1.0);
+    }
+    block_add(v, out);
 }
 
 // ------------------------------------------------------------ phase 4 ----
@@ -1498,7 +1521,6 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         DB_CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), st));
         DB_CK(cudaMemsetAsync(sah, 0, 8, st));
         DB_CK(cudaMemcpyAsync(gkeys, keys0, sizeof(keys0), cudaMemcpyHostToDevice, st));
-        DB_CK(cudaMemsetAsync(bnodes, 0xff, (size_t)L.max_nodes * sizeof(BNode), st));   // left = right = kNone
         DB_CK(cudaMemsetAsync(P(L.visits), 0, (size_t)L.max_nodes * 4, st));
         k_tri_boxes<<<blocks_for(T, 256), 256, 0, st>>>(pos, nv, idx, T, box, refs[0], gkeys, cnt);
         DB_CK(cudaGetLastError());
@@ -1585,10 +1607,11 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         const uint32_t nb = hc.nodes;
         // ---- phase 3 ----
         if (optimal)
-            k_collapse<<<blocks_for(nb, 256), 256, 0, st>>>(bnodes, nb, (uint32_t*)P(L.visits), (float*)P(L.cost),
-                                                            (uint8_t*)P(L.dec), (uint8_t*)P(L.isplit), max_leaf,
-                                                            tri_cost, cnt);
-        k_sah_cost<<<blocks_for(nb, 256), 256, 0, st>>>(bnodes, nb, sah);
+            k_collapse<<<blocks_for(nb, 256), 256, 0, st>>>(bnodes, nb, (uint32_t*)P(L.visits), (float4*)P(L.cost),
+                                                            (uint2*)P(L.dec), (uint8_t*)P(L.isplit), max_leaf,
+                                                            tri_cost, sah, cnt);
+        else
+            k_sah_cost<<<blocks_for(nb, 256), 256, 0, st>>>(bnodes, nb, sah);
         DB_CK(cudaGetLastError());
         // ---- phase 4 ----
         WideCfg wc;
