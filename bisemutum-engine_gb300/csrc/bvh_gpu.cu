@@ -11,22 +11,24 @@
 //   1. triangle boxes and the scene's box and centroid bounds, one thread per
 //      triangle;
 //   2. the binary BVH top-down, one breadth-first level per round while a node
-//      holds more than kSmall triangles.  Per level every CTA bins one chunk of
-//      one node's triangle references into 3 x 32 centroid bins in shared
-//      memory and merges them into the node's bins with one atomic per bin
-//      value; one warp per node picks the split of least SAH cost; a stable
-//      partition writes the children's references (warp ballots, one CTA per
-//      chunk); the children become leaves, small nodes or next-level nodes.
-//      Nodes of at most kSmall triangles are then finished by one warp each,
-//      with their references in shared memory;
+//      holds more than kSmall triangles. Per level every CTA bins chunks of a
+//      node's triangle references into 3 x 32 centroid bins in shared memory and
+//      merges them into the node's bins with one atomic per bin value; one warp
+//      per node picks the split of least SAH cost; a stable partition writes the
+//      children's references (warp ballots, chunk offsets from the chunks' own
+//      bin counts); the children become leaves, small nodes or next-level nodes.
+//      The host queues the levels in batches and looks only then. Nodes of at
+//      most kSmall triangles are finished by one warp each in shared memory, from
+//      32 triangles on with a triangle per lane;
 //   3. the collapse's dynamic programme bottom-up: a thread per binary leaf
 //      climbs towards the root and stops at every node whose other child is not
 //      done yet (the second thread to arrive computes the node; Karras 2012);
-//   4. the 8-wide nodes top-down, one level per round: each node gathers its up
-//      to eight children and assigns octant slots, a scan over the level gives
-//      each node its first child and first triangle, and a second pass writes
-//      the quantised node, its leaf triangles and the next level's queue, so
-//      nodes and triangles come out in breadth-first order as on the host.
+//   4. the 8-wide nodes top-down, one level per round, eight lanes per node: each
+//      node gathers its up to eight children, assigns octant slots and quantises
+//      their boxes; a scan over the level gives each node its first child and
+//      first triangle, and a second pass writes the leaf triangles and the next
+//      level's queue, so nodes and triangles come out in breadth-first order as
+//      on the host.
 // Split decisions use exact bin counts and boxes (order-independent atomics on
 // ordered float keys), and every partition is stable, so the tree does not
 // depend on the order in which CTAs run.
@@ -45,7 +47,11 @@ namespace {
 
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr int kBins = 32;                  // lanes of a warp: one bin per lane
-constexpr uint32_t kChunk = 4096;          // references per CTA in a level pass
+constexpr uint32_t kChunk = 4096;          // references per CTA in a level pass, at most
+// Chunks of a build of T triangles: large ones cost fewer merges, small ones fill the GPU in the top levels, where a
+// level has few nodes (builds of 20,504 / 250,050 / 1,482,242 / 4,973,058 triangles take 1.23 / 2.24 / 4.95 / 14.1 ms
+// with 4,096 per chunk, 1.14 / 2.10 / 4.90 / 14.3 with 2,048 and 1.10 / 1.97 / 4.98 / 14.7 with 1,024).
+uint32_t chunk_size(uint32_t T) { return T < 600000u ? 1024u : T < 3000000u ? 2048u : kChunk; }
 constexpr uint32_t kSmall = 128;           // nodes of at most this many triangles are finished by one warp
 constexpr int kSmallWarps = 4;             // warps per CTA of the small-node kernel
 constexpr uint32_t kLevelThreads = 256;
@@ -190,14 +196,14 @@ __global__ void k_bins_init(Bin* bins, uint32_t n, ChildAcc* acc, uint32_t nacc)
 
 // First chunk of every task (one block: a scan over the tasks) and the task of every chunk.
 __global__ void __launch_bounds__(1024) k_level_chunks(Task* __restrict__ tasks, uint32_t* __restrict__ chunk_task,
-                                                       uint32_t chunk_cap, Counters* cnt, int cur) {
+                                                       uint32_t chunk_cap, uint32_t chunk, Counters* cnt, int cur) {
     __shared__ uint32_t s_w[32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nt = cnt->error ? 0u : cnt->tasks[cur];
     uint32_t carry = 0;
     __syncthreads();   // every thread has read the counters that thread 0 writes below
     for (uint32_t base = 0; base < nt; base += blockDim.x) {
         const uint32_t i = base + threadIdx.x;
-        const uint32_t n = i < nt ? (tasks[i].end - tasks[i].begin + kChunk - 1u) / kChunk : 0u;
+        const uint32_t n = i < nt ? (tasks[i].end - tasks[i].begin + chunk - 1u) / chunk : 0u;
         uint32_t x = n;
         for (uint32_t o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -256,7 +262,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_bin(const uint32_t* __restric
                                                        const Task* __restrict__ tasks,
                                                        const uint32_t* __restrict__ refs,
                                                        const float4* __restrict__ box, Bin* __restrict__ gbins,
-                                                       ChunkBins* __restrict__ cbins, const Counters* cnt, int B) {
+                                                       ChunkBins* __restrict__ cbins, const Counters* cnt, uint32_t chunk, int B) {
     __shared__ Bin sb[3 * kBins];
     const uint32_t nch = cnt->error ? 0u : cnt->chunks;
     for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
@@ -267,7 +273,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_bin(const uint32_t* __restric
         __syncthreads();
         const uint32_t ti = chunk_task[c];
         const Task tk = tasks[ti];
-        const uint32_t begin = tk.begin + (c - tk.aux) * kChunk, end = min(tk.end, begin + kChunk);
+        const uint32_t begin = tk.begin + (c - tk.aux) * chunk, end = min(tk.end, begin + chunk);
         float sc[3];
         for (int a = 0; a < 3; ++a) sc[a] = axis_scale(tk, a, B);
         for (uint32_t base = begin; base < end; base += blockDim.x) {
@@ -393,7 +399,7 @@ __device__ __forceinline__ Split decide(int bax, int bbin, uint32_t bnl, float b
 // where its chunks' left references go.
 __global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins, const ChunkBins* __restrict__ cbins,
                         const BNode* __restrict__ nodes, Split* __restrict__ splits, uint32_t* __restrict__ left_base,
-                        Counters* cnt, int cur, int B, uint32_t max_leaf) {
+                        Counters* cnt, int cur, uint32_t chunk, int B, uint32_t max_leaf) {
     const int lane = threadIdx.x & 31;
     const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur], warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nt; w += warps) {
@@ -413,15 +419,15 @@ __global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins,
         const BNode nd = nodes[tk.node];
         const Split s = decide(bax, bbin, bnl, best, tk.end - tk.begin, area6(nd.lo, nd.hi), max_leaf);
         if (lane == 0) splits[w] = s;
-        const uint32_t n = (tk.end - tk.begin + kChunk - 1u) / kChunk;
+        const uint32_t n = (tk.end - tk.begin + chunk - 1u) / chunk;
         uint32_t carry = 0;
         for (uint32_t base = 0; base < n; base += 32) {
             const uint32_t c = base + lane;
             uint32_t left = 0;
             if (c < n) {
-                const uint32_t size = min(kChunk, tk.end - tk.begin - c * kChunk);
+                const uint32_t size = min(chunk, tk.end - tk.begin - c * chunk);
                 if (s.leaf) left = size;
-                else if (s.axis < 0) left = s.nl > c * kChunk ? min(size, s.nl - c * kChunk) : 0u;
+                else if (s.axis < 0) left = s.nl > c * chunk ? min(size, s.nl - c * chunk) : 0u;
                 else left = cbins[tk.aux + c].below[s.axis][s.bin];
             }
             uint32_t x = left;
@@ -454,7 +460,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __r
                                                              const uint32_t* __restrict__ in,
                                                              uint32_t* __restrict__ out,
                                                              const float4* __restrict__ box,
-                                                             ChildAcc* __restrict__ acc, const Counters* cnt, int B) {
+                                                             ChildAcc* __restrict__ acc, const Counters* cnt, uint32_t chunk, int B) {
     __shared__ uint32_t s_wl[kLevelThreads / 32], s_wr[kLevelThreads / 32];
     __shared__ float s_red[kLevelThreads / 32][24];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -464,7 +470,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __r
         const uint32_t ti = chunk_task[c];
         const Task tk = tasks[ti];
         const Split sp = splits[ti];
-        const uint32_t begin = tk.begin + (c - tk.aux) * kChunk, end = min(tk.end, begin + kChunk);
+        const uint32_t begin = tk.begin + (c - tk.aux) * chunk, end = min(tk.end, begin + chunk);
         float v[24];   // side s: box lo(3) hi(3), centroid lo(3) hi(3) at 12 s
         for (int s = 0; s < 2; ++s)
             for (int k = 0; k < 3; ++k) {
@@ -764,8 +770,8 @@ __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_
 // stack (every entry holds two or more references of a disjoint range, so at
 // most kSmall / 2 entries are live).  Splitting every node on its own, with
 // bins and three scans for two references as for a hundred, took 3.38 ms of the
-// 1.48 M-triangle terrain's build; 1.25 ms now.
-__global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __restrict__ small, uint32_t nsmall,
+// 1.48 M-triangle terrain's build; 1.18 ms now (predicated instead of branching sums: 1.39).
+__global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __restrict__ small, uint32_t nsmall,
                                                             const uint32_t* __restrict__ refs0,
                                                             const uint32_t* __restrict__ refs1,
                                                             uint32_t* __restrict__ final_refs,
@@ -927,16 +933,12 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 4) k_small(const Task* __res
 }
 
 // ------------------------------------------------------------ phase 3 ----
-__device__ __forceinline__ void block_add(double v, double* out) {   // blocks of 256 threads
-    __shared__ double s[8];
+// Adds to one of kSahSums partial sums, a warp at a time: no barrier, since a block's last climbers are far behind
+// its first, and no address that every warp adds to.
+constexpr uint32_t kSahSums = 256;
+__device__ __forceinline__ void add_sah(double v, double* sums) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
-        atomicAdd(out, t);
-    }
+    if ((threadIdx.x & 31u) == 0u) atomicAdd(sums + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kSahSums, v);
 }
 
 // cost(n, i) for i = 1..8 and the decisions, as the host's Collapse::run; the
@@ -1012,8 +1014,7 @@ __global__ void __launch_bounds__(256) k_collapse(const BNode* __restrict__ node
                                                   uint32_t* __restrict__ visits, float4* __restrict__ cost,
                                                   uint2* __restrict__ dec, uint8_t* __restrict__ isplit,
                                                   uint32_t max_leaf, float tri_cost, double* sah, Counters* cnt) {
-    block_add(climb(nodes, n, blockIdx.x * blockDim.x + threadIdx.x, visits, cost, dec, isplit, max_leaf, tri_cost, cnt),
-              sah);
+    add_sah(climb(nodes, n, blockIdx.x * blockDim.x + threadIdx.x, visits, cost, dec, isplit, max_leaf, tri_cost, cnt), sah);
 }
 
 __global__ void __launch_bounds__(256) k_sah_cost(const BNode* __restrict__ nodes, uint32_t n, double* out) {
@@ -1023,7 +1024,7 @@ __global__ void __launch_bounds__(256) k_sah_cost(const BNode* __restrict__ node
         const BNode b = nodes[i];
         v = (double)area6(b.lo, b.hi) * (b.left == kNone ? (double)b.count : 1.0);
     }
-    block_add(v, out);
+    add_sah(v, out);
 }
 
 // ------------------------------------------------------------ phase 4 ----
@@ -1400,7 +1401,7 @@ Layout make_layout(uint32_t T) {
     L.max_nodes = 2 * T;
     L.task_cap = T / kSmall + 2;
     L.small_cap = T / 2 + 2;
-    L.chunk_cap = T / kChunk + L.task_cap + 2;
+    L.chunk_cap = T / chunk_size(T) + L.task_cap + 2;
     L.wnode_cap = T + 1;
     L.box = take((size_t)T * 32);
     L.refs0 = take((size_t)T * 4);
@@ -1427,7 +1428,7 @@ Layout make_layout(uint32_t T) {
     L.wnodes = take((size_t)L.wnode_cap * sizeof(CwNode));
     L.counters = take(sizeof(Counters));
     L.gkeys = take(12 * 4);
-    L.sah = take(8);
+    L.sah = take(kSahSums * 8);
     L.total = off;
     return L;
 }
@@ -1519,7 +1520,7 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         uint32_t keys0[12];
         for (int k = 0; k < 12; ++k) keys0[k] = (k % 6) >= 3 ? kKeyHi : kKeyLo;
         DB_CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), st));
-        DB_CK(cudaMemsetAsync(sah, 0, 8, st));
+        DB_CK(cudaMemsetAsync(sah, 0, kSahSums * 8, st));
         DB_CK(cudaMemcpyAsync(gkeys, keys0, sizeof(keys0), cudaMemcpyHostToDevice, st));
         DB_CK(cudaMemsetAsync(P(L.visits), 0, (size_t)L.max_nodes * 4, st));
         k_tri_boxes<<<blocks_for(T, 256), 256, 0, st>>>(pos, nv, idx, T, box, refs[0], gkeys, cnt);
@@ -1561,12 +1562,13 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
             nsmall = 1;
         } else {
             // ---- phase 2: levels of large nodes ----
-            // A level has at most 2^level tasks and T / 4096 chunks and one per task. The first batch of levels
+            // A level has at most 2^level tasks and T / chunk chunks and one per task. The first batch of levels
             // is as many as an even tree has plus four; after it the host looks whether tasks are left.
             DB_CK(cudaMemcpyAsync(tasks[0], &rt, sizeof(rt), cudaMemcpyHostToDevice, st));
             DB_CK(cudaMemcpyAsync(&cnt->tasks[0], &one, 4, cudaMemcpyHostToDevice, st));
             k_bins_init<<<blocks_for((uint64_t)L.task_cap * 3 * kBins, 256), 256, 0, st>>>(bins, L.task_cap * 3 * kBins, acc,
                                                                                           L.task_cap);
+            const uint32_t chunk = chunk_size(T);
             uint32_t batch = 4;
             while ((uint64_t)kSmall << (batch - 4) < T) ++batch;
             uint32_t ntasks = 1;
@@ -1575,14 +1577,15 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
                 for (uint32_t k = 0; k < batch; ++k, ++level) {
                     const int cur = (int)(level & 1u);   // tasks[cur] and refs[cur] are the level's
                     const uint32_t max_tasks = level < 31u ? std::min(1u << level, L.task_cap) : L.task_cap;
-                    const uint32_t max_chunks = std::min(T / kChunk + max_tasks + 1u, L.chunk_cap);
+                    const uint32_t max_chunks = std::min(T / chunk + max_tasks + 1u, L.chunk_cap);
                     const uint32_t grid = std::min(max_chunks, (uint32_t)sms * 8u);
-                    k_level_chunks<<<1, 1024, 0, st>>>(tasks[cur], chunk_task, L.chunk_cap, cnt, cur);
-                    k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, B);
+                    k_level_chunks<<<1, 1024, 0, st>>>(tasks[cur], chunk_task, L.chunk_cap, chunk, cnt, cur);
+                    k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, chunk,
+                                                          B);
                     k_split<<<std::min(blocks_for((uint64_t)max_tasks * 32, 128), (uint32_t)sms * 8u), 128, 0, st>>>(
-                        tasks[cur], bins, chunk_bins, bnodes, splits, left_base, cnt, cur, B, bin_leaf);
+                        tasks[cur], bins, chunk_bins, bnodes, splits, left_base, cnt, cur, chunk, B, bin_leaf);
                     k_partition<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], splits, left_base, refs[cur],
-                                                                refs[cur ^ 1], box, acc, cnt, B);
+                                                                refs[cur ^ 1], box, acc, cnt, chunk, B);
                     k_make_children<<<std::min(blocks_for(max_tasks, 64), (uint32_t)sms * 4u), 64, 0, st>>>(
                         tasks[cur], splits, acc, refs[cur ^ 1], bnodes, final_refs, tasks[cur ^ 1], L.task_cap, small,
                         L.small_cap, cnt, cur, L.max_nodes);
@@ -1654,9 +1657,10 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
         }
         const uint32_t level_base = hc.wide[wide_level & 1u].node_base, tri_cursor = hc.wide[wide_level & 1u].tri_base,
                        depth = hc.depth;
-        double hsah = 0.0;
-        DB_CK(cudaMemcpyAsync(&hsah, sah, 8, cudaMemcpyDeviceToHost, st));
+        double hsah = 0.0, part[kSahSums];
+        DB_CK(cudaMemcpyAsync(part, sah, sizeof(part), cudaMemcpyDeviceToHost, st));
         DB_CK(cudaStreamSynchronize(st));
+        for (double v : part) hsah += v;
         if (tri_cursor != T) { why = "device BVH build: triangle count mismatch"; goto done; }
         CwNode* nodes_out = nullptr;
         DB_CK(cudaMalloc(&nodes_out, (size_t)level_base * sizeof(CwNode)));
