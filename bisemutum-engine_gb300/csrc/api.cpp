@@ -1298,10 +1298,8 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
     CK(cudaMemcpyAsync(sc->insts.ptr, sc->inst_host.data(), sc->inst_host.size() * sizeof(InstDev),
                        cudaMemcpyHostToDevice, WS(ctx)));
     CK(cudaMemcpyAsync(sc->inst_box.ptr, boxes.data(), boxes.size() * 4, cudaMemcpyHostToDevice, WS(ctx)));
-    // refit bottom-up: one launch per breadth-first level, deepest first
-    for (size_t lv = sc->level_begin.size() - 1; lv-- > 0;)
-        launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, (const float*)sc->inst_box.ptr,
-                          sc->level_begin[lv], sc->level_begin[lv + 1]);
+    launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, (const float*)sc->inst_box.ptr,
+                      sc->level_begin.data(), (uint32_t)sc->level_begin.size() - 1u);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(WS(ctx)));
     return BSM_OK;

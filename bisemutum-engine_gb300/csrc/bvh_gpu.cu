@@ -40,7 +40,7 @@
 #include <cstring>
 #include <vector>
 
-#include "bvh_quant.h"
+#include "bvh_quant_lanes.cuh"
 
 namespace bsm {
 namespace {
@@ -1043,35 +1043,9 @@ __device__ __forceinline__ bool wide_leaf(const WideCfg& w, uint32_t x) {
 }
 
 // ---- 8 lanes per 8-wide node ----
-constexpr uint32_t kWideLanes = 8;
 constexpr uint32_t kWideThreads = 256;
 constexpr uint32_t kWideTile = kWideThreads / kWideLanes;   // nodes per block and round
 static_assert(kWideTile == 32, "one warp scans a tile's nodes");
-
-__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-
-// quant_exponent_hd: the smallest e with 253 * 2^e >= extent, biased and clamped.
-__device__ __forceinline__ int quant_exponent_dev(float extent) {
-    const double ext = (double)extent > 1e-30 ? (double)extent : 1e-30;
-    int e = ((__double2hiint(ext) >> 20) & 0x7ff) - 1023 - 7;
-    while (253.0 * pow2d(e - 1) >= ext) --e;
-    while (253.0 * pow2d(e) < ext) ++e;
-    const int biased = e + 127;
-    return biased < 1 ? 1 : (biased > 254 ? 254 : biased);
-}
-
-__device__ __forceinline__ float wide_min(float x) {
-    for (int o = 1; o < (int)kWideLanes; o <<= 1) x = fminf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-__device__ __forceinline__ float wide_max(float x) {
-    for (int o = 1; o < (int)kWideLanes; o <<= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
-}
-__device__ __forceinline__ uint32_t wide_or(uint32_t x) {
-    for (int o = 1; o < (int)kWideLanes; o <<= 1) x |= __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-}
 
 // The nodes of a level: each gathers its up to eight children, assigns octant
 // slots and quantises their boxes, a child per lane, with its first child and
@@ -1211,38 +1185,8 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_nodes(const uint32_t* __r
         }
         const uint32_t imask = wide_or(valid && !leaf && count != 0u ? 1u << slot : 0u);
         const uint32_t tmask = wide_or(leaf ? ((1u << count) - 1u) << (2u * slot) : 0u);
-        // the frame (tlas_quantise), an axis per lane, then this lane's child
-        int e = 0;
-        float org = 0.0f;
-        if (sub < 3u) {
-            const float l = sub == 0 ? nlo[0] : sub == 1 ? nlo[1] : nlo[2], h = sub == 0 ? nhi[0] : sub == 1 ? nhi[1] : nhi[2];
-            if (nc != 0u) {
-                e = quant_exponent_dev(h - l);
-                const double at = (double)l - pow2d(e - 127);
-                org = (float)at;
-                while ((double)org > at) org = nextafterf(org, -INFINITY);
-            }
-        }
         uint8_t* image = reinterpret_cast<uint8_t*>(s_image[g]);
-        for (int k = 0; k < 3; ++k) {
-            const int ek = __shfl_sync(kFull, e, (int)shift + k);
-            const float ok = __shfl_sync(kFull, org, (int)shift + k);
-            if (valid) {
-                const double sc = pow2d(ek - 127), inv = pow2d(127 - ek), o = (double)ok;
-                double l = floor(((double)lo[k] - o) * inv) - 1.0;
-                double h = ceil(((double)hi[k] - o) * inv) + 1.0;
-                l = l < 0.0 ? 0.0 : (l > 255.0 ? 255.0 : l);
-                h = h < 0.0 ? 0.0 : (h > 255.0 ? 255.0 : h);
-                while (l > 0.0 && o + l * sc > (double)lo[k]) l -= 1.0;
-                while (h < 255.0 && o + h * sc < (double)hi[k]) h += 1.0;
-                image[32 + 8 * k + slot] = (uint8_t)l;
-                image[56 + 8 * k + slot] = (uint8_t)h;
-            }
-            if (sub == 0 && nc != 0u) {
-                reinterpret_cast<float*>(image)[k] = ok;
-                image[12 + k] = (uint8_t)ek;
-            }
-        }
+        quantise_lanes(image, valid, slot, nc != 0u, lo, hi, nlo, nhi);
         if (valid) s_child[g][slot] = x;
         if (sub == 0) {
             image[15] = (uint8_t)imask;

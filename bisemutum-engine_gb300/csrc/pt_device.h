@@ -179,8 +179,8 @@ void launch_trace_count(cudaStream_t st, const DevScene& sc, const float4* rays,
 // indexed by `idx`, or a soup when idx is null); all pointers are device memory.
 void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const float* vn, const uint32_t* idx,
                            float4* out);
-void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box, uint32_t begin,
-                       uint32_t end);
+void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box,
+                       const uint32_t* level_begin, uint32_t levels);   // levels + 1 boundaries (host memory)
 // Traces the view's camera rays and writes the outputs that are not null (the hit records wait in one of them).
 void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView& v, float near_z,
                     float far_z, float* depth, float4* const gb[4], float4* hitpos, uint32_t* work);

@@ -24,7 +24,7 @@
 #include "pt_scene.cuh"
 #include "pt_lights.cuh"
 #include "pt_gbuffer.cuh"
-#include "bvh_quant.h"
+#include "bvh_quant_lanes.cuh"
 #include "mlp.cuh"
 
 namespace bsm {
@@ -768,43 +768,75 @@ __global__ void __launch_bounds__(256) k_trace_count(DevScene sc, const float4* 
 }
 
 // ------------------------------------------------------------- TLAS refit ----
-// Refits the TLAS for new instance boxes, one BFS level per launch from the
-// deepest up (nodes of a level are contiguous in the builder's breadth-first
-// order).  A node's eight child boxes come from the instance boxes of its leaf
-// slots (TLAS leaves hold one instance) and from the boxes its internal
-// children wrote one launch earlier; the node's frame and bytes are then
-// quantised outward exactly as the host builder does (tlas_quantise).
-__global__ void k_tlas_refit(CwNode* __restrict__ nodes, float* __restrict__ node_box,
-                             const float* __restrict__ inst_box, uint32_t begin, uint32_t end) {
-    uint32_t ni = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (ni >= end) return;
-    CwNode n = nodes[ni];
-    float lo[8][3], hi[8][3];
-    uint32_t used = 0;
-    for (int s = 0; s < 8; ++s) {
-        bool inner = (n.imask >> s) & 1u;
-        if (!inner && ((n.tri_mask >> (2 * s)) & 3u) == 0u) continue;
-        used |= 1u << s;
-        const float* b;
-        if (inner) {
-            uint32_t ci = n.child_base + (uint32_t)__popc((uint32_t)n.imask & ((1u << s) - 1u));
-            b = node_box + 6 * (size_t)ci;
-        } else {
-            b = inst_box + 6 * (size_t)(n.tri_base + (uint32_t)__popc((uint32_t)n.tri_mask & ((1u << (2 * s)) - 1u)));
-        }
-        for (int k = 0; k < 3; ++k) { lo[s][k] = b[k]; hi[s][k] = b[3 + k]; }
+// Refits the TLAS for new instance boxes, a breadth-first level at a time from
+// the deepest up (nodes of a level are contiguous in the builder's order).  A
+// node's eight child boxes come from the instance boxes of its leaf slots (TLAS
+// leaves hold one instance) and from the boxes its internal children wrote a
+// level earlier; the node's frame and bytes are then quantised outward exactly as
+// the host builder does (tlas_quantise), a slot per lane.  A launch per level
+// with a thread per node took 42 us for each of the five levels of 1,000
+// instances; REFIT_NOW.
+__device__ __forceinline__ void refit_node(CwNode* nodes, float* node_box, const float* inst_box, uint32_t ni, bool in) {
+    const uint32_t s = threadIdx.x % kWideLanes;
+    uint32_t imask = 0, tmask = 0, child = 0, tri = 0;
+    if (in) {
+        const CwNode* n = nodes + ni;
+        imask = n->imask;
+        tmask = n->tri_mask;
+        child = n->child_base;
+        tri = n->tri_base;
+    }
+    const bool inner = (imask >> s) & 1u, leaf = !inner && ((tmask >> (2u * s)) & 3u) != 0u;
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (inner || leaf) {
+        const float* b = inner ? node_box + 6 * (size_t)(child + (uint32_t)__popc(imask & ((1u << s) - 1u)))
+                               : inst_box + 6 * (size_t)(tri + (uint32_t)__popc(tmask & ((1u << (2u * s)) - 1u)));
+        for (int k = 0; k < 3; ++k) { lo[k] = b[k]; hi[k] = b[3 + k]; }
     }
     float nlo[3], nhi[3];
-    tlas_quantise(n, lo, hi, used, nlo, nhi);
-    nodes[ni] = n;
-    for (int k = 0; k < 3; ++k) { node_box[6 * (size_t)ni + k] = nlo[k]; node_box[6 * (size_t)ni + 3 + k] = nhi[k]; }
+    for (int k = 0; k < 3; ++k) { nlo[k] = wide_min(lo[k]); nhi[k] = wide_max(hi[k]); }
+    quantise_lanes(reinterpret_cast<uint8_t*>(nodes + ni), inner || leaf, s, in, lo, hi, nlo, nhi);
+    if (in && s < 6u) node_box[6 * (size_t)ni + s] = s == 0 ? nlo[0] : s == 1 ? nlo[1] : s == 2 ? nlo[2]
+                                                   : s == 3 ? nhi[0] : s == 4 ? nhi[1] : nhi[2];
+}
+constexpr uint32_t kRefitThreads = 1024, kRefitNodes = kRefitThreads / kWideLanes;
+struct RefitLevels { uint32_t begin[kMaxTlasDepth + 2]; };
+
+// Levels [0, n) by one block, with barriers between them.
+__global__ void __launch_bounds__(kRefitThreads) k_tlas_refit(CwNode* nodes, float* node_box, const float* inst_box,
+                                                              RefitLevels lv, uint32_t n) {
+    for (uint32_t l = n; l-- > 0u;) {
+        for (uint32_t base = lv.begin[l]; base < lv.begin[l + 1]; base += kRefitNodes) {
+            const uint32_t ni = base + threadIdx.x / kWideLanes;
+            refit_node(nodes, node_box, inst_box, ni, ni < lv.begin[l + 1]);
+        }
+        __syncthreads();
+    }
+}
+// One level by as many blocks as it needs.
+__global__ void __launch_bounds__(256) k_tlas_level(CwNode* nodes, float* node_box, const float* inst_box,
+                                                    uint32_t begin, uint32_t end) {
+    const uint32_t ni = begin + (blockIdx.x * blockDim.x + threadIdx.x) / kWideLanes;
+    refit_node(nodes, node_box, inst_box, ni, ni < end);
 }
 
 // ------------------------------------------------------------ launchers ----
-void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box, uint32_t begin,
-                       uint32_t end) {
-    if (end <= begin) return;
-    k_tlas_refit<<<(end - begin + 127) / 128, 128, 0, st>>>(nodes, node_box, inst_box, begin, end);
+void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box,
+                       const uint32_t* level_begin, uint32_t levels) {
+    // one block takes the levels below the first one that is too wide for a few rounds of it
+    uint32_t narrow = 0;
+    while (narrow < levels && narrow <= (uint32_t)kMaxTlasDepth &&
+           level_begin[narrow + 1] - level_begin[narrow] <= 8u * kRefitNodes)
+        ++narrow;
+    for (uint32_t l = levels; l-- > narrow;) {
+        const uint32_t n = level_begin[l + 1] - level_begin[l];
+        k_tlas_level<<<(n * kWideLanes + 255u) / 256u, 256, 0, st>>>(nodes, node_box, inst_box, level_begin[l],
+                                                                   level_begin[l + 1]);
+    }
+    if (narrow == 0) return;
+    RefitLevels lv{};
+    for (uint32_t l = 0; l <= narrow; ++l) lv.begin[l] = level_begin[l];
+    k_tlas_refit<<<1, kRefitThreads, 0, st>>>(nodes, node_box, inst_box, lv, narrow);
 }
 void launch_camera(const LaunchCfg& lc, cudaStream_t st, const DevView* views, uint32_t n_views,
                    uint64_t path_begin, uint32_t path_count, const Wavefront& wf, uint32_t max_segments) {
