@@ -60,6 +60,7 @@ struct Scene {
     std::vector<uint32_t> level_begin;      // TLAS breadth-first level boundaries (levels + 1 entries)
     std::vector<InstDev> inst_host;         // records in leaf order
     DevBuf insts, inst_box, node_box, mat_tr;
+    DevBuf inst_src, inst_move;             // bsm_scene_update_instances: InstSrc per instance; its working memory
     DevScene dev{};
 };
 
@@ -538,7 +539,7 @@ bsm_status build_tlas(bsm_context* ctx, Scene* sc);
 // Device buffers of a scene; an instanced scene also lets go of its geometries.
 void free_scene_buffers(bsm_context* ctx, Scene& sc) {
     for (DevBuf* b : {&sc.nodes, &sc.tris, &sc.materials, &sc.texels, &sc.sky_alias, &sc.pdf_tab, &sc.tri_normals,
-                      &sc.insts, &sc.inst_box, &sc.node_box, &sc.mat_tr})
+                      &sc.insts, &sc.inst_box, &sc.node_box, &sc.mat_tr, &sc.inst_src, &sc.inst_move})
         dev_free(ctx, *b);
     if (sc.instanced)
         for (const bsm_instance& in : sc.instances) {
@@ -1038,6 +1039,8 @@ void instance_world_box(const float* m, const float glo[3], const float ghi[3], 
     }
 }
 
+constexpr size_t kMoveHeader = 256;   // the sums of launch_inst_move; the moved records and the transforms follow
+
 bool valid_transform(const float* m) {
     for (int i = 0; i < 12; ++i)
         if (!std::isfinite(m[i])) return false;
@@ -1114,6 +1117,16 @@ bsm_status build_tlas(bsm_context* ctx, Scene* sc) {
     CK(cudaMemcpy(sc->nodes.ptr, r.nodes.data(), r.nodes.size() * sizeof(CwNode), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(sc->insts.ptr, sc->inst_host.data(), (size_t)n * sizeof(InstDev), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(sc->inst_box.ptr, boxes.data(), boxes.size() * 4, cudaMemcpyHostToDevice));
+    std::vector<InstSrc> src(n);
+    for (uint32_t i = 0; i < n; ++i) {
+        const Geometry* g = ctx->geoms.at(sc->instances[i].geometry_id).get();
+        src[i].leaf = sc->leaf_of[i];
+        std::memcpy(src[i].lo, g->lo, sizeof(src[i].lo));
+        std::memcpy(src[i].hi, g->hi, sizeof(src[i].hi));
+    }
+    if ((st = dev_alloc(ctx, sc->inst_src, (size_t)n * sizeof(InstSrc)))) return st;
+    if ((st = dev_alloc(ctx, sc->inst_move, kMoveHeader + (size_t)n * (sizeof(InstMoved) + 48)))) return st;
+    CK(cudaMemcpy(sc->inst_src.ptr, src.data(), (size_t)n * sizeof(InstSrc), cudaMemcpyHostToDevice));
     DevScene& ds = sc->dev;
     ds.nodes = (const CwNode*)sc->nodes.ptr;
     ds.tris = nullptr;
@@ -1266,26 +1279,37 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
     if (ctx->server) return fail(ctx, BSM_ERR_BAD_STATE, "scenes cannot change while the server runs");
     if (num_instances != sc->instances.size())
         return fail(ctx, BSM_ERR_INVALID_ARG, "transform count differs from the scene's instances");
-    for (uint32_t i = 0; i < num_instances; ++i)
-        if (!valid_transform(transforms + 12 * (size_t)i))
-            return fail(ctx, BSM_ERR_INVALID_ARG, "instance " + std::to_string(i) + ": transform not finite / invertible");
+    if (!sc->inst_src.ptr || !sc->inst_move.ptr) return fail(ctx, BSM_ERR_BAD_STATE, "the scene's last TLAS build failed");
+    // the new records and boxes beside the current ones, which stay if a transform is refused
+    char* mem = (char*)sc->inst_move.ptr;
+    uint32_t* sum_dev = (uint32_t*)mem;
+    InstMoved* moved = (InstMoved*)(mem + kMoveHeader);
+    float* xf_dev = (float*)(mem + kMoveHeader + (size_t)num_instances * sizeof(InstMoved));
+    uint32_t sum[7];
+    CK(cudaMemsetAsync(sum_dev, 0, sizeof(sum), WS(ctx)));
+    CK(cudaMemcpyAsync(xf_dev, transforms, (size_t)num_instances * 48, cudaMemcpyHostToDevice, WS(ctx)));
+    launch_inst_move(WS(ctx), xf_dev, (const InstSrc*)sc->inst_src.ptr, num_instances, moved, sum_dev);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(sum, sum_dev, sizeof(sum), cudaMemcpyDeviceToHost, WS(ctx)));
+    CK(cudaStreamSynchronize(WS(ctx)));  // also: no render may read the records while they change
+    if (sum[0] != 0u)
+        return fail(ctx, BSM_ERR_INVALID_ARG, "instance " + std::to_string(~sum[0]) + ": transform not finite / invertible");
     for (uint32_t i = 0; i < num_instances; ++i)
         std::memcpy(sc->instances[i].transform, transforms + 12 * (size_t)i, 12 * sizeof(float));
-    std::vector<float> boxes;
-    fill_instances(ctx, sc, boxes);
     // the scene bounds (ray offset, radiance-cache normalisation) follow the instances, as a rebuild's would
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (size_t l = 0; l < sc->inst_host.size(); ++l)
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = std::min(lo[k], boxes[6 * l + k]);
-            hi[k] = std::max(hi[k], boxes[6 * l + 3 + k]);
-        }
+    auto unkey = [](uint32_t k) {
+        const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+        float f;
+        std::memcpy(&f, &b, 4);
+        return f;
+    };
+    float lo[3], hi[3];
+    for (int k = 0; k < 3; ++k) { lo[k] = unkey(~sum[1 + k]); hi[k] = unkey(sum[4 + k]); }
     float extent = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), std::max(hi[2] - lo[2], 1e-6f));
     DevScene& ds = sc->dev;
     bool moved_bounds = extent != sc->extent;
     for (int k = 0; k < 3; ++k)
         moved_bounds = moved_bounds || ds.box_lo[k] != lo[k] || ds.box_inv[k] != 1.0f / std::max(hi[k] - lo[k], 1e-6f);
-    CK(cudaStreamSynchronize(WS(ctx)));  // no render may read the records while they change
     if (moved_bounds) {
         sc->extent = extent;
         ds.ray_offset = 2e-5f * extent;
@@ -1295,9 +1319,7 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
         }
         clear_graphs(ctx);  // captured launches hold the scene record by value
     }
-    CK(cudaMemcpyAsync(sc->insts.ptr, sc->inst_host.data(), sc->inst_host.size() * sizeof(InstDev),
-                       cudaMemcpyHostToDevice, WS(ctx)));
-    CK(cudaMemcpyAsync(sc->inst_box.ptr, boxes.data(), boxes.size() * 4, cudaMemcpyHostToDevice, WS(ctx)));
+    launch_inst_apply(WS(ctx), moved, num_instances, (InstDev*)sc->insts.ptr, (float*)sc->inst_box.ptr);
     launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, (const float*)sc->inst_box.ptr,
                       sc->level_begin.data(), (uint32_t)sc->level_begin.size() - 1u);
     CK(cudaGetLastError());
@@ -1311,7 +1333,7 @@ extern "C" bsm_status bsm_scene_device_bytes(bsm_context* ctx, uint32_t scene_id
     if (!sc) return fail(ctx, BSM_ERR_NOT_FOUND, "unknown scene id");
     uint64_t b = 0;
     for (DevBuf* x : {&sc->nodes, &sc->tris, &sc->materials, &sc->texels, &sc->sky_alias, &sc->pdf_tab,
-                      &sc->tri_normals, &sc->insts, &sc->inst_box, &sc->node_box, &sc->mat_tr})
+                      &sc->tri_normals, &sc->insts, &sc->inst_box, &sc->node_box, &sc->mat_tr, &sc->inst_src, &sc->inst_move})
         b += x->bytes;
     *bytes = b;
     return BSM_OK;

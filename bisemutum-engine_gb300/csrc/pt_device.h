@@ -179,6 +179,14 @@ void launch_trace_count(cudaStream_t st, const DevScene& sc, const float4* rays,
 // indexed by `idx`, or a soup when idx is null); all pointers are device memory.
 void launch_gather_normals(cudaStream_t st, const CwTri* tris, uint32_t n, const float* vn, const uint32_t* idx,
                            float4* out);
+// Moved instances: an instance's TLAS leaf and its geometry's box (caller order), and what its transform gives (leaf
+// order).  launch_inst_move checks the transforms and fills `out` and `sum` (7 words, zero before: see k_inst_move);
+// launch_inst_apply puts the records and boxes in place.
+struct InstSrc { uint32_t leaf; float lo[3], hi[3]; uint32_t pad; };
+struct InstMoved { float w2o[12], o2w[12], box[6], pad[2]; };
+void launch_inst_move(cudaStream_t st, const float* transforms, const InstSrc* src, uint32_t n, InstMoved* out,
+                      uint32_t* sum);
+void launch_inst_apply(cudaStream_t st, const InstMoved* moved, uint32_t n, InstDev* insts, float* inst_box);
 void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const float* inst_box,
                        const uint32_t* level_begin, uint32_t levels);   // levels + 1 boundaries (host memory)
 // Traces the view's camera rays and writes the outputs that are not null (the hit records wait in one of them).
