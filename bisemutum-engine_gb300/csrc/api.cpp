@@ -1407,7 +1407,7 @@ void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t 
             if (count_traversal) launch_extend_count(lc, st, sc->dev, wf, q, seg);
             else launch_trace(lc, st, sc->dev, wf, q, seg, split || seg == 0 ? kNoSegment : seg - 1, accum, count);
             mark(1);
-            launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, cache_wb != nullptr);
+            launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, count, cache_wb != nullptr);
             mark(2);
             if (split || seg + 1 == max_seg) launch_trace(lc, st, sc->dev, wf, q, kNoSegment, seg, accum, count);
             mark(3);

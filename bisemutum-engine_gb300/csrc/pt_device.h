@@ -160,7 +160,7 @@ void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
                          uint32_t seg);
 // `cache`: some view of the launch queries the radiance cache
 void launch_shade(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView* views,
-                  const Wavefront& wf, int q, uint32_t seg, float4* accum, bool cache = false);
+                  const Wavefront& wf, int q, uint32_t seg, float4* accum, uint32_t paths, bool cache = false);
 void launch_resolve(cudaStream_t st, const float4* accum, uint32_t width, uint32_t height, float inv_spp,
                     float4* out, uint32_t pitch_px);
 // accum[p] += fx[3p .. 3p + 2] * 2^-32 for the n accumulator pixels (one add per pixel: deterministic)

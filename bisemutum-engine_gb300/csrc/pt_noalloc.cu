@@ -206,7 +206,7 @@ extern "C" bsm_status bsm_render_noalloc(bsm_context* ctx, uint32_t scene_id, co
         int q = 0;
         for (uint32_t seg = 0; seg < max_seg; ++seg) {
             launch_trace(lc, st, sc, wf, q, seg, seg ? seg - 1 : kNoSegment, accum, count);
-            launch_shade(lc, st, sc, view_dev, wf, q, seg, accum);
+            launch_shade(lc, st, sc, view_dev, wf, q, seg, accum, count);
             q ^= 1;
         }
         launch_trace(lc, st, sc, wf, q, kNoSegment, max_seg - 1, accum, count);

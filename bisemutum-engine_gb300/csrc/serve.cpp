@@ -238,7 +238,7 @@ bool launch_chunk(Server& S, Lane& lane, uint32_t scene) {
     int q = 0;
     for (uint32_t seg = 0; seg < max_seg; ++seg) {
         launch_trace(S.lc, st, sc, lane.wf, q, seg, seg ? seg - 1 : kNoSegment, S.pool_mem, (uint32_t)base);
-        launch_shade(S.lc, st, sc, lane.views_dev, lane.wf, q, seg, S.pool_mem);
+        launch_shade(S.lc, st, sc, lane.views_dev, lane.wf, q, seg, S.pool_mem, (uint32_t)base);
         q ^= 1;
     }
     launch_trace(S.lc, st, sc, lane.wf, q, kNoSegment, max_seg - 1, S.pool_mem, (uint32_t)base);
