@@ -274,6 +274,30 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_trace(const CwNode* __restr
     trace_queue<false, kOpacity>(nodes, tris, rays.n, rays.work(), rays, nullptr, a.postpone_sp, a.refill_min);
 }
 
+// The camera rays of chunks over the group kernel's limit: a ray per thread,
+// in queue order and without the persistent loop.  The rays of a warp are an
+// 8x4 tile of pixels or the samples of one pixel and walk the same nodes, so
+// handing finished lanes rays of another tile gains nothing, and the loop's
+// votes, queue reads and postponed leaves are instructions in a launch that is
+// bound by their issue.  Against k_trace for these rays: 1920x1080 frame of
+// the 1.48 M-triangle terrain with 64 spp 161.4 -> 158.5 ms, with one
+// 3744 -> 3620 us, 256x256x16 room 1119 -> 1088 us.  64 registers (8 blocks of
+// 128 an SM): without the bound 159.6 ms.  In two levels the same change loses
+// (1287 -> 1395 us): rays of one tile enter different instances.
+template <bool kOpacity>
+__global__ void __launch_bounds__(128, 8) k_trace_first(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
+                                                        const __grid_constant__ TraceArgs a) {
+    const TraceRays rays = trace_rays(a);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rays.n) return;
+    float4 o, d;
+    rays.load(i, o, d);
+    float t, u, v;
+    const uint32_t leaf =
+        trace_ray<false, false>(make_ray(o, d), d.w, nodes, tris, t, u, v, nullptr, kOpacity ? rays.seed(i) : 0u);
+    rays.hit(i, leaf, t, u, v, kMissPrim);
+}
+
 // k_trace for small chunks and short queues: eight lanes per ray.  A
 // kernel of its own, because its loop in k_trace costs that one registers
 // (1080p 64-spp frame 160.8 -> 168.7 ms with both), and 80 registers are worth
@@ -983,6 +1007,12 @@ void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, cons
                 lc.postpone_sp, lc.refill_min};
     const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr;
     const bool only = paths <= (two ? kGroupPaths2 : kGroupPaths), mix = !only && paths <= kMixedPaths && ext != 0u;
+    if (!only && !two && ext == 0u && shd == kNoSegment) {
+        const uint32_t grid = (uint32_t)(((uint64_t)paths + 127u) / 128u);
+        if (op) k_trace_first<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+        else k_trace_first<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+        return;
+    }
     const uint32_t limit = two ? kGroupQueue2 : kGroupQueue;
     if (only || mix) {
         if (mix) a.max_rays = limit;
