@@ -228,15 +228,17 @@ __global__ void __launch_bounds__(1024) k_level_chunks(Task* __restrict__ tasks,
 
 // Adds a warp's references to one axis' shared bins.  Neighbouring references
 // mostly share a bin (they are in input order within a node), and 32 atomics on
-// one address take turns, so up to three groups of lanes with a common bin are
-// reduced in registers first.
+// one address take turns, so up to three groups of eight or more lanes with a
+// common bin are reduced in registers first (builds of 1.48 M / 4.97 M triangles:
+// one group 4.78 / 13.56 ms, two 4.69 / 13.26, three 4.70 / 13.36, six 4.73 / 13.46;
+// three groups of at least 2 / 4 / 8 lanes 4.73 / 13.57, 4.70 / 13.36, 4.68 / 13.21).
 __device__ __forceinline__ void bin_axis(Bin* sb, bool act, uint32_t bin, const uint32_t* kl, const uint32_t* kh) {
     uint32_t rest = __ballot_sync(0xffffffffu, act);
     for (int round = 0; round < 3 && rest != 0u; ++round) {
         const int leader = __ffs(rest) - 1;
         const uint32_t lb = __shfl_sync(0xffffffffu, bin, leader);
         const uint32_t m = __ballot_sync(0xffffffffu, bin == lb) & rest;
-        if (__popc(m) < 4) break;
+        if (__popc(m) < 8) break;
         if ((m >> (threadIdx.x & 31u)) & 1u) {
             uint32_t lo[3], hi[3];
             for (int k = 0; k < 3; ++k) { lo[k] = __reduce_min_sync(m, kl[k]); hi[k] = __reduce_max_sync(m, kh[k]); }
@@ -276,15 +278,20 @@ __global__ void __launch_bounds__(kLevelThreads) k_bin(const uint32_t* __restric
         const uint32_t begin = tk.begin + (c - tk.aux) * chunk, end = min(tk.end, begin + chunk);
         float sc[3];
         for (int a = 0; a < 3; ++a) sc[a] = axis_scale(tk, a, B);
-        for (uint32_t base = begin; base < end; base += blockDim.x) {
-            const uint32_t i = base + threadIdx.x;
+        uint32_t i = begin + threadIdx.x;
+        float4 nl = make_float4(0, 0, 0, 0), nh = nl;
+        auto fetch = [&]() {
+            if (i >= end) return;
+            const uint32_t r = refs[i];
+            nl = box[2 * (size_t)r];
+            nh = box[2 * (size_t)r + 1];
+        };
+        fetch();
+        for (uint32_t base = begin; base < end; base += kLevelThreads) {
             const bool act = i < end;
-            float4 l = make_float4(0, 0, 0, 0), h = l;
-            if (act) {
-                const uint32_t r = refs[i];
-                l = box[2 * (size_t)r];
-                h = box[2 * (size_t)r + 1];
-            }
+            const float4 l = nl, h = nh;
+            i += kLevelThreads;
+            fetch();   // the next references' boxes, while these are binned (42 -> 39 us a level)
             const uint32_t kl[3] = {fkey(l.x), fkey(l.y), fkey(l.z)}, kh[3] = {fkey(h.x), fkey(h.y), fkey(h.z)};
             for (int a = 0; a < 3; ++a) {
                 if (!(sc[a] > 0.0f)) continue;   // the same for the whole block
@@ -313,9 +320,11 @@ static_assert(kBins == 32 && kChunk < 65536, "a warp scans an axis' bins; a chun
 // The least-cost split over three axes of binned SAH (bvh_build.cpp Builder::build):
 // cost(split before bin b) = area(left) * n_left + area(right) * n_right, axes
 // in order and bins ascending, the first minimum kept.  One warp; lane = bin.
-// `bins(a)` returns this lane's bin of axis a.  Returns the axis (-1: none).
+// `bins(a)` returns this lane's bin of axis a.  Returns the axis (-1: none); the
+// boxes of the two sides are left in lane *best_bin.
 template <class GetBin>
-__device__ int warp_best_split(const Task& tk, int B, GetBin bins, int* best_bin, uint32_t* best_nl, float* best_cost) {
+__device__ int warp_best_split(const Task& tk, int B, GetBin bins, int* best_bin, uint32_t* best_nl, float* best_cost,
+                               float side[2][6]) {
     const int lane = threadIdx.x & 31;
     float best = INFINITY;
     int bax = -1, bbin = 0;
@@ -368,7 +377,10 @@ __device__ int warp_best_split(const Task& tk, int B, GetBin bins, int* best_bin
             if (om < m || (om == m && ol < ml)) { m = om; ml = ol; }
         }
         uint32_t nl_at = __shfl_sync(0xffffffffu, pn, ml);
-        if (m < best) { best = m; bax = a; bbin = ml; bnl = nl_at; }
+        if (m < best) {
+            best = m; bax = a; bbin = ml; bnl = nl_at;
+            for (int k = 0; k < 3; ++k) { side[0][k] = pl[k]; side[0][3 + k] = ph[k]; side[1][k] = rlo[k]; side[1][3 + k] = rhi[k]; }
+        }
     }
     *best_bin = bbin;
     *best_nl = bnl;
@@ -399,19 +411,22 @@ __device__ __forceinline__ Split decide(int bax, int bbin, uint32_t bnl, float b
 // where its chunks' left references go.
 __global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins, const ChunkBins* __restrict__ cbins,
                         const BNode* __restrict__ nodes, Split* __restrict__ splits, uint32_t* __restrict__ left_base,
-                        Counters* cnt, int cur, uint32_t chunk, int B, uint32_t max_leaf) {
+                        ChildAcc* __restrict__ acc, Counters* cnt, int cur, uint32_t chunk, int B, uint32_t max_leaf) {
     const int lane = threadIdx.x & 31;
     const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur], warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nt; w += warps) {
         const Task tk = tasks[w];
         int bbin;
         uint32_t bnl;
-        float best;
+        float best, side[2][6];
         int bax = warp_best_split(tk, B, [&](int a) {
             Bin e;
             e.cnt = 0;
             return lane < B ? gbins[((size_t)w * 3 + a) * kBins + lane] : e;
-        }, &bbin, &bnl, &best);
+        }, &bbin, &bnl, &best, side);
+        if (bax >= 0 && lane == bbin)
+            for (int c = 0; c < 2; ++c)
+                for (int k = 0; k < 6; ++k) acc[w].box[c][k] = fkey(side[c][k]);
         Bin z;
         z.cnt = 0;
         for (int k = 0; k < 3; ++k) { z.lo[k] = kKeyLo; z.hi[k] = kKeyHi; }
@@ -451,9 +466,16 @@ __device__ __forceinline__ bool goes_left(const Task& tk, const Split& sp, uint3
 }
 
 // Stable partition of a chunk: its left references from left_base on, its right
-// ones behind the task's left part (both in chunk order); the children's boxes
-// and centroid bounds are reduced over the block and merged into the task's.
-__global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __restrict__ chunk_task,
+// ones behind the task's left part (both in chunk order); the children's
+// centroid bounds are reduced over the block and merged into the task's.  Their
+// boxes are already there, from the split's bins, unless the task was split by
+// index.  Bound by the latency of reference, box and barrier in turn: the next
+// box is fetched over the one barrier of a round, and without the boxes'
+// minima the kernel fits five blocks an SM (51 registers; 70 before, 1.6 waves
+// of the 724 chunks of 1.48 M triangles).  37 -> 17 us a level there, 0.53 ->
+// 0.31 ms over the build; with four blocks an SM the build takes 4.75 ms
+// against 4.70.
+__global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* __restrict__ chunk_task,
                                                              const Task* __restrict__ tasks,
                                                              const Split* __restrict__ splits,
                                                              const uint32_t* __restrict__ left_base,
@@ -461,9 +483,10 @@ __global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __r
                                                              uint32_t* __restrict__ out,
                                                              const float4* __restrict__ box,
                                                              ChildAcc* __restrict__ acc, const Counters* cnt, uint32_t chunk, int B) {
-    __shared__ uint32_t s_wl[kLevelThreads / 32], s_wr[kLevelThreads / 32];
-    __shared__ float s_red[kLevelThreads / 32][24];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    constexpr int kWarps = kLevelThreads / 32;
+    __shared__ uint32_t s_wl[2][kWarps], s_wr[2][kWarps];
+    __shared__ float s_red[kWarps][12];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t nch = cnt->error ? 0u : cnt->chunks;   // after an error the offsets may be wrong
     for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
@@ -471,70 +494,62 @@ __global__ void __launch_bounds__(kLevelThreads) k_partition(const uint32_t* __r
         const Task tk = tasks[ti];
         const Split sp = splits[ti];
         const uint32_t begin = tk.begin + (c - tk.aux) * chunk, end = min(tk.end, begin + chunk);
-        float v[24];   // side s: box lo(3) hi(3), centroid lo(3) hi(3) at 12 s
-        for (int s = 0; s < 2; ++s)
-            for (int k = 0; k < 3; ++k) {
-                v[12 * s + k] = v[12 * s + 6 + k] = INFINITY;
-                v[12 * s + 3 + k] = v[12 * s + 9 + k] = -INFINITY;
-            }
+        float v[12];   // centroid lo(3) hi(3) of the left side, then of the right
+        for (int k = 0; k < 12; ++k) v[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
         uint32_t lb = left_base[c], rb = tk.begin + sp.nl + (begin - lb);
-        for (uint32_t base = begin; base < end; base += blockDim.x) {
-            const uint32_t i = base + threadIdx.x;
+        uint32_t r = 0, i = begin + threadIdx.x;
+        float4 l = make_float4(0, 0, 0, 0), h = l;
+        if (i < end) { r = in[i]; l = box[2 * (size_t)r]; h = box[2 * (size_t)r + 1]; }
+        int par = 0;
+        for (uint32_t base = begin; base < end; base += kLevelThreads, i += kLevelThreads, par ^= 1) {
             const bool act = i < end;
-            uint32_t r = 0;
-            float4 l = make_float4(0, 0, 0, 0), h = l;
-            bool left = false;
-            if (act) {
-                r = in[i];
-                l = box[2 * (size_t)r];
-                h = box[2 * (size_t)r + 1];
-                left = goes_left(tk, sp, i, l, h, B);
-            }
-            const bool right = act && !left;
+            const bool left = act && goes_left(tk, sp, i, l, h, B), right = act && !left;
             const uint32_t wl = __ballot_sync(0xffffffffu, left), wr = __ballot_sync(0xffffffffu, right);
-            if (lane == 0) { s_wl[warp] = __popc(wl); s_wr[warp] = __popc(wr); }
-            __syncthreads();
-            uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
-            for (int w = 0; w < nw; ++w) {
-                if (w < warp) { pl += s_wl[w]; pr += s_wr[w]; }
-                tl += s_wl[w];
-                tr += s_wr[w];
-            }
-            if (left) out[lb + pl + __popc(wl & lt)] = r;
-            if (right) out[rb + pr + __popc(wr & lt)] = r;
-            lb += tl;
-            rb += tr;
-            __syncthreads();
+            if (lane == 0) { s_wl[par][warp] = __popc(wl); s_wr[par][warp] = __popc(wr); }
+            // the next references' boxes are on their way over the barrier (which also keeps this half of the
+            // counts until every warp is past the reads below)
+            const uint32_t r_now = r;
+            const float4 l_now = l, h_now = h;
+            if (i + kLevelThreads < end) { r = in[i + kLevelThreads]; l = box[2 * (size_t)r]; h = box[2 * (size_t)r + 1]; }
             if (act) {
-                const float lo[3] = {l.x, l.y, l.z}, hi[3] = {h.x, h.y, h.z};
-                for (int k = 0; k < 3; ++k) {
-                    const float cc = 0.5f * (lo[k] + hi[k]);
-                    if (left) {
-                        v[k] = fminf(v[k], lo[k]); v[3 + k] = fmaxf(v[3 + k], hi[k]);
-                        v[6 + k] = fminf(v[6 + k], cc); v[9 + k] = fmaxf(v[9 + k], cc);
-                    } else {
-                        v[12 + k] = fminf(v[12 + k], lo[k]); v[15 + k] = fmaxf(v[15 + k], hi[k]);
-                        v[18 + k] = fminf(v[18 + k], cc); v[21 + k] = fmaxf(v[21 + k], cc);
+                if (sp.axis < 0)   // no bins: one centroid for all of them
+                    for (int k = 0; k < 3; ++k) {
+                        uint32_t* b = acc[ti].box[left ? 0 : 1];
+                        atomicMin(b + k, fkey(k == 0 ? l_now.x : k == 1 ? l_now.y : l_now.z));
+                        atomicMax(b + 3 + k, fkey(k == 0 ? h_now.x : k == 1 ? h_now.y : h_now.z));
                     }
+                for (int k = 0; k < 3; ++k) {
+                    const float cc = centroid(l_now, h_now, k);
+                    if (left) { v[k] = fminf(v[k], cc); v[3 + k] = fmaxf(v[3 + k], cc); }
+                    else { v[6 + k] = fminf(v[6 + k], cc); v[9 + k] = fmaxf(v[9 + k], cc); }
                 }
             }
+            __syncthreads();
+            uint32_t pl = 0, pr = 0, tl = 0, tr = 0;
+            for (int w = 0; w < kWarps; ++w) {
+                if (w < warp) { pl += s_wl[par][w]; pr += s_wr[par][w]; }
+                tl += s_wl[par][w];
+                tr += s_wr[par][w];
+            }
+            if (left) out[lb + pl + __popc(wl & lt)] = r_now;
+            if (right) out[rb + pr + __popc(wr & lt)] = r_now;
+            lb += tl;
+            rb += tr;
         }
-        for (int k = 0; k < 24; ++k) {
+        for (int k = 0; k < 12; ++k) {
             const uint32_t key = fkey(v[k]);
-            const bool mx = (k % 6) >= 3;
-            const uint32_t m = mx ? __reduce_max_sync(0xffffffffu, key) : __reduce_min_sync(0xffffffffu, key);
+            const uint32_t m = (k % 6) >= 3 ? __reduce_max_sync(0xffffffffu, key) : __reduce_min_sync(0xffffffffu, key);
             if (lane == 0) s_red[warp][k] = funkey(m);
         }
         __syncthreads();
-        if (threadIdx.x < 24) {
+        if (threadIdx.x < 12) {
             const int k = threadIdx.x;
             const bool mx = (k % 6) >= 3;
-            float r = s_red[0][k];
-            for (int w = 1; w < nw; ++w) r = mx ? fmaxf(r, s_red[w][k]) : fminf(r, s_red[w][k]);
-            if (r != INFINITY && r != -INFINITY) {   // else that side is empty in this chunk
-                const int side = k / 12, j = k % 12;
-                uint32_t* dst = j < 6 ? &acc[ti].box[side][j] : &acc[ti].cen[side][j - 6];
-                if (mx) atomicMax(dst, fkey(r)); else atomicMin(dst, fkey(r));
+            float x = s_red[0][k];
+            for (int w = 1; w < kWarps; ++w) x = mx ? fmaxf(x, s_red[w][k]) : fminf(x, s_red[w][k]);
+            if (x != INFINITY && x != -INFINITY) {   // else that side is empty in this chunk
+                uint32_t* dst = &acc[ti].cen[k / 6][k % 6];
+                if (mx) atomicMax(dst, fkey(x)); else atomicMin(dst, fkey(x));
             }
         }
         __syncthreads();
@@ -847,18 +862,15 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __res
         __syncwarp();
         int bbin;
         uint32_t bnl;
-        float best;
+        float best, bx[2][6];
         int bax = warp_best_split(tk, B, [&](int a) {
             Bin z;
             z.cnt = 0;
             return lane < B ? SB[a * kBins + lane] : z;
-        }, &bbin, &bnl, &best);
+        }, &bbin, &bnl, &best, bx);
         const Split s = decide(bax, bbin, bnl, best, n, area, max_leaf);   // never a leaf: leaves hold at most two
         __syncwarp();
-        // stable partition through T, with the children's boxes
-        float bx[2][6];
-        for (int c = 0; c < 2; ++c)
-            for (int k = 0; k < 3; ++k) { bx[c][k] = INFINITY; bx[c][3 + k] = -INFINITY; }
+        // stable partition through T
         uint32_t lc = 0, rc = 0;
         for (uint32_t base = b; base < e; base += 32) {
             const uint32_t i = base + lane;
@@ -880,12 +892,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __res
             if (act) {
                 const uint32_t at = left ? lc + __popc(wl & lt) : s.nl + rc + __popc(wr & lt);
                 T.ref[at] = S.ref[i];
-                for (int k = 0; k < 3; ++k) {
-                    T.lo[k][at] = lo[k];
-                    T.hi[k][at] = hi[k];
-                    if (left) { bx[0][k] = fminf(bx[0][k], lo[k]); bx[0][3 + k] = fmaxf(bx[0][3 + k], hi[k]); }
-                    else { bx[1][k] = fminf(bx[1][k], lo[k]); bx[1][3 + k] = fmaxf(bx[1][3 + k], hi[k]); }
-                }
+                for (int k = 0; k < 3; ++k) { T.lo[k][at] = lo[k]; T.hi[k][at] = hi[k]; }
             }
             lc += __popc(wl);
             rc += __popc(wr);
@@ -895,9 +902,21 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __res
             S.ref[b + i] = T.ref[i];
             for (int k = 0; k < 3; ++k) { S.lo[k][b + i] = T.lo[k][i]; S.hi[k][b + i] = T.hi[k][i]; }
         }
-        for (int c = 0; c < 2; ++c)
-            for (int k = 0; k < 3; ++k) { bx[c][k] = warp_min(bx[c][k]); bx[c][3 + k] = warp_max(bx[c][3 + k]); }
         const uint32_t mid = b + s.nl;
+        int writer = bbin;   // the children's boxes are in the lane of the split's bin
+        if (s.axis < 0) {    // split by index: no bins
+            writer = 0;
+            for (int c = 0; c < 2; ++c)
+                for (int k = 0; k < 3; ++k) {
+                    float lo = INFINITY, hi = -INFINITY;
+                    for (uint32_t i = (c ? mid : b) + lane; i < (c ? e : mid); i += 32) {
+                        lo = fminf(lo, T.lo[k][i - b]);
+                        hi = fmaxf(hi, T.hi[k][i - b]);
+                    }
+                    bx[c][k] = warp_min(lo);
+                    bx[c][3 + k] = warp_max(hi);
+                }
+        }
         uint32_t id = 0;
         if (lane == 0) id = atomicAdd(&cnt->nodes, 2u);
         id = __shfl_sync(0xffffffffu, id, 0);
@@ -905,7 +924,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __res
             if (lane == 0) atomicOr(&cnt->error, kErrNodes);
             return;
         }
-        if (lane == 0) {
+        if (lane == writer) {
             nodes[node].left = id;
             nodes[node].right = id + 1u;
             write_child(nodes, id, node, bx[0], bx[0] + 3, root.begin + b, s.nl);
@@ -1527,7 +1546,7 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
                     k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, chunk,
                                                           B);
                     k_split<<<std::min(blocks_for((uint64_t)max_tasks * 32, 128), (uint32_t)sms * 8u), 128, 0, st>>>(
-                        tasks[cur], bins, chunk_bins, bnodes, splits, left_base, cnt, cur, chunk, B, bin_leaf);
+                        tasks[cur], bins, chunk_bins, bnodes, splits, left_base, acc, cnt, cur, chunk, B, bin_leaf);
                     k_partition<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], splits, left_base, refs[cur],
                                                                 refs[cur ^ 1], box, acc, cnt, chunk, B);
                     k_make_children<<<std::min(blocks_for(max_tasks, 64), (uint32_t)sms * 4u), 64, 0, st>>>(
