@@ -962,6 +962,11 @@ __device__ __forceinline__ void add_sah(double v, double* sums) {
 
 // cost(n, i) for i = 1..8 and the decisions, as the host's Collapse::run; the
 // nodes' areas and leaf counts go to the tree's SAH cost on the way.
+// A climb is one round trip to L2 after another: the parent's node is loaded
+// while its counter is on the way, the node's own costs stay in registers, and
+// the counter's atomic releases and acquires by itself, which costs less than a
+// full fence on both sides of it (builds of 1.48 M / 4.97 M triangles 4.67 /
+// 13.2 -> 4.63 / 13.05 ms; with the fences kept 4.69 / 13.3).
 __device__ __forceinline__ double climb(const BNode* __restrict__ nodes, uint32_t n, uint32_t i,
                                         uint32_t* __restrict__ visits, float4* __restrict__ cost,
                                         uint2* __restrict__ dec, uint8_t* __restrict__ isplit, uint32_t max_leaf,
@@ -970,29 +975,32 @@ __device__ __forceinline__ double climb(const BNode* __restrict__ nodes, uint32_
     const BNode L = nodes[i];
     if (L.left != kNone) return 0.0;   // climbs start at leaves
     double sah;
+    float c[8];   // the costs of the node just finished
     {
         const float a = area6(L.lo, L.hi);
         sah = (double)a * (double)L.count;
         const float leaf = L.count <= max_leaf ? a * (float)L.count * tri_cost : INFINITY;
+        for (int k = 0; k < 8; ++k) c[k] = leaf;
         cost[2 * (size_t)i] = make_float4(leaf, leaf, leaf, leaf);
         cost[2 * (size_t)i + 1] = make_float4(leaf, leaf, leaf, leaf);
         constexpr uint32_t same = kDecSame * 0x01010101u;
         dec[i] = make_uint2((same & 0xffffff00u) | kDecLeaf, same);
     }
-    __threadfence();
-    uint32_t x = L.parent;
+    uint32_t x = L.parent, from = i;
     for (uint32_t guard = 0; x != kNone; ++guard) {
         if (guard > n) { atomicOr(&cnt->error, kErrClimb); return sah; }
-        if (atomicAdd(&visits[x], 1u) == 0u) return sah;   // the other child is not done yet
-        __threadfence();
+        // the parent's node (earlier kernels') comes with the answer whether the other child is done
         const BNode X = nodes[x];
+        uint32_t before;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(visits + x) : "memory");
+        if (before == 0u) return sah;
+        const bool right = X.right == from;
+        const uint32_t other = right ? X.left : X.right;
+        const float4 oa = __ldcg(&cost[2 * (size_t)other]), ob = __ldcg(&cost[2 * (size_t)other + 1]);
+        const float o[8] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
         float cl[8], cr[8];
-        {
-            const float4 a = __ldcg(&cost[2 * (size_t)X.left]), b = __ldcg(&cost[2 * (size_t)X.left + 1]);
-            const float4 c = __ldcg(&cost[2 * (size_t)X.right]), d = __ldcg(&cost[2 * (size_t)X.right + 1]);
-            cl[0] = a.x; cl[1] = a.y; cl[2] = a.z; cl[3] = a.w; cl[4] = b.x; cl[5] = b.y; cl[6] = b.z; cl[7] = b.w;
-            cr[0] = c.x; cr[1] = c.y; cr[2] = c.z; cr[3] = c.w; cr[4] = d.x; cr[5] = d.y; cr[6] = d.z; cr[7] = d.w;
-        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { cl[k] = right ? o[k] : c[k]; cr[k] = right ? c[k] : o[k]; }
         float dist[9];
         uint32_t arg[9];
 #pragma unroll
@@ -1009,7 +1017,6 @@ __device__ __forceinline__ double climb(const BNode* __restrict__ nodes, uint32_
         sah += (double)a;
         const float leaf = X.count <= max_leaf ? a * (float)X.count * tri_cost : INFINITY;
         const float inner = a + dist[8];   // node cost 1
-        float c[8];
         uint32_t d[2] = {0u, 0u};
         if (leaf <= inner) { c[0] = leaf; d[0] = kDecLeaf; } else { c[0] = inner; d[0] = kDecInner; }
 #pragma unroll
@@ -1023,13 +1030,13 @@ __device__ __forceinline__ double climb(const BNode* __restrict__ nodes, uint32_
         cost[2 * (size_t)x + 1] = make_float4(c[4], c[5], c[6], c[7]);
         dec[x] = make_uint2(d[0], d[1]);
         isplit[x] = (uint8_t)arg[8];
-        __threadfence();
+        from = x;
         x = X.parent;
     }
     return sah;
 }
 
-__global__ void __launch_bounds__(256) k_collapse(const BNode* __restrict__ nodes, uint32_t n,
+__global__ void __launch_bounds__(256, 6) k_collapse(const BNode* __restrict__ nodes, uint32_t n,
                                                   uint32_t* __restrict__ visits, float4* __restrict__ cost,
                                                   uint2* __restrict__ dec, uint8_t* __restrict__ isplit,
                                                   uint32_t max_leaf, float tri_cost, double* sah, Counters* cnt) {
