@@ -94,6 +94,7 @@ struct bsm_context {
     cudaStream_t stream = nullptr;     // the context's own stream (and the one renders are captured on)
     cudaStream_t user_stream = nullptr;  // bsm_set_stream: the caller's stream, or null
     bool has_user_stream = false;
+    cudaStream_t side = nullptr;       // a cached frame's training, beside its render (made by the first such frame)
     uint32_t pending_flags = 0;        // device error flags read back but not yet reported
     uint32_t* noalloc_counters = nullptr;  // counters of the last bsm_render_noalloc call (its fixed array)
     bsm_render_stats last_stats{};     // host-side part of the last render's statistics
@@ -456,6 +457,7 @@ extern "C" void bsm_destroy(bsm_context* ctx) {
     cudaFree(ctx->stage_work);
     for (auto& ev : ctx->ev) if (ev) cudaEventDestroy(ev);
     for (auto& ev : ctx->stage_ev) cudaEventDestroy(ev);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -1366,6 +1368,14 @@ extern "C" void bsm_pt_settings_default(bsm_pt_settings* s) {
 
 namespace {
 
+// The cache's answers to the queries of a chunk's paths.
+void record_cache(bsm_context* ctx, cudaStream_t st, const void* cache_wb, uint32_t capacity, uint32_t fx_px) {
+    const Wavefront& wf = ctx->wf;
+    launch_mlp_infer(ctx->device, st, cache_wb, wf.cache_q, wf.counters + kCntCache, capacity,
+                     (float4*)ctx->accum.ptr, fx_px ? (unsigned long long*)ctx->accum_fx.ptr : nullptr,
+                     wf.counters + kCntError);
+}
+
 // Records the launch sequence of one render (all chunks) on `st` (the capture
 // stream when a graph is being recorded, else the work stream).
 // With `ev` non-null an event is recorded after every launch (no host waits):
@@ -1375,7 +1385,7 @@ namespace {
 // call's fx_px accumulator pixels, added to the FP32 accumulator at the end.
 void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t n_views, uint64_t total_paths,
                    uint32_t capacity, uint32_t max_seg, bool count_traversal, std::vector<cudaEvent_t>* ev,
-                   std::vector<int>* tags, const void* cache_wb = nullptr, uint32_t fx_px = 0) {
+                   std::vector<int>* tags, bool cached, const void* cache_wb = nullptr, uint32_t fx_px = 0) {
     const LaunchCfg& lc = ctx->lc;
     const DevView* views = (const DevView*)ctx->views_dev.ptr;
     float4* accum = (float4*)ctx->accum.ptr;
@@ -1407,17 +1417,15 @@ void record_render(bsm_context* ctx, cudaStream_t st, const Scene* sc, uint32_t 
             if (count_traversal) launch_extend_count(lc, st, sc->dev, wf, q, seg);
             else launch_trace(lc, st, sc->dev, wf, q, seg, split || seg == 0 ? kNoSegment : seg - 1, accum, count);
             mark(1);
-            launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, count, cache_wb != nullptr);
+            launch_shade(lc, st, sc->dev, views, wf, q, seg, accum, count, cached);
             mark(2);
             if (split || seg + 1 == max_seg) launch_trace(lc, st, sc->dev, wf, q, kNoSegment, seg, accum, count);
             mark(3);
             q ^= 1;
         }
-        if (cache_wb)
-            launch_mlp_infer(ctx->device, st, cache_wb, wf.cache_q, wf.counters + kCntCache, capacity, accum,
-                             wf.accum_fx, wf.counters + kCntError);
+        if (cache_wb) record_cache(ctx, st, cache_wb, capacity, fx_px);
     }
-    if (fx_px) launch_fold_fixed(st, wf.accum_fx, accum, fx_px);
+    if (fx_px && (cache_wb || !cached)) launch_fold_fixed(st, wf.accum_fx, accum, fx_px);
 }
 
 }  // namespace
@@ -1456,10 +1464,25 @@ struct ViewReq {
     uint64_t seed;
 };
 
+// The training of a cached frame whose paths are being traced on the side stream while its render runs.
+struct SideTraining {
+    bsm_cache* cache;
+    const bsm_cache_settings& cs;
+    float* loss;
+    bool done = false;
+    bsm_status finish(bsm_context* ctx) {
+        done = true;
+        bsm_status e = cache_train_steps(cache, cs, ctx->side, loss);
+        return e ? fail(ctx, e, "radiance-cache training failed") : BSM_OK;
+    }
+};
+
+// With `train` the frame is rendered up to its cache queries first, then the training ends, then the queries are
+// answered with the trained weights (`cache_wb` is not read: training may change which weights renders use).
 bsm_status render_impl(bsm_context* ctx, uint32_t scene_id, const std::vector<ViewReq>& req,
                        const bsm_pt_settings& s, const bsm_view_output* outputs, bsm_render_stats* stats,
                        const void* cache_wb = nullptr, uint32_t cache_seg = 0, float cache_rough = 0.0f,
-                       bool start_recorded = false) {
+                       bool start_recorded = false, SideTraining* train = nullptr) {
     const uint32_t n_views = (uint32_t)req.size();
     cudaSetDevice(ctx->device);
     Scene* sc = find_scene(ctx, scene_id);
@@ -1554,6 +1577,13 @@ bsm_status render_impl(bsm_context* ctx, uint32_t scene_id, const std::vector<Vi
         clear_graphs(ctx);
         if ((st = dev_alloc(ctx, ctx->accum_fx, (size_t)fx_px * 24))) return st;
     }
+    if (train && total_paths > capacity) {   // every chunk ends with its queries
+        if ((st = train->finish(ctx))) return st;
+        cache_wb = cache_render_weights(train->cache);
+        train = nullptr;
+    }
+    const bool cached = cache_wb != nullptr;
+    if (train) cache_wb = nullptr;
     float stage_ms[4] = {0, 0, 0, 0};
     std::vector<int> tags;
     if (!start_recorded) CK(cudaEventRecord(ctx->ev[8], WS(ctx)));   // start of the device time of this render
@@ -1562,7 +1592,7 @@ bsm_status render_impl(bsm_context* ctx, uint32_t scene_id, const std::vector<Vi
         std::vector<uint8_t> key(72);
         uint64_t kv[9] = {(uint64_t)scene_id, (uint64_t)n_views, total_paths,
                           capacity | ((uint64_t)ctx->lc.postpone_sp << 32) | ((uint64_t)ctx->lc.refill_min << 40),
-                          max_seg | ((uint64_t)(uintptr_t)cache_wb << 8), (uint64_t)(uintptr_t)ctx->wf_buf.ptr,
+                          max_seg | ((train ? 1u : (uint64_t)(uintptr_t)cache_wb) << 8), (uint64_t)(uintptr_t)ctx->wf_buf.ptr,
                           (uint64_t)(uintptr_t)ctx->accum.ptr,
                           (uint64_t)(uintptr_t)ctx->views_dev.ptr ^ ((uint64_t)ctx->lc_block << 56),
                           fx_px ? (uint64_t)(uintptr_t)ctx->accum_fx.ptr : 0u};
@@ -1573,7 +1603,7 @@ bsm_status render_impl(bsm_context* ctx, uint32_t scene_id, const std::vector<Vi
             cudaGraph_t graph;
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
             record_render(ctx, ctx->stream, sc, n_views, total_paths, capacity, max_seg, false, nullptr, nullptr,
-                          cache_wb, fx_px);
+                          cached, cache_wb, fx_px);
             CK(cudaStreamEndCapture(ctx->stream, &graph));
             CK(cudaGraphInstantiate(&exec, graph, 0));
             cudaGraphDestroy(graph);
@@ -1586,9 +1616,19 @@ bsm_status render_impl(bsm_context* ctx, uint32_t scene_id, const std::vector<Vi
         CK(cudaGraphLaunch(exec, WS(ctx)));
     } else {
         record_render(ctx, WS(ctx), sc, n_views, total_paths, capacity, max_seg, counting,
-                      timing ? &ctx->stage_ev : nullptr, &tags, cache_wb, fx_px);
+                      timing ? &ctx->stage_ev : nullptr, &tags, cached, cache_wb, fx_px);
     }
     CK(cudaGetLastError());
+    if (train) {
+        if ((st = train->finish(ctx))) {
+            for (uint32_t v = 0; v < n_views; ++v) ctx->hist[v].valid = false;   // the sums hold part of this frame
+            return st;
+        }
+        // the training is over on the device too: its last call waits for the side stream
+        record_cache(ctx, WS(ctx), cache_render_weights(train->cache), capacity, fx_px);
+        if (fx_px) launch_fold_fixed(WS(ctx), (unsigned long long*)ctx->accum_fx.ptr, (float4*)ctx->accum.ptr, fx_px);
+        CK(cudaGetLastError());
+    }
     CK(cudaEventRecord(ctx->ev[9], WS(ctx)));
     for (uint32_t v = 0; v < n_views; ++v) ctx->hist[v].spp += req[v].spp;
 
@@ -1686,22 +1726,42 @@ extern "C" bsm_status bsm_render_cached(bsm_context* ctx, uint32_t scene_id, con
     if (bsm_status e = prepare_launch(ctx, sc, *settings)) return e;
     // the frame's device time (stats->ms_total) starts before its training step
     CK(cudaEventRecord(ctx->ev[8], WS(ctx)));
-    if (cs.train_steps > 0 && cs.train_paths > 0) {
+    const bool train = cs.train_steps > 0 && cs.train_paths > 0;
+    const bool bad = !(cs.min_roughness >= 0.0f) || cs.cache_segment + 1 + cs.extra_segments > (uint32_t)kMaxSeg;
+    // The training paths wait for memory on half of the SMs' warps and take as long as the frame's longest stage, so
+    // they run beside the render; only the cache queries at its end need the trained weights. Frames, us, one after
+    // the other / side by side (32,768 paths, 4 steps): 1280x720 of the room 1040 / 822, of 1.48 M triangles
+    // 2000 / 1597, 1920x1080 of these 3329 / 2886, 128x72 838 / 707. (A stream of higher priority: the same within
+    // 2 %.) Timed and counted stages stay one after the other.
+    bool side = train && !bad && !(settings->flags & (BSM_PT_STAGE_TIMING | BSM_PT_COUNT_TRAVERSAL));
+    if (side && !ctx->side && cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        side = false;
+    }
+    cudaStream_t ts = side ? ctx->side : WS(ctx);
+    if (side) CK(cudaStreamWaitEvent(ts, ctx->ev[8], 0));   // after everything queued on the work stream
+    if (train) {
         DevView dv{};
         make_view(*cam, dv);
         dv.ray_length = settings->ray_length;
         dv.t_min = settings->t_min;
         dv.seed = settings->seed;
         dv.max_segments = std::min(std::max(cs.train_segments, 1u), 16u);
-        bsm_status e = cache_train_frame(cache, sc->dev, dv, cs, ctx->lc, WS(ctx), train_loss, nullptr);
+        bsm_status e = cache_train_paths(cache, sc->dev, dv, cs, ctx->lc, ts);
+        if (!e && !side) e = cache_train_steps(cache, cs, ts, train_loss);
         if (e) return fail(ctx, e, "radiance-cache training failed");
     }
     std::vector<ViewReq> req(1);
-    if (!(cs.min_roughness >= 0.0f) || cs.cache_segment + 1 + cs.extra_segments > (uint32_t)kMaxSeg)
+    if (bad)
         return fail(ctx, BSM_ERR_INVALID_ARG, "min_roughness must be >= 0 and cache_segment + extra_segments <= 15");
     req[0] = ViewReq{*cam, settings->spp, cs.cache_segment + 1 + cs.extra_segments, settings->seed};
-    return render_impl(ctx, scene_id, req, *settings, output, stats, cache_render_weights(cache), cs.cache_segment,
-                       cs.extra_segments ? cs.min_roughness : 0.0f, /*start_recorded=*/true);
+    SideTraining tail{cache, cs, train_loss};
+    bsm_status st = render_impl(ctx, scene_id, req, *settings, output, stats, cache_render_weights(cache),
+                                cs.cache_segment, cs.extra_segments ? cs.min_roughness : 0.0f,
+                                /*start_recorded=*/true, side ? &tail : nullptr);
+    if (side && !tail.done)   // a call that the render refuses has trained all the same
+        if (bsm_status e = tail.finish(ctx)) return e;
+    return st;
 }
 
 extern "C" bsm_status bsm_render_batch(bsm_context* ctx, uint32_t scene_id, const bsm_view_desc* views,

@@ -300,8 +300,8 @@ static bsm_status ensure_train_verts(bsm_cache* c, uint32_t paths, uint32_t vert
     return BSM_OK;
 }
 
-bsm_status cache_train_frame(bsm_cache* c, const DevScene& sc, const DevView& view, const bsm_cache_settings& cs,
-                             const LaunchCfg& lc, cudaStream_t st, float* loss_out, uint32_t* samples_out) {
+bsm_status cache_train_paths(bsm_cache* c, const DevScene& sc, const DevView& view, const bsm_cache_settings& cs,
+                             const LaunchCfg& lc, cudaStream_t st) {
     const uint32_t segs = std::max(1u, std::min(cs.train_segments, 16u));
     const uint32_t cap = cs.train_paths * segs;
     if (c->sample_cap < cap) {
@@ -333,13 +333,15 @@ bsm_status cache_train_frame(bsm_cache* c, const DevScene& sc, const DevView& vi
     launch_train_paths(st, sc, c->view_dev, cs.train_paths, c->frame++, tv, q);
     launch_trace(lc, st, sc, q, 0, kNoSegment, 0, c->tv_rad, cap);
     launch_train_targets(st, cs.train_paths, tv, c->samples, c->sample_count, c->sample_cap);
-    if (cudaGetLastError() != cudaSuccess) return BSM_ERR_CUDA;
+    return cudaGetLastError() == cudaSuccess ? BSM_OK : BSM_ERR_CUDA;
+}
+
+bsm_status cache_train_steps(bsm_cache* c, const bsm_cache_settings& cs, cudaStream_t st, float* loss_out) {
     uint32_t n = 0;
     cudaMemcpyAsync(&n, c->sample_count, 4, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return BSM_ERR_CUDA;
     n = std::min(n, c->sample_cap);
     uint32_t use = std::min(n, cs.train_batch * cs.train_steps);
-    if (samples_out) *samples_out = n;
     return train_device(c, c->samples, use, cs.train_batch, cs.lr, st, loss_out, cs.ema_decay);
 }
 }  // namespace bsm

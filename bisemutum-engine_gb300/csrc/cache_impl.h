@@ -49,7 +49,9 @@ struct bsm_cache {
 namespace bsm {
 // The bf16 weights renders read: the corrected moving average once it holds a step, else the current ones.
 inline const void* cache_render_weights(const bsm_cache* c) { return c->ema_steps > 0 ? c->w_ema_bf16 : c->w_bf16; }
-// Runs train paths + Adam steps for one camera (cache.cpp).
-bsm_status cache_train_frame(bsm_cache* c, const DevScene& sc, const DevView& view, const bsm_cache_settings& cs,
-                             const LaunchCfg& lc, cudaStream_t st, float* loss_out, uint32_t* samples_out);
+// A frame's training (cache.cpp): the first call queues the training paths of a camera on `st`, the second waits for
+// them and runs the Adam steps; when it returns, `st` is idle.
+bsm_status cache_train_paths(bsm_cache* c, const DevScene& sc, const DevView& view, const bsm_cache_settings& cs,
+                             const LaunchCfg& lc, cudaStream_t st);
+bsm_status cache_train_steps(bsm_cache* c, const bsm_cache_settings& cs, cudaStream_t st, float* loss_out);
 }
