@@ -635,7 +635,12 @@ struct SmallSet {
 // every lane sums up the boxes left and right of its own bin over its node's
 // references (broadcast by shuffles), for the three axes at once.  The counts,
 // boxes and costs are those of the bins, and the least cost of the first axis
-// and then the lowest bin is taken as k_split takes it.
+// and then the lowest bin is taken as k_split takes it.  Bound by the issue of
+// minima and maxima (half rate), not by warps in flight: centroid bounds and
+// the least cost come from scans over a node's lanes (log2 of its size in steps)
+// instead of loops over its references: 1.48 M / 4.97 M triangles in 4.51 / 12.7
+// ms, with the loops 4.61 / 13.06.  Scans over lanes sorted by bin in place of
+// the remaining loop gain 1 % more for twice the code and were left out.
 __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_t n, uint32_t root_first, uint32_t node,
                                              float area, BNode* __restrict__ nodes, Counters* cnt, int B,
                                              uint32_t max_leaf, uint32_t max_nodes) {
@@ -656,14 +661,13 @@ __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_
         if (most == 0u) break;
         float cen[3], cl[3], ch[3];
         for (int k = 0; k < 3; ++k) { cen[k] = 0.5f * (lo[k] + hi[k]); cl[k] = ch[k] = cen[k]; }
-        for (uint32_t j = 0; j < most; ++j) {
-            const uint32_t src = open && j < sc ? s0 + j : lane;
+        const int last = (int)(s0 + sc - 1u);   // of this lane's node
+        for (uint32_t o = 1; o < most; o <<= 1)
             for (int k = 0; k < 3; ++k) {
-                const float c = __shfl_sync(kFull, cen[k], (int)src);
-                cl[k] = fminf(cl[k], c);
-                ch[k] = fmaxf(ch[k], c);
+                const float l = __shfl_up_sync(kFull, cl[k], o), h = __shfl_up_sync(kFull, ch[k], o);
+                if (lane >= s0 + o) { cl[k] = fminf(cl[k], l); ch[k] = fmaxf(ch[k], h); }
             }
-        }
+        for (int k = 0; k < 3; ++k) { cl[k] = __shfl_sync(kFull, cl[k], last); ch[k] = __shfl_sync(kFull, ch[k], last); }
         uint32_t bins = 0;       // this lane's bin per axis, 8 bits each
         bool use[3];
         for (int k = 0; k < 3; ++k) {
@@ -701,12 +705,13 @@ __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_
             const float c = area6(L[a], L[a] + 3) * (float)nl[a] + area6(R[a], R[a] + 3) * (float)(sc - nl[a]);
             if (c < best) { best = c; key = ((uint32_t)a << 16) | (((bins >> (8 * a)) & 255u) << 8) | lane; }
         }
-        for (uint32_t j = 0; j < most; ++j) {
-            const uint32_t src = open && j < sc ? s0 + j : lane;
-            const float ob = __shfl_sync(kFull, best, (int)src);
-            const uint32_t ok = __shfl_sync(kFull, key, (int)src);
-            if (ob < best || (ob == best && ok < key)) { best = ob; key = ok; }
+        for (uint32_t o = 1; o < most; o <<= 1) {
+            const float ob = __shfl_up_sync(kFull, best, o);
+            const uint32_t ok = __shfl_up_sync(kFull, key, o);
+            if (lane >= s0 + o && (ob < best || (ob == best && ok < key))) { best = ob; key = ok; }
         }
+        best = __shfl_sync(kFull, best, last);
+        key = __shfl_sync(kFull, key, last);
         const bool split_axis = key != kNone;
         const int axis = split_axis ? (int)(key >> 16) : -1;
         const Split sp = decide(axis, 0, 0u, best, sc, area, max_leaf);
@@ -785,7 +790,8 @@ __device__ __forceinline__ void finish_lanes(SmallSet& S, uint32_t base, uint32_
 // stack (every entry holds two or more references of a disjoint range, so at
 // most kSmall / 2 entries are live).  Splitting every node on its own, with
 // bins and three scans for two references as for a hundred, took 3.38 ms of the
-// 1.48 M-triangle terrain's build; 1.18 ms now (predicated instead of branching sums: 1.39).
+// 1.48 M-triangle terrain's build; 1.09 ms now (predicated instead of branching sums: 1.39;
+// nodes of up to 64 / 96 references here and larger ones in the level passes: builds 4.64 / 4.60 ms against 4.51).
 __global__ void __launch_bounds__(kSmallWarps * 32, 5) k_small(const Task* __restrict__ small, uint32_t nsmall,
                                                             const uint32_t* __restrict__ refs0,
                                                             const uint32_t* __restrict__ refs1,
