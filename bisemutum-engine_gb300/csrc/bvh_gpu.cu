@@ -85,7 +85,7 @@ struct Split { int axis; int bin; uint32_t leaf; uint32_t nl; };
 struct ChunkBins { uint16_t below[3][kBins]; };   // a chunk's references in the bins below each, per axis
 struct ChildAcc { uint32_t box[2][6]; uint32_t cen[2][6]; };   // per side: lo xyz, hi xyz (keys)
 struct WideLevel { uint32_t nodes, node_base, tri_base, pad; };   // a level's 8-wide nodes, its first node and triangle
-struct Counters { uint32_t nodes, tasks[2], chunks, small_tasks, error, depth, pad; WideLevel wide[2]; };
+struct Counters { uint32_t nodes, tasks[2], chunks[2], small_tasks, error, depth; WideLevel wide[2]; uint32_t wide_blocks, pad[3]; };
 struct WideRec { uint32_t child[8]; };     // binary node per slot (kNone: empty slot)
 
 // Order-preserving map of floats to unsigned keys (-0 below +0), so that
@@ -194,38 +194,6 @@ __global__ void k_bins_init(Bin* bins, uint32_t n, ChildAcc* acc, uint32_t nacc)
     }
 }
 
-// First chunk of every task (one block: a scan over the tasks) and the task of every chunk.
-__global__ void __launch_bounds__(1024) k_level_chunks(Task* __restrict__ tasks, uint32_t* __restrict__ chunk_task,
-                                                       uint32_t chunk_cap, uint32_t chunk, Counters* cnt, int cur) {
-    __shared__ uint32_t s_w[32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nt = cnt->error ? 0u : cnt->tasks[cur];
-    uint32_t carry = 0;
-    __syncthreads();   // every thread has read the counters that thread 0 writes below
-    for (uint32_t base = 0; base < nt; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t n = i < nt ? (tasks[i].end - tasks[i].begin + chunk - 1u) / chunk : 0u;
-        uint32_t x = n;
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31u) s_w[warp] = x;
-        __syncthreads();
-        uint32_t before = 0, all = 0;
-        for (uint32_t w = 0; w < 32; ++w) { const uint32_t v = s_w[w]; before += w < warp ? v : 0u; all += v; }
-        __syncthreads();
-        const uint32_t first = carry + before + x - n;
-        if (i < nt) {
-            tasks[i].aux = first;
-            if (first + n > chunk_cap) atomicOr(&cnt->error, kErrNodes);
-            else
-                for (uint32_t c = 0; c < n; ++c) chunk_task[first + c] = i;
-        }
-        carry += all;
-    }
-    if (threadIdx.x == 0) { cnt->chunks = min(carry, chunk_cap); cnt->tasks[cur ^ 1] = 0u; }
-}
-
 // Adds a warp's references to one axis' shared bins.  Neighbouring references
 // mostly share a bin (they are in input order within a node), and 32 atomics on
 // one address take turns, so up to three groups of eight or more lanes with a
@@ -264,9 +232,9 @@ __global__ void __launch_bounds__(kLevelThreads) k_bin(const uint32_t* __restric
                                                        const Task* __restrict__ tasks,
                                                        const uint32_t* __restrict__ refs,
                                                        const float4* __restrict__ box, Bin* __restrict__ gbins,
-                                                       ChunkBins* __restrict__ cbins, const Counters* cnt, uint32_t chunk, int B) {
+                                                       ChunkBins* __restrict__ cbins, const Counters* cnt, int cur, uint32_t chunk, int B) {
     __shared__ Bin sb[3 * kBins];
-    const uint32_t nch = cnt->error ? 0u : cnt->chunks;
+    const uint32_t nch = cnt->error ? 0u : cnt->chunks[cur];
     for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
         for (int i = threadIdx.x; i < 3 * kBins; i += blockDim.x) {
             sb[i].cnt = 0;
@@ -413,6 +381,7 @@ __global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins,
                         const BNode* __restrict__ nodes, Split* __restrict__ splits, uint32_t* __restrict__ left_base,
                         ChildAcc* __restrict__ acc, Counters* cnt, int cur, uint32_t chunk, int B, uint32_t max_leaf) {
     const int lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->tasks[cur ^ 1] = cnt->chunks[cur ^ 1] = 0u;   // the last level's
     const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur], warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nt; w += warps) {
         const Task tk = tasks[w];
@@ -482,13 +451,13 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
                                                              const uint32_t* __restrict__ in,
                                                              uint32_t* __restrict__ out,
                                                              const float4* __restrict__ box,
-                                                             ChildAcc* __restrict__ acc, const Counters* cnt, uint32_t chunk, int B) {
+                                                             ChildAcc* __restrict__ acc, const Counters* cnt, int cur, uint32_t chunk, int B) {
     constexpr int kWarps = kLevelThreads / 32;
     __shared__ uint32_t s_wl[2][kWarps], s_wr[2][kWarps];
     __shared__ float s_red[kWarps][12];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t nch = cnt->error ? 0u : cnt->chunks;   // after an error the offsets may be wrong
+    const uint32_t nch = cnt->error ? 0u : cnt->chunks[cur];   // after an error the offsets may be wrong
     for (uint32_t c = blockIdx.x; c < nch; c += gridDim.x) {
         const uint32_t ti = chunk_task[c];
         const Task tk = tasks[ti];
@@ -558,12 +527,16 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
 
 // Children of every split task: two binary nodes each; a child of one triangle
 // is a leaf, a child of at most kSmall goes to the small list with the buffer
-// that holds its references, any other to the next level.
+// that holds its references, any other to the next level, with its chunks.
+// Chunks are handed out by a counter, in any order of tasks: nothing depends on
+// it, and a scan over the tasks was a launch of its own (builds of 20 k / 1.48 M
+// triangles 1.06 / 4.52 -> 1.035 / 4.46 ms without it).
 __global__ void k_make_children(const Task* __restrict__ tasks, const Split* __restrict__ splits,
                                 ChildAcc* __restrict__ acc, const uint32_t* __restrict__ refs,
                                 BNode* __restrict__ nodes, uint32_t* __restrict__ final_refs, Task* __restrict__ next,
-                                uint32_t next_cap, Task* __restrict__ small, uint32_t small_cap, Counters* cnt, int cur,
-                                uint32_t max_nodes) {
+                                uint32_t next_cap, Task* __restrict__ small, uint32_t small_cap,
+                                uint32_t* __restrict__ chunk_task, uint32_t chunk_cap, uint32_t chunk, Counters* cnt,
+                                int cur, uint32_t max_nodes) {
     const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         const Task tk = tasks[i];
@@ -607,7 +580,14 @@ __global__ void k_make_children(const Task* __restrict__ tasks, const Split* __r
                 if (slot < small_cap) small[slot] = c; else atomicOr(&cnt->error, kErrNodes);
             } else {
                 const uint32_t slot = atomicAdd(&cnt->tasks[cur ^ 1], 1u);
-                if (slot < next_cap) next[slot] = c; else atomicOr(&cnt->error, kErrNodes);
+                const uint32_t nc = (n.count + chunk - 1u) / chunk;
+                c.aux = atomicAdd(&cnt->chunks[cur ^ 1], nc);
+                if (slot < next_cap && c.aux + nc <= chunk_cap) {
+                    next[slot] = c;
+                    for (uint32_t k = 0; k < nc; ++k) chunk_task[c.aux + k] = slot;
+                } else {
+                    atomicOr(&cnt->error, kErrNodes);
+                }
             }
         }
         acc[i] = z;   // for the next level's task
@@ -1079,6 +1059,49 @@ constexpr uint32_t kWideThreads = 256;
 constexpr uint32_t kWideTile = kWideThreads / kWideLanes;   // nodes per block and round
 static_assert(kWideTile == 32, "one warp scans a tile's nodes");
 
+// First child and triangle of every tile within the level, and the next level, by the last block of k_wide_nodes
+// (a launch of its own per level cost builds of 20 k / 1.48 M triangles 0.02 ms).
+__device__ __forceinline__ void wide_scan(uint2* sums, const WideLevel& lv, uint32_t wnode_cap, uint32_t num_tris,
+                                          Counters* cnt, int cur) {
+    __shared__ uint2 s_w[kWideThreads / 32];
+    const uint32_t n = __syncthreads_or(__ldcg(&cnt->error) != 0u) ? 0u : (lv.nodes + kWideTile - 1u) / kWideTile;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint2 carry = make_uint2(0u, 0u);
+    for (uint32_t base = 0; base < n; base += kWideThreads) {
+        const uint32_t i = base + threadIdx.x;
+        const uint2 v = i < n ? __ldcg(sums + i) : make_uint2(0u, 0u);
+        uint2 x = v;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t yx = __shfl_up_sync(0xffffffffu, x.x, o), yy = __shfl_up_sync(0xffffffffu, x.y, o);
+            if (lane >= o) { x.x += yx; x.y += yy; }
+        }
+        if (lane == 31u) s_w[warp] = x;
+        __syncthreads();
+        uint2 before = make_uint2(0u, 0u), all = before;
+        for (uint32_t k = 0; k < kWideThreads / 32; ++k) {
+            const uint2 t = s_w[k];
+            if (k < warp) { before.x += t.x; before.y += t.y; }
+            all.x += t.x;
+            all.y += t.y;
+        }
+        __syncthreads();
+        if (i < n) sums[i] = make_uint2(carry.x + before.x + x.x - v.x, carry.y + before.y + x.y - v.y);
+        carry.x += all.x;
+        carry.y += all.y;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        WideLevel next{carry.x, lv.node_base + lv.nodes, lv.tri_base + carry.y, 0u};
+        if (n == 0u) next = WideLevel{0u, lv.node_base, lv.tri_base, 0u};
+        else cnt->depth += 1u;
+        if ((uint64_t)next.node_base + next.nodes > wnode_cap || next.tri_base > num_tris) {
+            atomicOr(&cnt->error, kErrWide);
+            next.nodes = 0u;
+        }
+        cnt->wide[cur ^ 1] = next;
+    }
+}
+
 // The nodes of a level: each gathers its up to eight children, assigns octant
 // slots and quantises their boxes, a child per lane, with its first child and
 // triangle counted from the start of its tile.  (A thread per node took 0.50 ms
@@ -1088,7 +1111,7 @@ static_assert(kWideTile == 32, "one warp scans a tile's nodes");
 __global__ void __launch_bounds__(kWideThreads) k_wide_nodes(const uint32_t* __restrict__ queue, WideCfg w,
                                                              WideRec* __restrict__ rec, uint2* __restrict__ tile_sums,
                                                              CwNode* __restrict__ wnodes, uint32_t wnode_cap,
-                                                             Counters* cnt, int cur) {
+                                                             uint32_t num_tris, Counters* cnt, int cur) {
     __shared__ uint2 s_entry[kWideTile][kWideLanes];
     __shared__ uint32_t s_child[kWideTile][kWideLanes];
     __shared__ uint4 s_image[kWideTile][sizeof(CwNode) / 16];
@@ -1251,49 +1274,18 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_nodes(const uint32_t* __r
         }
         __syncthreads();
     }
-}
-
-// First child and triangle of every tile within the level (one block), and the next level.
-__global__ void __launch_bounds__(1024) k_wide_scan(uint2* __restrict__ sums, uint32_t wnode_cap, uint32_t num_tris,
-                                                    Counters* cnt, int cur) {
-    __shared__ uint2 s_w[32];
-    const WideLevel lv = cnt->wide[cur];
-    const uint32_t n = cnt->error ? 0u : (lv.nodes + kWideTile - 1u) / kWideTile;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint2 carry = make_uint2(0u, 0u);
-    for (uint32_t base = 0; base < n; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const uint2 v = i < n ? sums[i] : make_uint2(0u, 0u);
-        uint2 x = v;
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-            const uint32_t yx = __shfl_up_sync(0xffffffffu, x.x, o), yy = __shfl_up_sync(0xffffffffu, x.y, o);
-            if (lane >= o) { x.x += yx; x.y += yy; }
-        }
-        if (lane == 31u) s_w[warp] = x;
-        __syncthreads();
-        uint2 before = make_uint2(0u, 0u), all = before;
-        for (uint32_t k = 0; k < 32; ++k) {
-            const uint2 t = s_w[k];
-            if (k < warp) { before.x += t.x; before.y += t.y; }
-            all.x += t.x;
-            all.y += t.y;
-        }
-        __syncthreads();
-        if (i < n) sums[i] = make_uint2(carry.x + before.x + x.x - v.x, carry.y + before.y + x.y - v.y);
-        carry.x += all.x;
-        carry.y += all.y;
-    }
+    // the block that ends last scans the tiles
+    __shared__ bool s_last;
+    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        WideLevel next{carry.x, lv.node_base + lv.nodes, lv.tri_base + carry.y, 0u};
-        if (n == 0u) next = WideLevel{0u, lv.node_base, lv.tri_base, 0u};
-        else cnt->depth += 1u;
-        if ((uint64_t)next.node_base + next.nodes > wnode_cap || next.tri_base > num_tris) {
-            atomicOr(&cnt->error, kErrWide);
-            next.nodes = 0u;
-        }
-        cnt->wide[cur ^ 1] = next;
+        s_last = atomicAdd(&cnt->wide_blocks, 1u) == gridDim.x - 1u;
+        if (s_last) cnt->wide_blocks = 0u;
     }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    wide_scan(tile_sums, lv, wnode_cap, num_tris, cnt, cur);
 }
 
 struct TriSrc {
@@ -1544,7 +1536,9 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
             DB_CK(cudaMemcpyAsync(&cnt->tasks[0], &one, 4, cudaMemcpyHostToDevice, st));
             k_bins_init<<<blocks_for((uint64_t)L.task_cap * 3 * kBins, 256), 256, 0, st>>>(bins, L.task_cap * 3 * kBins, acc,
                                                                                           L.task_cap);
-            const uint32_t chunk = chunk_size(T);
+            const uint32_t chunk = chunk_size(T), root_chunks = (T + chunk - 1u) / chunk;
+            DB_CK(cudaMemcpyAsync(&cnt->chunks[0], &root_chunks, 4, cudaMemcpyHostToDevice, st));
+            DB_CK(cudaMemsetAsync(chunk_task, 0, (size_t)root_chunks * 4, st));
             uint32_t batch = 4;
             while ((uint64_t)kSmall << (batch - 4) < T) ++batch;
             uint32_t ntasks = 1;
@@ -1555,16 +1549,15 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
                     const uint32_t max_tasks = level < 31u ? std::min(1u << level, L.task_cap) : L.task_cap;
                     const uint32_t max_chunks = std::min(T / chunk + max_tasks + 1u, L.chunk_cap);
                     const uint32_t grid = std::min(max_chunks, (uint32_t)sms * 8u);
-                    k_level_chunks<<<1, 1024, 0, st>>>(tasks[cur], chunk_task, L.chunk_cap, chunk, cnt, cur);
-                    k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, chunk,
+                    k_bin<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], refs[cur], box, bins, chunk_bins, cnt, cur, chunk,
                                                           B);
                     k_split<<<std::min(blocks_for((uint64_t)max_tasks * 32, 128), (uint32_t)sms * 8u), 128, 0, st>>>(
                         tasks[cur], bins, chunk_bins, bnodes, splits, left_base, acc, cnt, cur, chunk, B, bin_leaf);
                     k_partition<<<grid, kLevelThreads, 0, st>>>(chunk_task, tasks[cur], splits, left_base, refs[cur],
-                                                                refs[cur ^ 1], box, acc, cnt, chunk, B);
+                                                                refs[cur ^ 1], box, acc, cnt, cur, chunk, B);
                     k_make_children<<<std::min(blocks_for(max_tasks, 64), (uint32_t)sms * 4u), 64, 0, st>>>(
                         tasks[cur], splits, acc, refs[cur ^ 1], bnodes, final_refs, tasks[cur ^ 1], L.task_cap, small,
-                        L.small_cap, cnt, cur, L.max_nodes);
+                        L.small_cap, chunk_task, L.chunk_cap, chunk, cnt, cur, L.max_nodes);
                 }
                 DB_CK(cudaGetLastError());
                 DB_CK(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
@@ -1620,8 +1613,7 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
                 const uint32_t max_nodes = wide_level < 10u ? std::min(1u << (3 * wide_level), L.wnode_cap) : L.wnode_cap;
                 const uint32_t grid = std::min(blocks_for(max_nodes, kWideTile), (uint32_t)sms * 8u);
                 k_wide_nodes<<<grid, kWideThreads, 0, st>>>(queue[cur], wc, (WideRec*)P(L.rec), (uint2*)P(L.tile_sums),
-                                                            (CwNode*)P(L.wnodes), L.wnode_cap, cnt, cur);
-                k_wide_scan<<<1, 1024, 0, st>>>((uint2*)P(L.tile_sums), L.wnode_cap, T, cnt, cur);
+                                                            (CwNode*)P(L.wnodes), L.wnode_cap, T, cnt, cur);
                 k_wide_emit<<<grid, kWideThreads, 0, st>>>((const WideRec*)P(L.rec), (const uint2*)P(L.tile_sums), wc, ts,
                                                            (CwNode*)P(L.wnodes), wtris, T, queue[cur ^ 1], cnt, cur);
             }
