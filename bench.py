@@ -322,7 +322,8 @@ def run_ours(a, dist: Dist):
         ms_cam += st.ms_camera
         rays += st.extend_rays
         shadow_rays += st.shadow_rays
-        launches += st.chunks * (1 + 3 * a.segments)
+        # a camera launch, three per segment, and one for the first hits' light rays of chunks of over 3 M paths
+        launches += st.chunks * (1 + 3 * a.segments + (1 if st.paths > 3000000 * st.chunks else 0))
         ext_launches = st.extend_launches
         seg_rays = [int(st.rays_per_segment[k]) for k in range(a.segments)]
     ctx.sync()

@@ -331,7 +331,7 @@ bsm_status cache_train_paths(bsm_cache* c, const DevScene& sc, const DevView& vi
     cudaMemsetAsync(c->sample_count, 0, 4, st);
     cudaMemsetAsync(q.counters, 0, kCntWords * 4, st);
     launch_train_paths(st, sc, c->view_dev, cs.train_paths, c->frame++, tv, q);
-    launch_trace(lc, st, sc, q, 0, kNoSegment, 0, c->tv_rad, cap);
+    launch_trace(lc, st, sc, q, 0, kNoSegment, 0, c->tv_rad, cap, false);
     launch_train_targets(st, cs.train_paths, tv, c->samples, c->sample_count, c->sample_cap);
     return cudaGetLastError() == cudaSuccess ? BSM_OK : BSM_ERR_CUDA;
 }

@@ -89,7 +89,8 @@ enum : uint32_t {
     kCntWork = kCntShadow + 16,    // [2 * kMaxSeg] persistent-kernel work counters
     kCntSky = kCntWork + 32,       // [kMaxSeg] sky shadow rays of segment s (queue back)
     kCntCache = kCntSky + 16,      // radiance-cache queries of the chunk
-    kCntError = kCntCache + 1,     // error flags (bit 0: queue overflow, bit 1: a tensor-core wait timed out);
+    kCntZero = kCntCache + 1,      // nothing counts here: the size of a queue that a launch leaves out
+    kCntError = kCntZero + 1,      // error flags (bit 0: queue overflow, bit 1: a tensor-core wait timed out);
                                    // words below it are cleared per chunk
     kCntWords = kCntError + 1
 };
@@ -152,9 +153,10 @@ void launch_camera(const LaunchCfg& lc, cudaStream_t st, const DevView* views, u
                    uint64_t path_begin, uint32_t path_count, const Wavefront& wf, uint32_t max_segments);
 // The extension rays of segment `ext` (queue q) and the shadow rays of segment `shd` in one launch; kNoSegment
 // leaves one kind out.  The two kinds are independent of each other: shading segment s queues both shd = s and
-// ext = s + 1.  `paths` (the chunk's paths) bounds both queues and picks the kernel.
+// ext = s + 1.  `paths` (the chunk's paths) bounds both queues and picks the kernel; `first`: the shadow rays of
+// segment 0 are those of camera rays' hits, in the order of the pixels.
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
-                  uint32_t shd, float4* accum, uint32_t paths);
+                  uint32_t shd, float4* accum, uint32_t paths, bool first = true);
 // The extension rays of `seg` with the traversal counters of BSM_PT_COUNT_TRAVERSAL.
 void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q,
                          uint32_t seg);

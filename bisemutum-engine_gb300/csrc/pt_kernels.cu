@@ -217,6 +217,7 @@ struct TraceArgs {
     uint32_t* counters;
     unsigned long long* stats;
     uint32_t ext, shd, sh_last;   // segments (kNoSegment: none); the shadow queue's last slot
+    uint32_t ext_cnt, sun_cnt, sky_cnt;   // the queues' sizes in `counters` (kCntZero: left out)
     uint32_t min_rays, max_rays;  // the kernel leaves queues of other lengths alone
     int postpone_sp, refill_min;
 };
@@ -251,12 +252,7 @@ struct TraceRays {
 };
 // The launch's queue sizes from the device counters; the first thread adds them to the statistics.
 __device__ __forceinline__ TraceRays trace_rays(const TraceArgs& a) {
-    const uint32_t n_ext = a.ext < kNoSegment ? a.counters[kCntQueue + a.ext] : 0u;
-    uint32_t n_sun = 0, n_sky = 0;
-    if (a.shd < kNoSegment) {
-        n_sun = a.counters[kCntShadow + a.shd];
-        n_sky = a.counters[kCntSky + a.shd];
-    }
+    const uint32_t n_ext = a.counters[a.ext_cnt], n_sun = a.counters[a.sun_cnt], n_sky = a.counters[a.sky_cnt];
     const uint32_t n = n_ext + n_sun + n_sky;
     if (n < a.min_rays || n > a.max_rays) return TraceRays{a, 0u, 0u, 0u};
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -296,6 +292,27 @@ __global__ void __launch_bounds__(128, 8) k_trace_first(const CwNode* __restrict
     const uint32_t leaf =
         trace_ray<false, false>(make_ray(o, d), d.w, nodes, tris, t, u, v, nullptr, kOpacity ? rays.seed(i) : 0u);
     rays.hit(i, leaf, t, u, v, kMissPrim);
+}
+
+// The shadow rays of the camera rays' hits towards the lights, in the same way:
+// those of one pixel's samples or of a tile start next to one another and head
+// the same way.  In k_trace's queue behind the extension rays the warps reach
+// them with rays at every stage of their walks and never hold a pixel's 32 rays
+// together; a launch of its own keeps them so (k_trace alone for them already
+// gains from 16 spp on).
+template <bool kOpacity>
+__global__ void __launch_bounds__(128, 8) k_trace_sun(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
+                                                      const __grid_constant__ TraceArgs a) {
+    const TraceRays rays = trace_rays(a);
+    for (uint64_t k = blockIdx.x * blockDim.x + threadIdx.x; k < rays.n; k += gridDim.x * blockDim.x) {
+        const uint32_t i = (uint32_t)k;
+        float4 o, d;
+        rays.load(i, o, d);
+        float t, u, v;
+        if (trace_ray<true, false>(make_ray(o, d), d.w, nodes, tris, t, u, v, nullptr,
+                                   kOpacity ? rays.seed(i) : 0u) == kMissPrim)
+            rays.miss(i, d.w);
+    }
 }
 
 // k_trace for small chunks and short queues: eight lanes per ray.  A
@@ -1000,11 +1017,17 @@ constexpr uint32_t kGroupPaths = 40960, kGroupPaths2 = 98304, kMixedPaths = 1000
 // 90,000 are level, 120,000 is slower (641x359 1240 / 1238 / 1311 us).
 constexpr uint32_t kGroupQueue = 56000, kGroupQueue2 = 90000;
 
+// Chunks of more paths than this trace the first hits' rays to the lights in a launch of their own. Frames of 8
+// segments, us, in one queue / on their own: 1920x1080 of 1.48 M triangles 64 spp 158500 / 155000, 4 spp 11502 /
+// 11361, 1 spp 3616 / 3634; 1280x720x4 5553 / 5520 (250 k triangles 4005 / 3952), 1024^2 2636 / 2685.
+constexpr uint32_t kFirstShadowPaths = 3000000;
+
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
-                  uint32_t shd, float4* accum, uint32_t paths) {
+                  uint32_t shd, float4* accum, uint32_t paths, bool first) {
     TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
-                wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u, 0u, 0xffffffffu,
-                lc.postpone_sp, lc.refill_min};
+                wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u,
+                ext < kNoSegment ? kCntQueue + ext : kCntZero, shd < kNoSegment ? kCntShadow + shd : kCntZero,
+                shd < kNoSegment ? kCntSky + shd : kCntZero, 0u, 0xffffffffu, lc.postpone_sp, lc.refill_min};
     const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr;
     const bool only = paths <= (two ? kGroupPaths2 : kGroupPaths), mix = !only && paths <= kMixedPaths && ext != 0u;
     if (!only && !two && ext == 0u && shd == kNoSegment) {
@@ -1012,6 +1035,14 @@ void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, cons
         if (op) k_trace_first<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
         else k_trace_first<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
         return;
+    }
+    if (first && shd == 0u && !two && paths > kFirstShadowPaths && sc.num_lights != 0u) {
+        TraceArgs b = a;
+        b.ext_cnt = b.sky_cnt = kCntZero;
+        const uint32_t grid = (uint32_t)(((uint64_t)paths + 127u) / 128u);   // one light's rays; the loop takes others'
+        if (op) k_trace_sun<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, b);
+        else k_trace_sun<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, b);
+        a.sun_cnt = kCntZero;
     }
     const uint32_t limit = two ? kGroupQueue2 : kGroupQueue;
     if (only || mix) {
