@@ -391,7 +391,7 @@ def run_ours(a, dist: Dist):
             # per launch: segment 0's rays at the primary launch's bytes per ray, the others at the bounce figure
             b0, b1 = prof["dram_bytes_per_ray_primary"], prof["dram_bytes_per_ray_bounce"]
             traffic = round((b0 * seg_rays[0] + b1 * sum(seg_rays[1:])) / max(1, ext_launches))
-        roofline = {"bound": "hbm", "kernel": "k_extend", "achieved": round(achieved, 2) if achieved else None,
+        roofline = {"bound": "hbm", "kernel": "k_trace", "achieved": round(achieved, 2) if achieved else None,
                     "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 5) if achieved else None,
                     "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
                     "traffic": traffic,
