@@ -1019,7 +1019,8 @@ constexpr uint32_t kGroupQueue = 56000, kGroupQueue2 = 90000;
 
 // Chunks of more paths than this trace the first hits' rays to the lights in a launch of their own. Frames of 8
 // segments, us, in one queue / on their own: 1920x1080 of 1.48 M triangles 64 spp 158500 / 155000, 4 spp 11502 /
-// 11361, 1 spp 3616 / 3634; 1280x720x4 5553 / 5520 (250 k triangles 4005 / 3952), 1024^2 2636 / 2685.
+// 11361, 1 spp 3616 / 3634; 1280x720x4 5553 / 5520 (250 k triangles 4005 / 3952), 1024^2 2636 / 2685. (First in the
+// common queue instead of a launch: 64 spp 155700, but 1 spp 3641, with the longer extension rays as its tail.)
 constexpr uint32_t kFirstShadowPaths = 3000000;
 
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,

@@ -5,8 +5,8 @@
 // with MIS) and records every vertex k it reaches: the cache's raw inputs, the
 // path throughput there, and the radiance gathered there directly (the sky on
 // escape).  Its next-event shadow rays are not traced in the thread: they go
-// to a shadow queue, which the persistent any-hit kernel traces afterwards in
-// one launch, adding each unoccluded contribution to its vertex.  A thread's
+// to a shadow queue, which the wavefront's traversal kernels trace afterwards
+// in one pass, adding each unoccluded contribution to its vertex.  A thread's
 // serial chain is thus its closest-hit rays only (the shadow pass adds exact
 // fixed-point sums, so a vertex's radiance does not depend on the order of the
 // additions).  The targets kernels then
