@@ -382,7 +382,8 @@ __global__ void k_split(const Task* __restrict__ tasks, Bin* __restrict__ gbins,
                         ChildAcc* __restrict__ acc, Counters* cnt, int cur, uint32_t chunk, int B, uint32_t max_leaf) {
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt->tasks[cur ^ 1] = cnt->chunks[cur ^ 1] = 0u;   // the last level's
-    const uint32_t nt = cnt->error ? 0u : cnt->tasks[cur], warps = gridDim.x * (blockDim.x >> 5);
+    // other warps may set the error word while this one starts: its lanes have to agree on what they read
+    const uint32_t nt = __shfl_sync(0xffffffffu, cnt->error ? 0u : cnt->tasks[cur], 0), warps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nt; w += warps) {
         const Task tk = tasks[w];
         int bbin;
@@ -1322,10 +1323,11 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const WideRec* __res
                                                             const uint2* __restrict__ sums, WideCfg w, TriSrc src,
                                                             CwNode* __restrict__ wnodes, CwTri* __restrict__ wtris,
                                                             uint32_t num_tris, uint32_t* __restrict__ next_queue,
-                                                            Counters* cnt, int cur) {
+                                                            uint32_t queue_cap, Counters* cnt, int cur) {
     const WideLevel lv = cnt->wide[cur];
-    const uint32_t nq = cnt->error ? 0u : lv.nodes;
+    const uint32_t nq = __syncthreads_or(cnt->error != 0u) ? 0u : lv.nodes;   // read once, as in k_wide_nodes
     const uint32_t g = threadIdx.x / kWideLanes, s = threadIdx.x % kWideLanes;
+    const uint32_t node_lanes = 0xffu << (threadIdx.x & 31u & ~(kWideLanes - 1u));   // they agree on q
     for (uint32_t tile = blockIdx.x; tile * kWideTile < nq; tile += gridDim.x) {
         const uint32_t q = tile * kWideTile + g;
         if (q >= nq) continue;   // no barrier below
@@ -1335,13 +1337,17 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_emit(const WideRec* __res
         uint4 h = p[1];
         const uint32_t child = rec[q].child[s], tm = h.z & 0xffffu;
         const uint32_t first = sum.x + h.x, tri = lv.tri_base + sum.y + h.y;
-        __syncwarp(__activemask());   // every lane has read the header before it is rewritten
+        __syncwarp(node_lanes);   // every lane of the node has read the header before it is rewritten
         if (s == 0) {
             h.x = lv.node_base + lv.nodes + first;
             h.y = tri;
             p[1] = h;
         }
-        if ((imask >> s) & 1u) next_queue[first + (uint32_t)__popc(imask & ((1u << s) - 1u))] = child;
+        if ((imask >> s) & 1u) {
+            const uint32_t at = first + (uint32_t)__popc(imask & ((1u << s) - 1u));
+            if (at < queue_cap) next_queue[at] = child;
+            else atomicOr(&cnt->error, kErrWide);
+        }
         const uint32_t c = (uint32_t)__popc((tm >> (2u * s)) & 3u);
         if (c != 0u) {   // a leaf's references are consecutive, also those of a collapsed pair
             const uint32_t at = tri + (uint32_t)__popc(tm & ((1u << (2u * s)) - 1u)), ref = w.nodes[child].first;
@@ -1615,7 +1621,8 @@ bool build_cwbvh_device(cudaStream_t st, const float* pos, uint32_t nv, const ui
                 k_wide_nodes<<<grid, kWideThreads, 0, st>>>(queue[cur], wc, (WideRec*)P(L.rec), (uint2*)P(L.tile_sums),
                                                             (CwNode*)P(L.wnodes), L.wnode_cap, T, cnt, cur);
                 k_wide_emit<<<grid, kWideThreads, 0, st>>>((const WideRec*)P(L.rec), (const uint2*)P(L.tile_sums), wc, ts,
-                                                           (CwNode*)P(L.wnodes), wtris, T, queue[cur ^ 1], cnt, cur);
+                                                           (CwNode*)P(L.wnodes), wtris, T, queue[cur ^ 1], L.wnode_cap, cnt,
+                                                           cur);
             }
             DB_CK(cudaGetLastError());
             DB_CK(cudaMemcpyAsync(&hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
