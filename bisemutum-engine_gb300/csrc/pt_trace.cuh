@@ -1144,6 +1144,7 @@ __device__ __forceinline__ void trace_queue2_group(const CwNode* __restrict__ tl
                 break;
             }
         }
+        __syncwarp();   // every lane has taken its entry off the stack before the slot is written again
         if (enter.y != 0u) {
             // the nearest of the hit instances; the others wait below an exit marker
             const uint32_t bit = 31u - (uint32_t)__clz(enter.y);
