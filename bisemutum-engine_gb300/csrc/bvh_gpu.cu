@@ -435,6 +435,18 @@ __device__ __forceinline__ bool goes_left(const Task& tk, const Split& sp, uint3
     return bin_of(centroid(l, h, a), tk.clo[a], axis_scale(tk, a, B), B) < sp.bin;
 }
 
+// Adds the boxes of the lanes `m` (`in`: this lane is one of them) to a shared box of keys, for splits by index. With six
+// atomics per reference on the task's own box, 1,500,000 triangles through one point took 26.6 ms to build; 4.4 ms so.
+__device__ __forceinline__ void add_boxes(uint32_t* s_box, bool in, uint32_t m, const float4& l, const float4& h) {
+    if (!in) return;
+    const bool first = (threadIdx.x & 31u) == (uint32_t)__ffs(m) - 1u;
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t lo = __reduce_min_sync(m, fkey(k == 0 ? l.x : k == 1 ? l.y : l.z));
+        const uint32_t hi = __reduce_max_sync(m, fkey(k == 0 ? h.x : k == 1 ? h.y : h.z));
+        if (first) { atomicMin(s_box + k, lo); atomicMax(s_box + 3 + k, hi); }
+    }
+}
+
 // Stable partition of a chunk: its left references from left_base on, its right
 // ones behind the task's left part (both in chunk order); the children's
 // centroid bounds are reduced over the block and merged into the task's.  Their
@@ -456,6 +468,7 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
     constexpr int kWarps = kLevelThreads / 32;
     __shared__ uint32_t s_wl[2][kWarps], s_wr[2][kWarps];
     __shared__ float s_red[kWarps][12];
+    __shared__ uint32_t s_box[12];   // split by index: the boxes of the two sides as keys
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t nch = cnt->error ? 0u : cnt->chunks[cur];   // after an error the offsets may be wrong
@@ -470,6 +483,11 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
         uint32_t r = 0, i = begin + threadIdx.x;
         float4 l = make_float4(0, 0, 0, 0), h = l;
         if (i < end) { r = in[i]; l = box[2 * (size_t)r]; h = box[2 * (size_t)r + 1]; }
+        const bool by_index = sp.axis < 0;   // no bins (the same for the whole block)
+        if (by_index) {
+            if (threadIdx.x < 12) s_box[threadIdx.x] = threadIdx.x % 6 < 3 ? kKeyLo : kKeyHi;
+            __syncthreads();
+        }
         int par = 0;
         for (uint32_t base = begin; base < end; base += kLevelThreads, i += kLevelThreads, par ^= 1) {
             const bool act = i < end;
@@ -481,13 +499,11 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
             const uint32_t r_now = r;
             const float4 l_now = l, h_now = h;
             if (i + kLevelThreads < end) { r = in[i + kLevelThreads]; l = box[2 * (size_t)r]; h = box[2 * (size_t)r + 1]; }
+            if (by_index) {
+                add_boxes(s_box, left, wl, l_now, h_now);
+                add_boxes(s_box + 6, right, wr, l_now, h_now);
+            }
             if (act) {
-                if (sp.axis < 0)   // no bins: one centroid for all of them
-                    for (int k = 0; k < 3; ++k) {
-                        uint32_t* b = acc[ti].box[left ? 0 : 1];
-                        atomicMin(b + k, fkey(k == 0 ? l_now.x : k == 1 ? l_now.y : l_now.z));
-                        atomicMax(b + 3 + k, fkey(k == 0 ? h_now.x : k == 1 ? h_now.y : h_now.z));
-                    }
                 for (int k = 0; k < 3; ++k) {
                     const float cc = centroid(l_now, h_now, k);
                     if (left) { v[k] = fminf(v[k], cc); v[3 + k] = fmaxf(v[3 + k], cc); }
@@ -512,6 +528,10 @@ __global__ void __launch_bounds__(kLevelThreads, 5) k_partition(const uint32_t* 
             if (lane == 0) s_red[warp][k] = funkey(m);
         }
         __syncthreads();
+        if (by_index && threadIdx.x < 12) {   // (an empty side's keys change nothing)
+            uint32_t* dst = &acc[ti].box[threadIdx.x / 6][threadIdx.x % 6];
+            if (threadIdx.x % 6 < 3) atomicMin(dst, s_box[threadIdx.x]); else atomicMax(dst, s_box[threadIdx.x]);
+        }
         if (threadIdx.x < 12) {
             const int k = threadIdx.x;
             const bool mx = (k % 6) >= 3;
