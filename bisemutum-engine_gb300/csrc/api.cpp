@@ -317,7 +317,8 @@ uint32_t default_capacity(const bsm_context* ctx, uint64_t total_paths, uint32_t
 
 bsm_status ensure_wavefront(bsm_context* ctx, uint32_t capacity, uint32_t lights) {
     if (ctx->wf.capacity >= capacity && ctx->wf_lights >= lights && ctx->wf_buf.ptr) return BSM_OK;
-    // queue slots are 32-bit: the shadow queue holds (lights + 1) records per path
+    // queue slots are 32-bit: the shadow queue holds (lights + 1) records per path (launch_trace traces extension and
+    // shadow rays apart where both together would not count in 32 bits)
     if ((uint64_t)capacity * (lights + 1) >= (1ull << 32))
         return fail(ctx, BSM_ERR_INVALID_ARG, "wavefront_capacity x (lights + 1) must stay below 2^32");
     size_t C = capacity;

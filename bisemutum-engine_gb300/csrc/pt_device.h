@@ -36,6 +36,13 @@ enum : uint32_t { kLightDir = 0, kLightPoint = 1, kLightRect = 2 };
 struct DevLight { float4 a, b, c, d; };
 constexpr int kMaxSeg = 16;
 constexpr uint32_t kNoSegment = kMaxSeg;   // launch_trace: no rays of that kind
+// Rays of one traversal launch, at most. Queue indices and the work counter are 32 bits, and the counter runs past the
+// queue's end by up to a warp's lanes for every warp of the launch (0.4 M on this GPU).
+constexpr uint64_t kMaxTraceRays = (1ull << 32) - (1u << 20);
+// Whether the extension rays of a chunk of `paths` and its shadow rays, up to `lights` + 1 a path, count as one queue.
+constexpr bool one_trace_launch(uint32_t paths, uint32_t lights) {
+    return (uint64_t)paths * ((uint64_t)lights + 2u) <= kMaxTraceRays;
+}
 
 struct DevSky {
     uint32_t kind;             // BSM_SKY_CONSTANT / BSM_SKY_EQUIRECT

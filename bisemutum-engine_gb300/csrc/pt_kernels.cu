@@ -1025,6 +1025,11 @@ constexpr uint32_t kFirstShadowPaths = 3000000;
 
 void launch_trace(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const Wavefront& wf, int q, uint32_t ext,
                   uint32_t shd, float4* accum, uint32_t paths, bool first) {
+    if (ext < kNoSegment && shd < kNoSegment && !one_trace_launch(paths, sc.num_lights)) {
+        launch_trace(lc, st, sc, wf, q, kNoSegment, shd, accum, paths, first);
+        launch_trace(lc, st, sc, wf, q, ext, kNoSegment, accum, paths, first);
+        return;
+    }
     TraceArgs a{wf.ray_o[q], wf.ray_d[q], wf.path[q], wf.hit, wf.sh_o, wf.sh_d, wf.sh_c, wf.sh_seed, accum,
                 wf.accum_fx, wf.counters, wf.stats, ext, shd, wf.capacity * (sc.num_lights + 1u) - 1u,
                 ext < kNoSegment ? kCntQueue + ext : kCntZero, shd < kNoSegment ? kCntShadow + shd : kCntZero,
