@@ -178,7 +178,8 @@ void launch_fold_fixed(cudaStream_t st, const unsigned long long* fx, float4* ac
 // fold into a cleared accumulator followed by launch_resolve)
 void launch_resolve_fixed(cudaStream_t st, const unsigned long long* fx, uint32_t width, uint32_t height,
                           float inv_spp, float4* out, uint32_t pitch_px);
-// Stage entry points; `work`: two device words that are zero, and are zero again when the launch is done.
+// Stage entry points; `work`: two device words that are zero, and are zero again when the launch is done, or null:
+// the launch shares nothing with any other.
 void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
                           uint4* hits, uint32_t* work);
 void launch_trace_any(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,

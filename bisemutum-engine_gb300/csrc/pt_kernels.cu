@@ -644,7 +644,7 @@ struct StageArgs {
     const CwTri* tris;        // for the primitive ids
     const InstDev* insts;
     uint32_t n;
-    uint32_t* work;           // [2], zero between launches
+    uint32_t* work;           // [2], zero between launches; null: the launch takes its rays without a counter
     int postpone_sp, refill_min;
     DevView view;
 };
@@ -688,11 +688,40 @@ struct StageRays {
 
 // The work counter goes back to zero when the launch's last block is done with it.
 __device__ __forceinline__ void stage_done(uint32_t* work) {
+    if (!work) return;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(work + 1, 1u) == gridDim.x - 1u) { work[0] = 0u; work[1] = 0u; }
     }
+}
+// Eight lanes per ray: the first rays of every warp come without a counter, so a grid that holds all of them needs
+// none (the one in shared memory only says that the rays are out).
+__device__ __forceinline__ uint32_t* group_work(const StageArgs& a, uint32_t* s_work) {
+    if (a.work) return a.work;
+    if (threadIdx.x == 0) *s_work = 0u;
+    __syncthreads();
+    return s_work;
+}
+
+// A ray per thread: no queue and no counter.
+template <bool kAny, bool kTwoLevel>
+__global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNode* __restrict__ nodes,
+                                                                      const CwTri* __restrict__ tris,
+                                                                      const InstDev* __restrict__ insts,
+                                                                      const float* __restrict__ mat_tr,
+                                                                      const __grid_constant__ StageArgs a) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    const StageRays rays{a};
+    float4 o, d;
+    rays.load(i, o, d);
+    float t, u, v;
+    uint32_t inst = kMissPrim, leaf;
+    if (kTwoLevel) leaf = trace_ray2<kAny>(make_ray(o, d), d.w, nodes, insts, mat_tr, t, u, v, inst, rays.seed(i));
+    else leaf = trace_ray<kAny, false>(make_ray(o, d), d.w, nodes, tris, t, u, v, nullptr, rays.seed(i));
+    if (leaf == kMissPrim) rays.miss(i, d.w);
+    else rays.hit(i, leaf, t, u, v, inst);
 }
 
 // The caller's rays run on the persistent loops: with a ray per thread to the
@@ -711,7 +740,8 @@ __global__ void __launch_bounds__(kGroupBlock, 6) k_stage_group(const CwNode* __
                                                                 const CwTri* __restrict__ tris,
                                                                 const __grid_constant__ StageArgs a) {
     __shared__ GroupStacks stacks;
-    trace_queue_group<kOpacity>(nodes, tris, a.n, a.work, StageRays{a}, stacks);
+    __shared__ uint32_t s_work;
+    trace_queue_group<kOpacity>(nodes, tris, a.n, group_work(a, &s_work), StageRays{a}, stacks);
     stage_done(a.work);
 }
 template <bool kOpacity>
@@ -720,7 +750,8 @@ __global__ void __launch_bounds__(kGroupBlock, kGroup2Blocks) k_stage2_group(con
                                                                  const float* __restrict__ mat_tr,
                                                                  const __grid_constant__ StageArgs a) {
     __shared__ GroupStacks2 stacks;
-    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, a.n, a.work, StageRays{a}, stacks);
+    __shared__ uint32_t s_work;
+    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, a.n, group_work(a, &s_work), StageRays{a}, stacks);
     stage_done(a.work);
 }
 template <bool kOpacity>
@@ -1122,24 +1153,31 @@ static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
     a.insts = sc.insts;
     a.postpone_sp = 16;
     a.refill_min = 8;
-    const bool op = sc.has_non_opaque != 0;
-    const bool few = a.n <= (sc.insts ? kGroupRays2 : kGroupRays);
-    const uint32_t per_block = few ? 128u / kGroupLanes : 128u;
-    const uint32_t full = sc.insts ? (few ? lc.grid_group2 : lc.grid_stage2) : (few ? lc.grid_group : lc.grid_stage);
-    const uint32_t grid = min(full, (uint32_t)(((uint64_t)a.n + per_block - 1) / per_block));
-    if (sc.insts && few) {
-        if (op) k_stage2_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-        else k_stage2_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-    } else if (sc.insts) {
-        if (op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-        else k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-    } else if (few) {
-        if (op) k_stage_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+    const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr, any = a.occluded != nullptr;
+    if (a.n <= (two ? kGroupRays2 : kGroupRays)) {
+        const uint32_t all = (a.n + 128u / kGroupLanes - 1u) / (128u / kGroupLanes), full = two ? lc.grid_group2 : lc.grid_group;
+        if (all <= full) a.work = nullptr;
+        const uint32_t grid = a.work ? full : all;
+        if (two && op) k_stage2_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else if (two) k_stage2_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else if (op) k_stage_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
         else k_stage_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
-    } else {
-        if (op) k_stage<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
-        else k_stage<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+        return;
     }
+    const uint32_t all = (uint32_t)(((uint64_t)a.n + 127u) / 128u);
+    // without a counter, or with more rays than it can count, a ray per thread: 1,000,003 rays as above 990 us
+    if (!a.work || a.n > kMaxTraceRays) {
+        if (two && any) k_stage_ray<true, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+        else if (two) k_stage_ray<false, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+        else if (any) k_stage_ray<true, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+        else k_stage_ray<false, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+        return;
+    }
+    const uint32_t grid = min((uint32_t)(two ? lc.grid_stage2 : lc.grid_stage), all);
+    if (two && op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+    else if (two) k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+    else if (op) k_stage<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    else k_stage<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
 }
 void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
                           uint4* hits, uint32_t* work) {

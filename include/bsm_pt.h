@@ -391,7 +391,12 @@ BSM_API bsm_status bsm_import_history(bsm_context* ctx, uint32_t view_index, con
  * primitive id 0xffffffff and t = tmax.  Replaces TraceRay in rt_gbuffer_rgen
  * with the closest-hit shader (rt_gbuffer.hlsl:7-36, rt_gbuffer_hit.hlsl:6-18).
  * With location BSM_DEVICE both buffers are device memory and the call is
- * asynchronous on the work stream; with BSM_HOST it waits. */
+ * asynchronous on the work stream; with BSM_HOST it waits.  A call with device
+ * buffers may be captured into a caller's graph; a captured launch has no
+ * state but its buffers, so replays may run beside other calls of the context
+ * and, from several instances of the graph, beside one another (on the same
+ * rays, which get the same hits).  The same holds for bsm_trace_any and for
+ * bsm_render_primary. */
 BSM_API bsm_status bsm_trace_closest(bsm_context* ctx, uint32_t scene_id, const float* rays, uint32_t n,
                                      void* hits, uint32_t location);
 /* occluded: n bytes, 1 if any triangle lies in (tmin, tmax].  Replaces the
