@@ -645,6 +645,7 @@ struct StageArgs {
     const InstDev* insts;
     uint32_t n;
     uint32_t* work;           // [2], zero between launches; null: the launch takes its rays without a counter
+    float near;               // k_stage: how far apart the origins of rays that are traced side by side may be
     int postpone_sp, refill_min;
     DevView view;
 };
@@ -724,15 +725,45 @@ __global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNo
     else rays.hit(i, leaf, t, u, v, inst);
 }
 
-// The caller's rays run on the persistent loops: with a ray per thread to the
-// end, as before, every warp waited for its longest ray and the last rays of a
-// launch held whole blocks. Closest and any hit of 1,000,003 rays, 1.48 M
-// triangles: 1693 -> 854 us (of it 8 % from the node and triangle tests);
-// 4 M rays 6490 -> 2951 us; 300,000 rays in 1,000 instances 752 -> 411 us.
-template <bool kOpacity>
+// More rays than fit at once, whose lanes take new ones when theirs are done:
+// with a ray per thread every warp waits for its longest ray.  But rays that
+// start side by side and head the same way are done together, and the loop's
+// votes, queue reads and postponed leaves then cost more than the waiting (a
+// quarter of the time where materials are not opaque), so a warp whose 32 rays
+// are alike traces them a ray per lane and looks at the next 32.  A ray per
+// thread / the loop alone / this kernel, us, closest hits of 1,000,003 rays:
+// incoherent ones in 1.48 M triangles 653 / 416 / 419, in the room 384 / 266 / 270;
+// a camera's 246 / 301 / 273 and 219 / 299 / 256, with non-opaque materials 310 / 484 / 391.
+template <bool kOpacity, bool kAny>
 __global__ void __launch_bounds__(128, 8) k_stage(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
                                                   const __grid_constant__ StageArgs a) {
-    trace_queue<false, kOpacity>(nodes, tris, a.n, a.work, StageRays{a}, nullptr, a.postpone_sp, a.refill_min);
+    constexpr uint32_t kFull = 0xffffffffu;
+    const StageRays rays{a};
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t head = 0u;
+    while (true) {
+        if (lane == 0) head = atomicAdd(a.work, 32u);
+        head = __shfl_sync(kFull, head, 0);
+        if (head >= a.n) break;
+        const uint32_t i = min(head + lane, a.n - 1u);
+        float4 o, d;
+        rays.load(i, o, d);
+        const uint32_t oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+        const uint32_t oct0 = __shfl_sync(kFull, oct, 0);
+        const float x0 = __shfl_sync(kFull, o.x, 0), y0 = __shfl_sync(kFull, o.y, 0), z0 = __shfl_sync(kFull, o.z, 0);
+        const bool alike = oct == oct0 && fabsf(o.x - x0) <= a.near && fabsf(o.y - y0) <= a.near && fabsf(o.z - z0) <= a.near;
+        if (!__all_sync(kFull, alike)) break;
+        if (head + lane < a.n) {
+            float t, u, v;
+            const uint32_t leaf =
+                trace_ray<kAny, false>(make_ray(o, d), d.w, nodes, tris, t, u, v, nullptr, kOpacity ? rays.seed(i) : 0u);
+            if (leaf == kMissPrim) rays.miss(i, d.w);
+            else rays.hit(i, leaf, t, u, v, kMissPrim);
+        }
+        __syncwarp();
+    }
+    if (head < a.n)
+        trace_queue<false, kOpacity, true>(nodes, tris, a.n, a.work, rays, nullptr, a.postpone_sp, a.refill_min, head);
     stage_done(a.work);
 }
 template <bool kOpacity>
@@ -1138,23 +1169,38 @@ void launch_fold_fixed(cudaStream_t st, const unsigned long long* fx, float4* ac
     if (n == 0) return;
     k_fold_fixed<<<(unsigned)(((uint64_t)n + 255) / 256), 256, 0, st>>>(fx, accum, n);
 }
-// Calls of at most this many rays are traced with eight lanes per ray. Closest and any hit of half-random rays
-// take 76 / 103 us in groups and 115 / 152 lane by lane at 16,384 rays (room / 1.48 M triangles), 177 / 235 and
-// 132 / 194 us at 65,536.
-// In two levels 65 / 103 / 207 us in groups and 132 / 149 / 191 lane by lane at 3,000 / 30,000 / 100,000 rays.
-constexpr uint32_t kGroupRays = 40000, kGroupRays2 = 60000;
+// Which kernel traces a call's rays: eight lanes per ray up to `group` rays, then a ray per thread up to `thread`, then
+// lanes that take new rays.  Closest (c) and any (a) hits of incoherent rays and of a camera's, us, in the three ways:
+//  * one level: c in 1.48 M triangles 71 / 78 / 87 at 30,000 rays, 86 / 83 / 90 at 40,000, camera 68 / 74 / 80; a in the
+//    room 45 / 35 / 40 at 40,000.  A ray per thread while the GPU holds all of them (155,648: c - / 138 / 149, a - / 60 /
+//    66), and twice as many where materials are not opaque and the third loop is longest (300,007: - / 186 / 184, camera
+//    160 / 230);
+//  * two levels: c in 1,000 instances 188 / 195 / 170 at 60,000, camera 196 / 289 / 233.  Rays of few instances are short:
+//    a in eight 21 / 23 / 25 at 20,000, 33 / 19 / 23 at 40,000; 52 / 59 and camera 32 / 39 at 300,007 (second and third),
+//    140 / 118 and 74 / 82 at 1,000,003; c in eight 32 / 27 / 29 at 30,000, in 32 75 / 46 / 44 at 80,000.  Any hits are
+//    between: in 300 instances 61 / 52 / 60 and camera 39 / 67 / 60 at 40,000, 73 / 52 / 51 and 47 / 66 / 57 at 60,000; in
+//    1,000 93 / 76 / 78 and 76 / 122 / 110.
+struct StageLimits { uint32_t group, thread; };
+static StageLimits stage_limits(const LaunchCfg& lc, bool two, bool op, bool any, uint32_t instances) {
+    if (!two) return {40000u, (uint32_t)lc.grid_stage * 128u * (op ? 2u : 1u)};
+    if (instances < 64u) return any ? StageLimits{25000u, 400000u} : StageLimits{32000u, 100000u};
+    if (instances < 500u && any) return {40000u, 100000u};
+    return {60000u, 0u};
+}
 // Views of at most this many pixels take that way too, their hit records waiting in one of the outputs for
 // k_primary_rec: 35 / 58 us against 37 / 113 us in k_primary at 128x128 (room / 1.48 M triangles); at 230x170
-// 48 / 86 against 41 / 111.
-constexpr uint32_t kGroupPixels = 24576;
+// 48 / 86 against 41 / 111. Not for a pixel or two (a pick), where the second launch shows: 14.6 us against 12.5.
+constexpr uint32_t kGroupPixels = 24576, kMinGroupPixels = 4;
 
 static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, StageArgs& a) {
     a.tris = sc.tris;
     a.insts = sc.insts;
+    a.near = sc.ray_offset * 1562.5f;   // a 32nd of the scene's extent
     a.postpone_sp = 16;
     a.refill_min = 8;
     const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr, any = a.occluded != nullptr;
-    if (a.n <= (two ? kGroupRays2 : kGroupRays)) {
+    const StageLimits lim = stage_limits(lc, two, op, any, sc.num_instances);
+    if (a.n <= lim.group) {
         const uint32_t all = (a.n + 128u / kGroupLanes - 1u) / (128u / kGroupLanes), full = two ? lc.grid_group2 : lc.grid_group;
         if (all <= full) a.work = nullptr;
         const uint32_t grid = a.work ? full : all;
@@ -1165,8 +1211,7 @@ static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
         return;
     }
     const uint32_t all = (uint32_t)(((uint64_t)a.n + 127u) / 128u);
-    // without a counter, or with more rays than it can count, a ray per thread: 1,000,003 rays as above 990 us
-    if (!a.work || a.n > kMaxTraceRays) {
+    if (a.n <= lim.thread || !a.work || a.n > kMaxTraceRays) {   // (a counter is for as many rays as it can count)
         if (two && any) k_stage_ray<true, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
         else if (two) k_stage_ray<false, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
         else if (any) k_stage_ray<true, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
@@ -1176,8 +1221,10 @@ static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
     const uint32_t grid = min((uint32_t)(two ? lc.grid_stage2 : lc.grid_stage), all);
     if (two && op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
     else if (two) k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-    else if (op) k_stage<true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
-    else k_stage<false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    else if (op && any) k_stage<true, true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    else if (op) k_stage<true, false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    else if (any) k_stage<false, true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    else k_stage<false, false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
 }
 void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
                           uint4* hits, uint32_t* work) {
@@ -1205,7 +1252,7 @@ void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, co
     if (n == 0) return;
     const PrimaryOut out{depth, {gb[0], gb[1], gb[2], gb[3]}, hitpos, near_z, far_z};
     float4* rec = hitpos ? hitpos : gb[0] ? gb[0] : gb[1] ? gb[1] : gb[2] ? gb[2] : gb[3];
-    if (rec && !sc.insts && n <= kGroupPixels) {
+    if (rec && !sc.insts && n >= kMinGroupPixels && n <= kGroupPixels) {
         StageArgs a{};
         a.rec = rec;
         a.n = n;
@@ -1242,7 +1289,7 @@ void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     if (per_sm_shade < 1) per_sm_shade = 1;
     lc->block_trace = block_trace;
     int per_sm_stage = 0, per_sm_stage2 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage, k_stage<true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage, k_stage<true, true>, 128, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage2, k_stage2<true>, 128, 0);
     lc->grid_stage = sms * (per_sm_stage < 1 ? 1 : per_sm_stage);
     lc->grid_stage2 = sms * (per_sm_stage2 < 1 ? 1 : per_sm_stage2);

@@ -482,10 +482,13 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // `postpone_sp` (<= kPostponeMaxSp) is the stack depth below which triangle
 // groups may be postponed (0 disables postponing); `refill_min` is the number
 // of idle lanes that makes the warp fetch new rays.  Both are tuning knobs.
-template <bool kCount, bool kOpacity, class Rays>
+// With kHead the warp's first rays are `head` .. `head` + 31, which it has taken
+// from the queue already.
+template <bool kCount, bool kOpacity, bool kHead = false, class Rays>
 __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
                                             uint32_t n, uint32_t* work, const Rays& rays, TraceCounters* cnt,
-                                            int postpone_sp, int refill_min) {
+                                            int postpone_sp, int refill_min, uint32_t head = 0u) {
+    bool lead = kHead;
     postpone_sp = postpone_sp < kPostponeMaxSp ? postpone_sp : kPostponeMaxSp;
     const uint32_t lane = threadIdx.x & 31u;
     bool has = false;
@@ -502,9 +505,12 @@ __device__ __forceinline__ void trace_queue(const CwNode* __restrict__ nodes, co
         uint32_t act = ~idle;   // lanes holding a ray in this iteration (taken again after a refill)
         if (!exhausted && (__popc(idle) >= refill_min || idle == 0xffffffffu)) {
             uint32_t cntn = (uint32_t)__popc(idle);
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(work, cntn);
-            base = __shfl_sync(0xffffffffu, base, 0);
+            uint32_t base = head;
+            if (!kHead || !lead) {
+                if (lane == 0) base = atomicAdd(work, cntn);
+                base = __shfl_sync(0xffffffffu, base, 0);
+            }
+            lead = false;
             if (!has) {
                 uint32_t i = base + (uint32_t)__popc(idle & lanemask_lt());
                 if (i < n) {
