@@ -1233,21 +1233,15 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_nodes(const uint32_t* __r
         }
         // greedy octant slots: in every round the child and free slot whose direction agrees best, the first child
         // and then the first slot of equal ones
-        // (boxes whose centres or distances overflow: a NaN of the round's very first pair wins, any other loses, which
-        // is what comparing the pairs one after the other gives; the lanes of a node have to agree)
-        const bool far = !(fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]) < INFINITY);
         uint32_t used = 0, slot = kNone;
         const uint32_t nc = (uint32_t)__popc((__ballot_sync(kFull, valid) >> shift) & 0xffu);
         for (uint32_t round = 0; round < kWideLanes; ++round) {
             float best = -INFINITY;
             uint32_t key = kNone;
-            const bool wait = valid && slot == kNone;
-            const uint32_t waiting = (__ballot_sync(kFull, wait) >> shift) & 0xffu;
-            if (wait)
+            if (valid && slot == kNone)
                 for (uint32_t s = 0; s < 8u; ++s) {
                     if ((used >> s) & 1u) continue;
-                    float cost = ((s & 1u) ? d[0] : -d[0]) + ((s & 2u) ? d[1] : -d[1]) + ((s & 4u) ? d[2] : -d[2]);
-                    if (far && cost != cost) cost = key == kNone && (waiting & ((1u << sub) - 1u)) == 0u ? INFINITY : -INFINITY;
+                    const float cost = ((s & 1u) ? d[0] : -d[0]) + ((s & 2u) ? d[1] : -d[1]) + ((s & 4u) ? d[2] : -d[2]);
                     if (cost > best || key == kNone) { best = cost; key = (sub << 3) | s; }
                 }
             for (int o = 1; o < (int)kWideLanes; o <<= 1) {
@@ -1260,6 +1254,10 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_nodes(const uint32_t* __r
                 if ((key >> 3) == sub) slot = key & 7u;
             }
         }
+        // Where centres or distances overflow, costs are infinite or NaN and the lanes may not have agreed: the children
+        // take the slots in their order (as comparing the pairs one after the other gives if all costs are NaN).
+        const bool far = valid && !(fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]) < INFINITY);
+        if (((__ballot_sync(kFull, far) >> shift) & 0xffu) != 0u) slot = sub;
         if (leaf && (count == 0u || count > kMaxLeafTris)) {
             atomicOr(&cnt->error, kErrLeaf);
             leaf = false;

@@ -7,7 +7,7 @@ import zlib
 import numpy as np
 import pytest
 
-from test_gpu_bvh_build import device_tree
+from test_gpu_bvh_build import check_invariants, device_tree
 from test_gpu_bvh_edges import soup
 from test_bvh_host import decode
 
@@ -34,4 +34,13 @@ def test_centres_that_overflow(bsm, ctx, n):
     _, tris = decode(nb, tb)
     assert np.array_equal(np.sort(tris["prim"]), np.arange(n))
     assert (zlib.crc32(nb.tobytes()), zlib.crc32(tb.tobytes())) == TREES[n]
+    ctx.release(sid)
+
+
+@pytest.mark.parametrize("n", [5, 33, 200, 3000])
+def test_centres_that_overflow_in_part(bsm, ctx, n):
+    sc = soup(bsm, "scattered", n)
+    sc.positions = (1.6e38 + 0.7e38 * np.clip(sc.positions.astype(np.float64), -1.2, 1.2)).astype(np.float32)
+    sid, st, nb, tb = device_tree(bsm, ctx, sc, collapse=1)
+    check_invariants(sc, nb, tb, st)
     ctx.release(sid)
