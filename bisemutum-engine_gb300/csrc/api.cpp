@@ -172,16 +172,6 @@ bsm_status dev_alloc(bsm_context* ctx, DevBuf& b, size_t bytes) {
     ctx->used += bytes;
     return BSM_OK;
 }
-// The stage entry points' work counter; made with the first BVH, so that no trace allocates. Without it they do without.
-void make_stage_work(bsm_context* ctx) {
-    if (ctx->stage_work) return;
-    if (cudaMalloc((void**)&ctx->stage_work, 8) != cudaSuccess) ctx->stage_work = nullptr;
-    else if (cudaMemsetAsync(ctx->stage_work, 0, 8, WS(ctx)) != cudaSuccess) {
-        cudaFree(ctx->stage_work);
-        ctx->stage_work = nullptr;
-    }
-    if (!ctx->stage_work) cudaGetLastError();
-}
 void dev_free(bsm_context* ctx, DevBuf& b) {
     if (b.ptr) { cudaFree(b.ptr); ctx->used -= b.bytes; }
     b.ptr = nullptr;
@@ -424,6 +414,16 @@ extern "C" bsm_status bsm_create(bsm_context** out, int device, uint64_t budget)
     ctx->device = device;
     if (cudaSetDevice(device) != cudaSuccess) { delete ctx; return BSM_ERR_CUDA; }
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return BSM_ERR_CUDA; }
+    // (made here and not with the first BVH, behind which it costs every later build of a small mesh 40 us of cudaMalloc
+    // and cudaFree: the room 1.005 -> 1.04 ms; bsm_set_stream orders the clear before work on other streams)
+    if (cudaMalloc((void**)&ctx->stage_work, 8) != cudaSuccess ||
+        cudaMemsetAsync(ctx->stage_work, 0, 8, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ctx->stage_work);
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+        return BSM_ERR_OUT_OF_MEMORY;
+    }
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     ctx->budget = budget ? budget : (uint64_t)((double)fr * 0.9);
@@ -900,7 +900,6 @@ extern "C" bsm_status bsm_scene_build_bvh(bsm_context* ctx, uint32_t scene_id, c
         sc->dev.tris = (const CwTri*)sc->tris.ptr;
         if ((st = make_tri_normals(ctx, sc))) return st;
         sc->has_bvh = true;
-        make_stage_work(ctx);
         sc->bvh_stats = s;
         clear_graphs(ctx);
         if (stats) *stats = s;
@@ -928,7 +927,6 @@ extern "C" bsm_status bsm_scene_build_bvh(bsm_context* ctx, uint32_t scene_id, c
     sc->dev.tris = (const CwTri*)sc->tris.ptr;
     if ((st = make_tri_normals(ctx, sc))) return st;
     sc->has_bvh = true;
-    make_stage_work(ctx);
     bsm_bvh_stats s{};
     s.num_nodes = (uint32_t)r.nodes.size();
     s.num_tris = (uint32_t)r.tris.size();
@@ -1143,7 +1141,6 @@ bsm_status build_tlas(bsm_context* ctx, Scene* sc) {
     bs.tri_bytes = (uint64_t)n * sizeof(InstDev);
     sc->bvh_stats = bs;
     sc->has_bvh = true;
-    make_stage_work(ctx);
     clear_graphs(ctx);
     return BSM_OK;
 }
@@ -1987,7 +1984,8 @@ namespace {
 // The work counter of a stage entry point's launch. Direct calls follow one another (bsm_set_stream keeps their order
 // across streams), so one counter serves them all. A launch that is captured into a caller's graph may be replayed
 // beside them, and beside itself from a second instance of the graph: it gets none.
-uint32_t* stage_work(bsm_context* ctx) {
+uint32_t* stage_work(bsm_context* ctx, uint64_t n) {
+    if (n <= 16u * (uint32_t)std::min(ctx->lc.grid_group, ctx->lc.grid_group2)) return nullptr;   // they fit at once
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(WS(ctx), &c) == cudaSuccess) return c == cudaStreamCaptureStatusNone ? ctx->stage_work : nullptr;
     cudaGetLastError();
@@ -2013,7 +2011,7 @@ extern "C" bsm_status bsm_trace_closest(bsm_context* ctx, uint32_t scene_id, con
     if (n == 0) return BSM_OK;
     if (!rays || !hits) return BSM_ERR_INVALID_ARG;
     if (location == BSM_DEVICE) {
-        launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, (uint4*)hits, stage_work(ctx));
+        launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, (uint4*)hits, stage_work(ctx, n));
         CK(cudaGetLastError());
         return BSM_OK;   // queued on the work stream
     }
@@ -2021,7 +2019,7 @@ extern "C" bsm_status bsm_trace_closest(bsm_context* ctx, uint32_t scene_id, con
     if ((st = dev_alloc(ctx, ctx->tmp, rb + hb))) return st;
     char* b = (char*)ctx->tmp.ptr;
     CK(cudaMemcpyAsync(b, rays, rb, cudaMemcpyHostToDevice, WS(ctx)));
-    launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint4*)(b + rb), stage_work(ctx));
+    launch_trace_closest(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint4*)(b + rb), stage_work(ctx, n));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(hits, b + rb, hb, cudaMemcpyDeviceToHost, WS(ctx)));
     CK(cudaStreamSynchronize(WS(ctx)));
@@ -2036,7 +2034,7 @@ extern "C" bsm_status bsm_trace_any(bsm_context* ctx, uint32_t scene_id, const f
     if (n == 0) return BSM_OK;
     if (!rays || !occluded) return BSM_ERR_INVALID_ARG;
     if (location == BSM_DEVICE) {
-        launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, occluded, stage_work(ctx));
+        launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)rays, n, occluded, stage_work(ctx, n));
         CK(cudaGetLastError());
         return BSM_OK;   // queued on the work stream
     }
@@ -2044,7 +2042,7 @@ extern "C" bsm_status bsm_trace_any(bsm_context* ctx, uint32_t scene_id, const f
     if ((st = dev_alloc(ctx, ctx->tmp, rb + n + 16))) return st;
     char* b = (char*)ctx->tmp.ptr;
     CK(cudaMemcpyAsync(b, rays, rb, cudaMemcpyHostToDevice, WS(ctx)));
-    launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint8_t*)(b + rb), stage_work(ctx));
+    launch_trace_any(ctx->lc, WS(ctx), sc->dev, (const float4*)b, n, (uint8_t*)(b + rb), stage_work(ctx, n));
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(occluded, b + rb, n, cudaMemcpyDeviceToHost, WS(ctx)));
     CK(cudaStreamSynchronize(WS(ctx)));
@@ -2117,7 +2115,8 @@ extern "C" bsm_status bsm_render_primary(bsm_context* ctx, uint32_t scene_id, co
             if (dst[k]) { dev[k] = (float*)b; b += (bytes[k] + 15) & ~(size_t)15; }   // float4 arrays follow
     }
     float4* gb[4] = {(float4*)dev[1], (float4*)dev[2], (float4*)dev[3], (float4*)dev[4]};
-    launch_primary(ctx->lc, WS(ctx), sc->dev, v, near_z, far_z, dev[0], gb, (float4*)dev[5], stage_work(ctx));
+    launch_primary(ctx->lc, WS(ctx), sc->dev, v, near_z, far_z, dev[0], gb, (float4*)dev[5],
+                   stage_work(ctx, (uint64_t)v.width * v.height));
     CK(cudaGetLastError());
     if (out->location == BSM_DEVICE) return BSM_OK;   // queued on the work stream
     for (int k = 0; k < 6; ++k)
