@@ -637,10 +637,10 @@ __global__ void k_gather_normals(const CwTri* __restrict__ tris, uint32_t n, con
 // Rays of the stage entry points (a caller's array) and of small views' primary
 // outputs (a pixel-centre camera ray per pixel), on the wavefront's loops.
 struct StageArgs {
-    const float4* rays;       // a caller's rays (origin/tmin, direction/tmax), or null: camera rays of `view`
+    const float4* rays;       // a caller's rays (origin/tmin, direction/tmax)
     uint4* hits;              // t, primitive id, u, v of each ray
     uint8_t* occluded;        // or whether it hit anything
-    float4* rec;              // camera rays: hit records (t, leaf, u, v) for k_primary_rec
+    float4* rec;              // or, of the camera rays of `view`, hit records (t, leaf, u, v) for k_primary_rec
     const CwTri* tris;        // for the primitive ids
     const InstDev* insts;
     uint32_t n;
@@ -649,11 +649,17 @@ struct StageArgs {
     int postpone_sp, refill_min;
     DevView view;
 };
+// A kernel is made for one kind of rays and output: asking which at every ray and hit cost the loops 2 to 4 % and
+// registers (non-opaque materials, 1,000,003 closest hits in the room: 376 -> 323 us). kStageEither, which asks, is for
+// two kernels that come out slower when they know (stage2_out).
+enum : int { kStageHits, kStageOccluded, kStageRec, kStageEither };
+template <int kOut>
 struct StageRays {
     const StageArgs& a;
-    __device__ __forceinline__ bool any(uint32_t) const { return a.occluded != nullptr; }
+    __device__ __forceinline__ bool to_hits() const { return kOut == kStageEither ? a.hits != nullptr : kOut == kStageHits; }
+    __device__ __forceinline__ bool any(uint32_t) const { return kOut == kStageEither ? a.occluded != nullptr : kOut == kStageOccluded; }
     __device__ __forceinline__ void load(uint32_t i, float4& o, float4& d) const {
-        if (a.rays) {
+        if (kOut == kStageEither ? a.rays != nullptr : kOut != kStageRec) {
             o = __ldg(a.rays + 2 * (size_t)i);
             d = __ldg(a.rays + 2 * (size_t)i + 1);
             return;
@@ -664,25 +670,25 @@ struct StageRays {
         d = make_float4(dw.x, dw.y, dw.z, a.view.ray_length);
     }
     __device__ __forceinline__ void hit(uint32_t i, uint32_t leaf, float t, float u, float v, uint32_t inst) const {
-        if (a.hits) {
+        if (to_hits()) {
             const uint32_t prim = inst != kMissPrim ? a.insts[inst].prim_base + a.insts[inst].tris[leaf].prim
                                                     : a.tris[leaf].prim;
             a.hits[i] = make_uint4(__float_as_uint(t), prim, __float_as_uint(u), __float_as_uint(v));
-        } else if (a.occluded) {
+        } else if (kOut == kStageEither ? a.occluded != nullptr : kOut != kStageRec) {
             a.occluded[i] = 1;
         } else {
             a.rec[i] = make_float4(t, __uint_as_float(leaf), u, v);
         }
     }
     __device__ __forceinline__ void miss(uint32_t i, float tmax) const {
-        if (a.hits) a.hits[i] = make_uint4(__float_as_uint(tmax), kMissPrim, 0u, 0u);
-        else if (a.occluded) a.occluded[i] = 0;
+        if (to_hits()) a.hits[i] = make_uint4(__float_as_uint(tmax), kMissPrim, 0u, 0u);
+        else if (kOut == kStageEither ? a.occluded != nullptr : kOut != kStageRec) a.occluded[i] = 0;
         else a.rec[i] = make_float4(tmax, __uint_as_float(kMissPrim), 0.0f, 0.0f);
     }
     // opacity decisions: a caller's rays draw with seed 0, a pixel's with the camera-ray PCG word of sample 0 of
     // an unjittered render
     __device__ __forceinline__ uint32_t seed(uint32_t i) const {
-        if (a.rays) return 0u;
+        if (kOut == kStageEither ? a.rays != nullptr : kOut != kStageRec) return 0u;
         return (uint32_t)pcg_seed(path_initstate(a.view.seed, a.view.sample_offset, i), (uint64_t)i).state;
     }
 };
@@ -706,7 +712,7 @@ __device__ __forceinline__ uint32_t* group_work(const StageArgs& a, uint32_t* s_
 }
 
 // A ray per thread: no queue and no counter.
-template <bool kAny, bool kTwoLevel>
+template <int kOut, bool kTwoLevel>
 __global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNode* __restrict__ nodes,
                                                                       const CwTri* __restrict__ tris,
                                                                       const InstDev* __restrict__ insts,
@@ -714,7 +720,8 @@ __global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNo
                                                                       const __grid_constant__ StageArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    const StageRays rays{a};
+    constexpr bool kAny = kOut == kStageOccluded;
+    const StageRays<kOut> rays{a};
     float4 o, d;
     rays.load(i, o, d);
     float t, u, v;
@@ -734,11 +741,12 @@ __global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNo
 // thread / the loop alone / this kernel, us, closest hits of 1,000,003 rays:
 // incoherent ones in 1.48 M triangles 653 / 416 / 419, in the room 384 / 266 / 270;
 // a camera's 246 / 301 / 273 and 219 / 299 / 256, with non-opaque materials 310 / 484 / 391.
-template <bool kOpacity, bool kAny>
+template <bool kOpacity, int kOut>
 __global__ void __launch_bounds__(128, 8) k_stage(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
                                                   const __grid_constant__ StageArgs a) {
     constexpr uint32_t kFull = 0xffffffffu;
-    const StageRays rays{a};
+    constexpr bool kAny = kOut == kStageOccluded;
+    const StageRays<kOut> rays{a};
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t head = 0u;
     while (true) {
@@ -766,30 +774,36 @@ __global__ void __launch_bounds__(128, 8) k_stage(const CwNode* __restrict__ nod
         trace_queue<false, kOpacity, true>(nodes, tris, a.n, a.work, rays, nullptr, a.postpone_sp, a.refill_min, head);
     stage_done(a.work);
 }
-template <bool kOpacity>
+template <bool kOpacity, int kOut>
 __global__ void __launch_bounds__(kGroupBlock, 6) k_stage_group(const CwNode* __restrict__ nodes,
                                                                 const CwTri* __restrict__ tris,
                                                                 const __grid_constant__ StageArgs a) {
     __shared__ GroupStacks stacks;
     __shared__ uint32_t s_work;
-    trace_queue_group<kOpacity>(nodes, tris, a.n, group_work(a, &s_work), StageRays{a}, stacks);
+    trace_queue_group<kOpacity>(nodes, tris, a.n, group_work(a, &s_work), StageRays<kOut>{a}, stacks);
     stage_done(a.work);
 }
-template <bool kOpacity>
+template <bool kOpacity, int kOut>
 __global__ void __launch_bounds__(kGroupBlock, kGroup2Blocks) k_stage2_group(const CwNode* __restrict__ tlas,
                                                                  const InstDev* __restrict__ insts,
                                                                  const float* __restrict__ mat_tr,
                                                                  const __grid_constant__ StageArgs a) {
     __shared__ GroupStacks2 stacks;
     __shared__ uint32_t s_work;
-    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, a.n, group_work(a, &s_work), StageRays{a}, stacks);
+    trace_queue2_group<kOpacity>(tlas, insts, mat_tr, a.n, group_work(a, &s_work), StageRays<kOut>{a}, stacks);
     stage_done(a.work);
 }
-template <bool kOpacity>
+// Closest hits of opaque and any hits of non-opaque scenes come out slower when their kernel knows its output, the other
+// two faster (1,500,003 incoherent rays, 300 instances, knowing / asking: closest 705 / 576 and non-opaque 628 / 697 us,
+// any 261 / 290 and 454 / 403).
+constexpr int stage2_out(bool opacity, int out) {
+    return opacity == (out == kStageOccluded) ? (int)kStageEither : out;
+}
+template <bool kOpacity, int kOut>
 __global__ void __launch_bounds__(128, 8) k_stage2(const CwNode* __restrict__ tlas, const InstDev* __restrict__ insts,
                                                    const float* __restrict__ mat_tr,
                                                    const __grid_constant__ StageArgs a) {
-    trace_queue2<kOpacity>(tlas, insts, mat_tr, a.n, a.work, StageRays{a}, a.postpone_sp, a.refill_min);
+    trace_queue2<kOpacity>(tlas, insts, mat_tr, a.n, a.work, StageRays<kOut>{a}, a.postpone_sp, a.refill_min);
     stage_done(a.work);
 }
 
@@ -1192,39 +1206,44 @@ static StageLimits stage_limits(const LaunchCfg& lc, bool two, bool op, bool any
 // 48 / 86 against 41 / 111. Not for a pixel or two (a pick), where the second launch shows: 14.6 us against 12.5.
 constexpr uint32_t kGroupPixels = 24576, kMinGroupPixels = 4;
 
+template <bool kOpacity, int kOut>
+static void launch_stage_kernel(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, StageArgs& a) {
+    const bool two = sc.insts != nullptr;
+    const StageLimits lim = stage_limits(lc, two, kOpacity, kOut == kStageOccluded, sc.num_instances);
+    if (kOut == kStageRec || a.n <= lim.group) {
+        const uint32_t all = (a.n + 128u / kGroupLanes - 1u) / (128u / kGroupLanes), full = two ? lc.grid_group2 : lc.grid_group;
+        if (all <= full) a.work = nullptr;
+        const uint32_t grid = a.work ? full : all;
+        if constexpr (kOut != kStageRec) {
+            if (two) {
+                k_stage2_group<kOpacity, kOut><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+                return;
+            }
+        }
+        k_stage_group<kOpacity, kOut><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
+        return;
+    }
+    if constexpr (kOut != kStageRec) {
+        const uint32_t all = (uint32_t)(((uint64_t)a.n + 127u) / 128u);
+        if (a.n <= lim.thread || !a.work || a.n > kMaxTraceRays) {   // (a counter is for as many rays as it can count)
+            if (two) k_stage_ray<kOut, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+            else k_stage_ray<kOut, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
+            return;
+        }
+        const uint32_t grid = min((uint32_t)(two ? lc.grid_stage2 : lc.grid_stage), all);
+        if (two) k_stage2<kOpacity, stage2_out(kOpacity, kOut)><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
+        else k_stage<kOpacity, kOut><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    }
+}
+template <int kOut>
 static void launch_stage(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, StageArgs& a) {
     a.tris = sc.tris;
     a.insts = sc.insts;
     a.near = sc.ray_offset * 1562.5f;   // a 32nd of the scene's extent
     a.postpone_sp = 16;
     a.refill_min = 8;
-    const bool op = sc.has_non_opaque != 0, two = sc.insts != nullptr, any = a.occluded != nullptr;
-    const StageLimits lim = stage_limits(lc, two, op, any, sc.num_instances);
-    if (a.n <= lim.group) {
-        const uint32_t all = (a.n + 128u / kGroupLanes - 1u) / (128u / kGroupLanes), full = two ? lc.grid_group2 : lc.grid_group;
-        if (all <= full) a.work = nullptr;
-        const uint32_t grid = a.work ? full : all;
-        if (two && op) k_stage2_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-        else if (two) k_stage2_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-        else if (op) k_stage_group<true><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
-        else k_stage_group<false><<<grid, kGroupBlock, 0, st>>>(sc.nodes, sc.tris, a);
-        return;
-    }
-    const uint32_t all = (uint32_t)(((uint64_t)a.n + 127u) / 128u);
-    if (a.n <= lim.thread || !a.work || a.n > kMaxTraceRays) {   // (a counter is for as many rays as it can count)
-        if (two && any) k_stage_ray<true, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
-        else if (two) k_stage_ray<false, true><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
-        else if (any) k_stage_ray<true, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
-        else k_stage_ray<false, false><<<all, 128, 0, st>>>(sc.nodes, sc.tris, sc.insts, sc.mat_tr, a);
-        return;
-    }
-    const uint32_t grid = min((uint32_t)(two ? lc.grid_stage2 : lc.grid_stage), all);
-    if (two && op) k_stage2<true><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-    else if (two) k_stage2<false><<<grid, 128, 0, st>>>(sc.nodes, sc.insts, sc.mat_tr, a);
-    else if (op && any) k_stage<true, true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
-    else if (op) k_stage<true, false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
-    else if (any) k_stage<false, true><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
-    else k_stage<false, false><<<grid, 128, 0, st>>>(sc.nodes, sc.tris, a);
+    if (sc.has_non_opaque) launch_stage_kernel<true, kOut>(lc, st, sc, a);
+    else launch_stage_kernel<false, kOut>(lc, st, sc, a);
 }
 void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
                           uint4* hits, uint32_t* work) {
@@ -1234,7 +1253,7 @@ void launch_trace_closest(const LaunchCfg& lc, cudaStream_t st, const DevScene& 
     a.hits = hits;
     a.n = n;
     a.work = work;
-    launch_stage(lc, st, sc, a);
+    launch_stage<kStageHits>(lc, st, sc, a);
 }
 void launch_trace_any(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const float4* rays, uint32_t n,
                       uint8_t* occluded, uint32_t* work) {
@@ -1244,7 +1263,7 @@ void launch_trace_any(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, 
     a.occluded = occluded;
     a.n = n;
     a.work = work;
-    launch_stage(lc, st, sc, a);
+    launch_stage<kStageOccluded>(lc, st, sc, a);
 }
 void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView& v, float near_z,
                     float far_z, float* depth, float4* const gb[4], float4* hitpos, uint32_t* work) {
@@ -1258,7 +1277,7 @@ void launch_primary(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, co
         a.n = n;
         a.work = work;
         a.view = v;
-        launch_stage(lc, st, sc, a);
+        launch_stage<kStageRec>(lc, st, sc, a);
         k_primary_rec<<<(n + 127) / 128, 128, 0, st>>>(sc, v, out, rec);
         return;
     }
@@ -1289,8 +1308,8 @@ void query_launch_cfg(int device, int block_trace, LaunchCfg* lc) {
     if (per_sm_shade < 1) per_sm_shade = 1;
     lc->block_trace = block_trace;
     int per_sm_stage = 0, per_sm_stage2 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage, k_stage<true, true>, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage2, k_stage2<true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage, k_stage<true, kStageHits>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_stage2, k_stage2<true, kStageEither>, 128, 0);
     lc->grid_stage = sms * (per_sm_stage < 1 ? 1 : per_sm_stage);
     lc->grid_stage2 = sms * (per_sm_stage2 < 1 ? 1 : per_sm_stage2);
     int per_sm_group = 0, per_sm_group2 = 0;
