@@ -59,8 +59,9 @@ struct Scene {
     std::vector<uint32_t> leaf_of;          // caller index -> TLAS leaf (InstDev record)
     std::vector<uint32_t> level_begin;      // TLAS breadth-first level boundaries (levels + 1 entries)
     std::vector<InstDev> inst_host;         // records in leaf order
-    DevBuf insts, inst_box, node_box, mat_tr;
-    DevBuf inst_src, inst_move;             // bsm_scene_update_instances: InstSrc per instance; its working memory
+    DevBuf insts, inst_src, node_box, mat_tr;   // inst_src: InstSrc per instance, then the instances' world boxes (leaf order)
+    DevBuf inst_move;                       // bsm_scene_update_instances: its working memory
+    float* inst_box() const { return (float*)((InstSrc*)inst_src.ptr + instances.size()); }
     DevScene dev{};
 };
 
@@ -538,7 +539,7 @@ bsm_status build_tlas(bsm_context* ctx, Scene* sc);
 // Device buffers of a scene; an instanced scene also lets go of its geometries.
 void free_scene_buffers(bsm_context* ctx, Scene& sc) {
     for (DevBuf* b : {&sc.nodes, &sc.tris, &sc.materials, &sc.texels, &sc.sky_alias, &sc.pdf_tab, &sc.tri_normals,
-                      &sc.insts, &sc.inst_box, &sc.node_box, &sc.mat_tr, &sc.inst_src, &sc.inst_move})
+                      &sc.insts, &sc.inst_src, &sc.node_box, &sc.mat_tr, &sc.inst_move})
         dev_free(ctx, *b);
     if (sc.instanced)
         for (const bsm_instance& in : sc.instances) {
@@ -1047,11 +1048,12 @@ bool valid_transform(const float* m) {
     return invert_affine(m, inv);
 }
 
-// Instance records (w2o, o2w, BLAS pointers) and world boxes of every instance, in leaf order.
-void fill_instances(bsm_context* ctx, Scene* sc, std::vector<float>& boxes) {
+// Instance records (w2o, o2w, BLAS pointers) in leaf order, and what inst_src holds.
+void fill_instances(bsm_context* ctx, Scene* sc, std::vector<InstSrc>& src) {
     const uint32_t n = (uint32_t)sc->instances.size();
     sc->inst_host.resize(n);
-    boxes.assign(6 * (size_t)n, 0.0f);
+    src.assign(n + ((size_t)n * 24 + sizeof(InstSrc) - 1) / sizeof(InstSrc), InstSrc{});
+    float* boxes = (float*)(src.data() + n);
     uint32_t prim_base = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const bsm_instance& in = sc->instances[i];
@@ -1067,6 +1069,9 @@ void fill_instances(bsm_context* ctx, Scene* sc, std::vector<float>& boxes) {
         r.id = i;
         r.pad = 0;
         prim_base += g->num_triangles;
+        src[i].leaf = leaf;
+        std::memcpy(src[i].lo, g->lo, sizeof(src[i].lo));
+        std::memcpy(src[i].hi, g->hi, sizeof(src[i].hi));
         instance_world_box(in.transform, g->lo, g->hi, &boxes[6 * (size_t)leaf], &boxes[6 * (size_t)leaf + 3]);
     }
 }
@@ -1105,27 +1110,18 @@ bsm_status build_tlas(bsm_context* ctx, Scene* sc) {
     for (uint32_t ni = 0; ni < r.nodes.size(); ++ni)
         if (ni == 0 || depth[ni] != depth[ni - 1]) sc->level_begin.push_back(ni);
     sc->level_begin.push_back((uint32_t)r.nodes.size());
-    std::vector<float> boxes;
-    fill_instances(ctx, sc, boxes);
+    std::vector<InstSrc> src;
+    fill_instances(ctx, sc, src);
     bsm_status st;
     dev_free(ctx, sc->nodes);
     if ((st = dev_alloc(ctx, sc->nodes, r.nodes.size() * sizeof(CwNode)))) return st;
     if ((st = dev_alloc(ctx, sc->insts, (size_t)n * sizeof(InstDev)))) return st;
-    if ((st = dev_alloc(ctx, sc->inst_box, boxes.size() * 4))) return st;
+    if ((st = dev_alloc(ctx, sc->inst_src, src.size() * sizeof(InstSrc)))) return st;
     if ((st = dev_alloc(ctx, sc->node_box, r.nodes.size() * 6 * 4))) return st;
     CK(cudaMemcpy(sc->nodes.ptr, r.nodes.data(), r.nodes.size() * sizeof(CwNode), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(sc->insts.ptr, sc->inst_host.data(), (size_t)n * sizeof(InstDev), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(sc->inst_box.ptr, boxes.data(), boxes.size() * 4, cudaMemcpyHostToDevice));
-    std::vector<InstSrc> src(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        const Geometry* g = ctx->geoms.at(sc->instances[i].geometry_id).get();
-        src[i].leaf = sc->leaf_of[i];
-        std::memcpy(src[i].lo, g->lo, sizeof(src[i].lo));
-        std::memcpy(src[i].hi, g->hi, sizeof(src[i].hi));
-    }
-    if ((st = dev_alloc(ctx, sc->inst_src, (size_t)n * sizeof(InstSrc)))) return st;
+    CK(cudaMemcpy(sc->inst_src.ptr, src.data(), src.size() * sizeof(InstSrc), cudaMemcpyHostToDevice));
     if ((st = dev_alloc(ctx, sc->inst_move, kMoveHeader + (size_t)n * (sizeof(InstMoved) + 48)))) return st;
-    CK(cudaMemcpy(sc->inst_src.ptr, src.data(), (size_t)n * sizeof(InstSrc), cudaMemcpyHostToDevice));
     DevScene& ds = sc->dev;
     ds.nodes = (const CwNode*)sc->nodes.ptr;
     ds.tris = nullptr;
@@ -1318,8 +1314,8 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
         }
         clear_graphs(ctx);  // captured launches hold the scene record by value
     }
-    launch_inst_apply(WS(ctx), moved, num_instances, (InstDev*)sc->insts.ptr, (float*)sc->inst_box.ptr);
-    launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, (const float*)sc->inst_box.ptr,
+    launch_inst_apply(WS(ctx), moved, num_instances, (InstDev*)sc->insts.ptr, sc->inst_box());
+    launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, sc->inst_box(),
                       sc->level_begin.data(), (uint32_t)sc->level_begin.size() - 1u);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(WS(ctx)));
@@ -1332,7 +1328,7 @@ extern "C" bsm_status bsm_scene_device_bytes(bsm_context* ctx, uint32_t scene_id
     if (!sc) return fail(ctx, BSM_ERR_NOT_FOUND, "unknown scene id");
     uint64_t b = 0;
     for (DevBuf* x : {&sc->nodes, &sc->tris, &sc->materials, &sc->texels, &sc->sky_alias, &sc->pdf_tab,
-                      &sc->tri_normals, &sc->insts, &sc->inst_box, &sc->node_box, &sc->mat_tr, &sc->inst_src, &sc->inst_move})
+                      &sc->tri_normals, &sc->insts, &sc->inst_src, &sc->node_box, &sc->mat_tr, &sc->inst_move})
         b += x->bytes;
     *bytes = b;
     return BSM_OK;
