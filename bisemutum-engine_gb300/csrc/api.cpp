@@ -1040,6 +1040,10 @@ void instance_world_box(const float* m, const float glo[3], const float ghi[3], 
 }
 
 constexpr size_t kMoveHeader = 256;   // the sums of launch_inst_move; the moved records and the transforms follow
+// Updates of up to this many instances are made on the host: two waits and three launches take the device longer than the
+// transforms take a core (updates of 2 / 9 / 100 / 201 / 301 / 601 instances, host 21 / 26 / 48 / 63 / 82 / 162 us, device
+// 57 / 64 / 77 / 82 / 83 / 99).
+constexpr uint32_t kHostMoves = 256;
 
 bool valid_transform(const float* m) {
     for (int i = 0; i < 12; ++i)
@@ -1275,31 +1279,48 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
     if (num_instances != sc->instances.size())
         return fail(ctx, BSM_ERR_INVALID_ARG, "transform count differs from the scene's instances");
     if (!sc->inst_src.ptr || !sc->inst_move.ptr) return fail(ctx, BSM_ERR_BAD_STATE, "the scene's last TLAS build failed");
-    // the new records and boxes beside the current ones, which stay if a transform is refused
-    char* mem = (char*)sc->inst_move.ptr;
-    uint32_t* sum_dev = (uint32_t*)mem;
-    InstMoved* moved = (InstMoved*)(mem + kMoveHeader);
-    float* xf_dev = (float*)(mem + kMoveHeader + (size_t)num_instances * sizeof(InstMoved));
-    uint32_t sum[7];
-    CK(cudaMemsetAsync(sum_dev, 0, sizeof(sum), WS(ctx)));
-    CK(cudaMemcpyAsync(xf_dev, transforms, (size_t)num_instances * 48, cudaMemcpyHostToDevice, WS(ctx)));
-    launch_inst_move(WS(ctx), xf_dev, (const InstSrc*)sc->inst_src.ptr, num_instances, moved, sum_dev);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(sum, sum_dev, sizeof(sum), cudaMemcpyDeviceToHost, WS(ctx)));
-    CK(cudaStreamSynchronize(WS(ctx)));  // also: no render may read the records while they change
-    if (sum[0] != 0u)
-        return fail(ctx, BSM_ERR_INVALID_ARG, "instance " + std::to_string(~sum[0]) + ": transform not finite / invertible");
-    for (uint32_t i = 0; i < num_instances; ++i)
-        std::memcpy(sc->instances[i].transform, transforms + 12 * (size_t)i, 12 * sizeof(float));
-    // the scene bounds (ray offset, radiance-cache normalisation) follow the instances, as a rebuild's would
-    auto unkey = [](uint32_t k) {
-        const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-        float f;
-        std::memcpy(&f, &b, 4);
-        return f;
-    };
+    InstMoved* moved = (InstMoved*)((char*)sc->inst_move.ptr + kMoveHeader);
+    std::vector<InstSrc> src;   // few instances: made on the host
     float lo[3], hi[3];
-    for (int k = 0; k < 3; ++k) { lo[k] = unkey(~sum[1 + k]); hi[k] = unkey(sum[4 + k]); }
+    if (num_instances <= kHostMoves) {
+        for (uint32_t i = 0; i < num_instances; ++i)
+            if (!valid_transform(transforms + 12 * (size_t)i))
+                return fail(ctx, BSM_ERR_INVALID_ARG, "instance " + std::to_string(i) + ": transform not finite / invertible");
+        for (uint32_t i = 0; i < num_instances; ++i)
+            std::memcpy(sc->instances[i].transform, transforms + 12 * (size_t)i, 12 * sizeof(float));
+        fill_instances(ctx, sc, src);
+        const float* boxes = (const float*)(src.data() + num_instances);
+        for (int k = 0; k < 3; ++k) { lo[k] = INFINITY; hi[k] = -INFINITY; }
+        for (uint32_t l = 0; l < num_instances; ++l)
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = std::min(lo[k], boxes[6 * (size_t)l + k]);
+                hi[k] = std::max(hi[k], boxes[6 * (size_t)l + 3 + k]);
+            }
+        CK(cudaStreamSynchronize(WS(ctx)));  // no render may read the records while they change
+    } else {
+        // the new records and boxes beside the current ones, which stay if a transform is refused
+        uint32_t* sum_dev = (uint32_t*)sc->inst_move.ptr;
+        float* xf_dev = (float*)(moved + num_instances);
+        uint32_t sum[7];
+        CK(cudaMemsetAsync(sum_dev, 0, sizeof(sum), WS(ctx)));
+        CK(cudaMemcpyAsync(xf_dev, transforms, (size_t)num_instances * 48, cudaMemcpyHostToDevice, WS(ctx)));
+        launch_inst_move(WS(ctx), xf_dev, (const InstSrc*)sc->inst_src.ptr, num_instances, moved, sum_dev);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(sum, sum_dev, sizeof(sum), cudaMemcpyDeviceToHost, WS(ctx)));
+        CK(cudaStreamSynchronize(WS(ctx)));  // also: no render may read the records while they change
+        if (sum[0] != 0u)
+            return fail(ctx, BSM_ERR_INVALID_ARG, "instance " + std::to_string(~sum[0]) + ": transform not finite / invertible");
+        for (uint32_t i = 0; i < num_instances; ++i)
+            std::memcpy(sc->instances[i].transform, transforms + 12 * (size_t)i, 12 * sizeof(float));
+        auto unkey = [](uint32_t k) {
+            const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+            float f;
+            std::memcpy(&f, &b, 4);
+            return f;
+        };
+        for (int k = 0; k < 3; ++k) { lo[k] = unkey(~sum[1 + k]); hi[k] = unkey(sum[4 + k]); }
+    }
+    // the scene bounds (ray offset, radiance-cache normalisation) follow the instances, as a rebuild's would
     float extent = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), std::max(hi[2] - lo[2], 1e-6f));
     DevScene& ds = sc->dev;
     bool moved_bounds = extent != sc->extent;
@@ -1314,7 +1335,13 @@ extern "C" bsm_status bsm_scene_update_instances(bsm_context* ctx, uint32_t scen
         }
         clear_graphs(ctx);  // captured launches hold the scene record by value
     }
-    launch_inst_apply(WS(ctx), moved, num_instances, (InstDev*)sc->insts.ptr, sc->inst_box());
+    if (!src.empty()) {
+        CK(cudaMemcpyAsync(sc->insts.ptr, sc->inst_host.data(), (size_t)num_instances * sizeof(InstDev),
+                           cudaMemcpyHostToDevice, WS(ctx)));
+        CK(cudaMemcpyAsync(sc->inst_src.ptr, src.data(), src.size() * sizeof(InstSrc), cudaMemcpyHostToDevice, WS(ctx)));
+    } else {
+        launch_inst_apply(WS(ctx), moved, num_instances, (InstDev*)sc->insts.ptr, sc->inst_box());
+    }
     launch_tlas_refit(WS(ctx), (CwNode*)sc->nodes.ptr, (float*)sc->node_box.ptr, sc->inst_box(),
                       sc->level_begin.data(), (uint32_t)sc->level_begin.size() - 1u);
     CK(cudaGetLastError());

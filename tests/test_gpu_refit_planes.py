@@ -1,6 +1,7 @@
 """The device refit's nodes against the host's quantiser (tlas_quantise of bvh_quant.h, compiled for the host): after
 bsm_scene_update_instances every TLAS node has the bytes that the quantiser gives for its children's boxes, the instance
-boxes being recomputed here in double precision. Transforms with negative, large and tiny coordinates and flat boxes; up
+boxes being recomputed here in double precision, on both sides of the 256 instances up to which records and boxes are made
+on the host. Transforms with negative, large and tiny coordinates and flat boxes; up
 to an instance count at which a level has more than the 1,024 nodes that one block refits in rounds, and levels of their
 own launches follow."""
 import ctypes as C
@@ -59,7 +60,7 @@ def moved_transforms(rng, n, spread):
     return xf.reshape(n, 12)
 
 
-@pytest.mark.parametrize("n,spread", [(1, 3.0), (300, 0.5), (300, 2e4), (20000, 30.0)])
+@pytest.mark.parametrize("n,spread", [(1, 3.0), (256, 5.0), (257, 5.0), (300, 0.5), (300, 2e4), (20000, 30.0)])
 def test_refitted_nodes_have_the_quantisers_bytes(bsm, ctx, quantise, n, spread):
     rng = np.random.default_rng(n + int(spread))
     box = np.array([[x, y, z] for x in (-1, 1) for y in (-1, 1) for z in (-1, 1)], np.float32)
