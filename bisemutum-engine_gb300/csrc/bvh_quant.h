@@ -1,8 +1,10 @@
-// bvh_quant.h — outward quantisation of one compressed-BVH node, shared by the
-// host and the device TLAS refit.  Same rules as the host builder
-// (bvh_build.cpp): per axis the smallest exponent e with 253 * 2^e >= the node
-// extent, the frame origin one step below the node box, and every child box
-// rounded outward by at least one step, each bound checked in double.
+// bvh_quant.h — outward quantisation of one compressed-BVH node: the definition
+// of what quantise_lanes (bvh_quant_lanes.cuh) computes for the device's builds
+// and refits; the tests compare refitted nodes with it byte for byte.  Same rules
+// as the host builder (bvh_build.cpp): per axis the smallest exponent e with
+// 253 * 2^e >= the node extent, the frame origin one step below the node box, and
+// every child box rounded outward by at least one step, each bound checked in
+// double.
 #pragma once
 #include <math.h>
 #include <stdint.h>

@@ -37,7 +37,7 @@ struct DevLight { float4 a, b, c, d; };
 constexpr int kMaxSeg = 16;
 constexpr uint32_t kNoSegment = kMaxSeg;   // launch_trace: no rays of that kind
 // Rays of one traversal launch, at most. Queue indices and the work counter are 32 bits, and the counter runs past the
-// queue's end by up to a warp's lanes for every warp of the launch (0.4 M on this GPU).
+// queue's end by what the launch's warps ask for when it is empty (0.3 M on this GPU).
 constexpr uint64_t kMaxTraceRays = (1ull << 32) - (1u << 20);
 // Whether the extension rays of a chunk of `paths` and its shadow rays, up to `lights` + 1 a path, count as one queue.
 constexpr bool one_trace_launch(uint32_t paths, uint32_t lights) {

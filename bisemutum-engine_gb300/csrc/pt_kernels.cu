@@ -116,9 +116,10 @@ __device__ __forceinline__ void tile_pixel(uint32_t k, uint32_t width, uint32_t 
     x = 8u * tile + p - dy * cols;
     y = 4u * band + dy;
 }
-// Views of fewer samples per pixel than this are traced in tiles. 1-spp 1080p frame of the terrain 3772 -> 3738 us,
-// 16-spp 256x256 room 1115 -> 1108; at 64 samples a warp holds half a pixel and the order of the pixels does not show
-// (161.1 -> 161.3 ms).
+// Views of fewer samples per pixel than this are traced in tiles; with more a warp holds one pixel's samples or fewer, and
+// rows need no divisions by the tile. Frames, ms, tiles / rows: 1 spp, 1080p terrain 3.738 / 3.772; 8 spp, 640x360 room
+// 1.484 / 1.493; 16 spp, 1080p terrain 41.52 / 41.66; 24 to 48 spp within 0.3 % either way; 64 spp, 1080p room
+// 70.14 / 69.86, terrain 160.5 / 160.3.
 constexpr uint32_t kTileSpp = 32;
 
 __global__ void k_camera(const DevView* __restrict__ views, uint32_t n_views, uint64_t path_begin,
@@ -1064,9 +1065,16 @@ void launch_tlas_refit(cudaStream_t st, CwNode* nodes, float* node_box, const fl
     for (uint32_t l = 0; l <= narrow; ++l) lv.begin[l] = level_begin[l];
     k_tlas_refit<<<1, kRefitThreads, 0, st>>>(nodes, node_box, inst_box, lv, narrow);
 }
+// Small chunks are generated and shaded in blocks of 128 threads, so that 16,384 paths reach 128 SMs and not 32; larger
+// ones in blocks of 512, over which the direction grouping of the next rays spans. 8-segment 1-spp frames, us, 512 / 128
+// threads for shading: room 128^2 376 / 362, 256^2 528 / 511, 512^2 896 / 875, 1.48 M triangles 512^2 1232 / 1213, 275,400
+// paths 1258 / 1235, from 724^2 on level; for camera rays the two differ by 0.2 % from 200,000 paths on. 64 spp at 1080p
+// take 161.3 ms with 512 for shading.
+constexpr uint32_t kSmallBlockPaths = 300000;
+
 void launch_camera(const LaunchCfg& lc, cudaStream_t st, const DevView* views, uint32_t n_views,
                    uint64_t path_begin, uint32_t path_count, const Wavefront& wf, uint32_t max_segments) {
-    const uint32_t block = path_count <= 200000u ? 128u : (uint32_t)lc.block_shade;   // as launch_shade's
+    const uint32_t block = path_count <= kSmallBlockPaths ? 128u : (uint32_t)lc.block_shade;
     uint32_t blocks = (path_count + block - 1) / block;
     if (blocks == 0) blocks = 1;
     k_camera<<<blocks, block, 0, st>>>(views, n_views, path_begin, path_count, wf, max_segments);
@@ -1160,11 +1168,7 @@ void launch_extend_count(const LaunchCfg& lc, cudaStream_t st, const DevScene& s
 }
 void launch_shade(const LaunchCfg& lc, cudaStream_t st, const DevScene& sc, const DevView* views,
                   const Wavefront& wf, int q, uint32_t seg, float4* accum, uint32_t paths, bool cache) {
-    // Small chunks in blocks of 128 threads, so that 16,384 paths reach 128 SMs and not 32; larger ones in blocks of
-    // 512, over which the direction grouping of the next rays spans. 8-segment 1-spp frames, us, 512 / 128 threads:
-    // room 128^2 376 / 362, 256^2 528 / 511, 512^2 896 / 875, 1.48 M triangles 512^2 1232 / 1213, from 724^2 on level;
-    // 64 spp at 1080p keeps its 161.3 ms with 512.
-    const uint32_t block = paths <= 300000 ? 128u : (uint32_t)lc.block_shade;
+    const uint32_t block = paths <= kSmallBlockPaths ? 128u : (uint32_t)lc.block_shade;
     const uint32_t grid = min((uint32_t)lc.grid_shade, (uint32_t)(((uint64_t)paths + block - 1) / block));
     if (cache || !sc.dir_lights_only) k_shade<true><<<grid, block, 0, st>>>(sc, views, wf, q, seg, accum);
     else k_shade<false><<<grid, block, 0, st>>>(sc, views, wf, q, seg, accum);
