@@ -424,6 +424,8 @@ def run_ours(a, dist: Dist):
                         "api": "bsm_render with a host camera and a pinned host RGBA32F output"},
                 "gpu_launches": launches,
                 "roofline": roofline, "cpu_baseline": cpu, "clocks": clk,
+                "timed_as": "stages launched one by one, with events around each; e2e renders as a caller does, with one "
+                            "traversal launch per segment boundary",
                 "stages_ms_per_step": {"camera": round(ms_cam / a.steps, 3), "extend": round(ms_ext / a.steps, 3),
                                        "shade": round(ms_shade / a.steps, 3),
                                        "shadow": round(ms_shadow / a.steps, 3)},
