@@ -740,8 +740,8 @@ __global__ void __launch_bounds__(128, kTwoLevel ? 5 : 8) k_stage_ray(const CwNo
 // quarter of the time where materials are not opaque), so a warp whose 32 rays
 // are alike traces them a ray per lane and looks at the next 32.  A ray per
 // thread / the loop alone / this kernel, us, closest hits of 1,000,003 rays:
-// incoherent ones in 1.48 M triangles 653 / 416 / 419, in the room 384 / 266 / 270;
-// a camera's 246 / 301 / 273 and 219 / 299 / 256, with non-opaque materials 310 / 484 / 391.
+// incoherent ones in 1.48 M triangles 653 / 416 / 408, in the room 384 / 266 / 261;
+// a camera's 246 / 301 / 261 and 219 / 299 / 247, with non-opaque materials 310 / 484 / 358.
 template <bool kOpacity, int kOut>
 __global__ void __launch_bounds__(128, 8) k_stage(const CwNode* __restrict__ nodes, const CwTri* __restrict__ tris,
                                                   const __grid_constant__ StageArgs a) {
